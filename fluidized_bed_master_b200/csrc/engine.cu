@@ -164,7 +164,7 @@ template <typename R>
 void alloc_work(Alloc& A, SphWork<R>& W, DemWork<double>& DW, int ns, int nd, int ncells) {
     W.m_new = A.get<R>(ns); W.rho_new = A.get<R>(ns); W.rho_ref = A.get<R>(ns); W.DEMpor = A.get<R>(ns);
     W.dDEMpor_prev = A.get<R>(ns);
-    W.Cm = A.get<R>((size_t)ns * 9);
+    W.Cm = A.get<R>((size_t)ns * 6);
     W.ftx = A.get<R>(ns); W.fty = A.get<R>(ns); W.ftz = A.get<R>(ns); W.ftot = A.get<R>(ns);
     W.fpx = A.get<R>(ns); W.fpy = A.get<R>(ns); W.fpz = A.get<R>(ns);
     W.pgfx = A.get<R>(ns); W.pgfy = A.get<R>(ns); W.pgfz = A.get<R>(ns);
@@ -185,6 +185,10 @@ void alloc_work(Alloc& A, SphWork<R>& W, DemWork<double>& DW, int ns, int nd, in
     W.rec.f1 = A.get<V4<R>>(ns);
     W.rec.up = A.get<V4<R>>(ns);
     W.rec.ut = A.get<V4<R>>(ns);
+    W.rec.pa = A.get<PvRec<R>>(ns);
+    W.rec.pb = A.get<PvRec<R>>(ns);
+    W.rec.pu = A.get<V4<R>>(ns);
+    W.rec.rp = A.get<R>(ns);
     DW.flt_s = A.get<double>(nd); DW.flt_sd = A.get<double>(nd); DW.flt_sd2 = A.get<double>(nd); DW.DEMpor = A.get<double>(nd);
     DW.ftx = A.get<double>(nd); DW.fty = A.get<double>(nd); DW.ftz = A.get<double>(nd);
     DW.tqx = A.get<double>(nd); DW.tqy = A.get<double>(nd); DW.tqz = A.get<double>(nd);
@@ -683,11 +687,9 @@ int enqueue_step(SphdemHandle* H, EngineHost<R>* EH, int flags, int64_t* nl) {
     int ns = P.ns, nd = P.nd;
     int so = E.cur_s, sn = 1 - E.cur_s, dox = E.cur_d, dn = 1 - E.cur_d;
     int r;
-    // Wendland C2 (the default): the neighbour passes are instantiated with
-    // the kernel type fixed
-    const bool kt3 = P.kernel_type == 3;
-    // ... and, for the common switch set, with the switches fixed too
-    const bool swc = kt3 && switch_set(P) == SW_COMMON;
+    // Wendland C2 and C6 (the configurations' kernels): the neighbour passes
+    // are instantiated with the kernel type fixed
+    const bool kt3 = P.kernel_type == 3, kt5 = P.kernel_type == 5;
     const bool fork = H->concurrent && ns > 0 && nd > 0 && H->dem_stream;
     cudaStream_t sd = fork ? H->dem_stream : st;
     // event k recorded on stream a / waited for on stream b (fork only)
@@ -728,7 +730,7 @@ int enqueue_step(SphdemHandle* H, EngineHost<R>* EH, int flags, int64_t* nl) {
             CK(launch_list<R>(EH, S, EH->list_mode, st));
         }
         CK(wait(1, st));
-        { KTIME(KT_PASSA); CK((launch_pdl(swc ? k_passA<R, 3, SW_COMMON> : kt3 ? k_passA<R, 3, -1> : k_passA<R, -1, -1>, bs, TPB, 0, st, P, S, W, D, DW.rows))); }
+        { KTIME(KT_PASSA); CK((launch_pdl(kt3 ? k_passA<R, 3> : kt5 ? k_passA<R, 5> : k_passA<R, -1>, bs, TPB, 0, st, P, S, W, D, DW.rows))); }
         *nl += 2;
         {
             KTIME(KT_PASSB);
@@ -736,8 +738,10 @@ int enqueue_step(SphdemHandle* H, EngineHost<R>* EH, int flags, int64_t* nl) {
                 CK((launch_pdl(kt3 ? k_sps<R, 3> : k_sps<R, -1>, bs, TPB, 0, st, P, S, W)));
                 *nl += 1;
             }
-            if (P.iface | P.fb | P.sps | P.ipf) CK((launch_pdl(kt3 ? k_passB<R, true, 3, -1> : k_passB<R, true, -1, -1>, bs, TPB, 0, st, P, S, W, E.flags)));
-            else CK((launch_pdl(swc ? k_passB<R, false, 3, SW_COMMON> : kt3 ? k_passB<R, false, 3, -1> : k_passB<R, false, -1, -1>, bs, TPB, 0, st, P, S, W, E.flags)));
+            auto kb = P.con ? (kt3 ? k_passB<R, false, 3, true> : kt5 ? k_passB<R, false, 5, true> : k_passB<R, false, -1, true>)
+                            : (kt3 ? k_passB<R, false, 3, false> : kt5 ? k_passB<R, false, 5, false> : k_passB<R, false, -1, false>);
+            if (P.iface | P.fb | P.sps | P.ipf | P.fva) kb = P.con ? k_passB<R, true, -1, true> : k_passB<R, true, -1, false>;
+            CK((launch_pdl(kb, bs, TPB, 0, st, P, S, W, E.flags)));
         }
         *nl += 1;
     }
@@ -777,7 +781,7 @@ int enqueue_step(SphdemHandle* H, EngineHost<R>* EH, int flags, int64_t* nl) {
         }
         {
             KTIME(KT_PPE);
-            if (H->p.ppe_mode == SPHDEM_PPE_REFERENCE) CK((launch_pdl(swc ? k_ppe<R, 3, SW_COMMON> : kt3 ? k_ppe<R, 3, -1> : k_ppe<R, -1, -1>, bs, TPB, 0, st, P, S, W)));
+            if (H->p.ppe_mode == SPHDEM_PPE_REFERENCE) CK((launch_pdl(kt3 ? k_ppe<R, 3> : kt5 ? k_ppe<R, 5> : k_ppe<R, -1>, bs, TPB, 0, st, P, S, W)));
             else if ((r = enqueue_krylov<R>(H, EH, S, W))) return r;
         }
         {
@@ -787,7 +791,7 @@ int enqueue_step(SphdemHandle* H, EngineHost<R>* EH, int flags, int64_t* nl) {
             else
                 CK((launch_pdl(k_neumann<R>, bww, TPB, 0, st, P, S, W, W.p_new, W.rows, 0)));
         }
-        { KTIME(KT_PASSC); CK((launch_pdl(swc ? k_passC<R, 3, SW_COMMON> : kt3 ? k_passC<R, 3, -1> : k_passC<R, -1, -1>, bs, TPB, 0, st, P, S, W))); }
+        { KTIME(KT_PASSC); CK((launch_pdl(kt3 ? k_passC<R, 3> : kt5 ? k_passC<R, 5> : k_passC<R, -1>, bs, TPB, 0, st, P, S, W))); }
         *nl += 3;
         if (P.open_bc > 0) {
             KTIME(KT_OPENBC);
@@ -796,7 +800,7 @@ int enqueue_step(SphdemHandle* H, EngineHost<R>* EH, int flags, int64_t* nl) {
         }
         if (P.xsph) {
             KTIME(KT_XSPH);
-            CK((launch_pdl(kt3 ? k_xsph<R, 3> : k_xsph<R, -1>, bs, TPB, 0, st, P, S, W)));
+            CK((launch_pdl(kt3 ? k_xsph<R, 3> : kt5 ? k_xsph<R, 5> : k_xsph<R, -1>, bs, TPB, 0, st, P, S, W)));
             *nl += 1;
         }
     }

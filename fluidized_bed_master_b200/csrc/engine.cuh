@@ -10,7 +10,8 @@
 //   DEM contact history: SPHDEM_NSLOT slot-major planes, partner id int32
 //     and tangential spring double[3]  (slot s of particle i at s*n+i)
 //   packed records of what the neighbour passes read of a neighbour
-//     (records.cuh): position + tag, {m,rho}, {m',rho',T,eps}, {u,p}, {u,T}
+//     (records.cuh): position + tag, {m,rho}, {m',rho',T,eps}, {u,p}, {u,T},
+//     position + volume, {eps u*,p}, eps rho'
 // Persistent fields live in two copies (A/B) that the per-step reorder
 // gathers between; work arrays are single copies overwritten each step.
 #pragma once
@@ -48,12 +49,16 @@ struct SphRec {
     V4<R>* f1;
     V4<R>* up;
     V4<R>* ut;
+    PvRec<R>* pa;
+    PvRec<R>* pb;
+    V4<R>* pu;
+    R* rp;
 };
 
 template <typename R>
 struct SphWork {
     R *m_new, *rho_new, *rho_ref, *DEMpor, *dDEMpor_prev;
-    R* Cm;                       // 9*n, row-major per particle plane: Cm[k*n+i]
+    R* Cm;                       // 6*n, planes xx, xy, xz, yy, yz, zz of the symmetric matrix
     R *ftx, *fty, *ftz, *ftot;
     R *fpx, *fpy, *fpz;
     R *pgfx, *pgfy, *pgfz;

@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(128) k_kry_assemble(DevParams P, SphState<R> S
     if (i >= n) return;
     const SphRec<R> rec = W.rec;
     int it = S.itype[i], pt = S.ptype[i], bt = S.btype[i];
-    V4<R> upi = rec.up[i];
+    V4<R> upi = rec.pu[i];   // {eps u*, p}
     if (!kry_solve_row(P, it, pt, bt)) {
         K.kcnt[i] = 0;
         K.wm[i] = 0.0;
@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(128) k_kry_assemble(DevParams P, SphState<R> S
             float* f = K.fraw + (size_t)i * MLP_FEAT;
 #pragma unroll
             for (int q = 0; q < MLP_FEAT; q++) f[q] = 0.f;
-            K.pprev[i] = (double)upi.w;
+            K.pprev[i] = (double)S.pres[i];
         }
         return;
     }
@@ -183,11 +183,9 @@ __global__ void __launch_bounds__(128) k_kry_assemble(DevParams P, SphState<R> S
     Knl<R> Kn = knl_make<R>(P, th);
     PosRec<R> qi = ldr(rec.pos + i);
     V4<R> fi = rec.f1[i];
-    R uxi = upi.x, uyi = upi.y, uzi = upi.z, rhoi = fi.y, pori = fi.w;
+    R rhoi = fi.y, pori = fi.w;
     R irhoi = rcp(rhoi), prhoi = pori * rhoi;
-    R pux = pori * uxi, puy = pori * uyi, puz = pori * uzi;
-    const bool kgc = P.kgc == 1;
-    Cm9<R> Cm = cm_load(W.Cm, n, i, kgc);
+    const Cm6<R> Cm = cm6_load(W.Cm, n, i, P.kgc == 1);
     int cnt = min(W.ncnt[i], P.nb_cap);
     R bx = 0, by = 0, bz = 0;
     double dsum = 0, bfix = 0;
@@ -203,7 +201,7 @@ __global__ void __launch_bounds__(128) k_kry_assemble(DevParams P, SphState<R> S
             NbQ44<R> t;
             t.q = ldr(rec.pos + j);
             t.a = ldr(rec.f1 + j);
-            t.b = ldr(rec.up + j);
+            t.b = ldr(rec.pu + j);
             return t;
         },
         [&](int j, const NbQ44<R>& t) {
@@ -217,11 +215,14 @@ __global__ void __launch_bounds__(128) k_kry_assemble(DevParams P, SphState<R> S
                 R mj = fj.x, rhoj = fj.y, porj = fj.w, irj = rcp(rhoj);
                 R dw = kdw(Kn, r);
                 R gx = dw * g.dx * rinv, gy = dw * g.dy * rinv, gz = dw * g.dz * rinv;
-                cm_apply(Cm, kgc, gx, gy, gz);
+                const Disp<R> cg = cm6_mul(Cm, gx, gy, gz);
+                gx = cg.dx;
+                gy = cg.dy;
+                gz = cg.dz;
                 R mr = mj * irj;
-                bx += mr * (pux - porj * uj.x) * gx;
-                by += mr * (puy - porj * uj.y) * gy;
-                bz += mr * (puz - porj * uj.z) * gz;
+                bx += mr * (upi.x - uj.x) * gx;
+                by += mr * (upi.y - uj.y) * gy;
+                bz += mr * (upi.z - uj.z) * gz;
                 R c = -(g.dx * gx + g.dy * gy + g.dz * gz) * rinv * rinv;
                 R a = mj * ((prhoi + porj * rhoj) * irj * irhoi) * c;
                 dsum += (double)a;
@@ -979,7 +980,7 @@ __global__ void __launch_bounds__(128) k_kry_final(DevParams P, SphState<R> S, S
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P.ns) return;
     bool solve = kry_solve_row(P, S.itype[i], S.ptype[i], S.btype[i]);
-    R pold = W.rec.up[i].w;
+    R pold = S.pres[i];
     double dp = solve ? K.x[i] - (double)pold : 0.0;
     W.p_new[i] = solve ? (R)K.x[i] : pold;
     S.dpres[i] = (R)dp;

@@ -25,6 +25,22 @@
 //                                      wall pressure by the first Neumann pass
 //   UT   {ux, uy, uz, temp}            corrector (pass C), patched by the
 //                                      open-boundary pass for buffer particles
+//   PA   position + V0 = m / rho       start of step (cell gather), read by pass A
+//   PB   position + V = m' / rho'      pass A; V of walls patched by the Neumann
+//                                      pass, of buffers by the open-boundary pass
+//   PU   {eps u*, p}                   SPH predictor, read by the pressure equation;
+//                                      wall pressure by the first Neumann pass
+//   RP   eps rho'                      pass A; walls patched by the Neumann pass
+// A pair of the neighbour sums needs of j only its displacement, its volume
+// m / rho and one more vector, so PA and PB carry the volume in the fourth
+// word of the position record and the passes load 16 to 36 bytes per pair
+// (24 to 48 with {m, rho, ...} beside the tagged position; the passes were
+// bound by L1 wavefronts and issue slots).  The sign of the volume tells the
+// types that the Shepard sums take (PA: p_type 1; PB: 1 or 3) from the
+// others, and a NaN volume marks a particle that a pass cannot take from the
+// record alone (outside the fixed-point range, p_type >= 1000, i_type 4, or
+// a volume that is not >= 0): pv_slow reads that pair from the tagged
+// records and the double positions.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -47,12 +63,14 @@ struct Vec<float> {
     typedef float4 v4;
     typedef float2 v2;
     typedef int4 pos;
+    typedef int4 pv;
 };
 template <>
 struct Vec<double> {
     typedef Dbl4 v4;
     typedef double2 v2;
     typedef QPos64 pos;
+    typedef Dbl4 pv;
 };
 
 template <typename R>
@@ -61,6 +79,8 @@ template <typename R>
 using V2 = typename Vec<R>::v2;
 template <typename R>
 using PosRec = typename Vec<R>::pos;
+template <typename R>
+using PvRec = typename Vec<R>::pv;   // position + volume
 
 // ---- tag -----------------------------------------------------------------
 constexpr int TAG_OOR = 1 << 4;
@@ -81,6 +101,8 @@ __device__ __forceinline__ Dbl4 ldr(const Dbl4* p) {
     double2 a = __ldg(q), b = __ldg(q + 1);
     return Dbl4{a.x, a.y, b.x, b.y};
 }
+__device__ __forceinline__ double ldr(const double* p) { return __ldg(p); }
+__device__ __forceinline__ float ldr(const float* p) { return __ldg(p); }
 __device__ __forceinline__ QPos64 ldr(const QPos64* p) {
     const double2* q = reinterpret_cast<const double2*>(p);
     double2 a = __ldg(q), b = __ldg(q + 1);
@@ -288,10 +310,11 @@ __device__ __forceinline__ double fdiv(double a, double b) { return a / b; }
 // ---- smoothing kernel with per-particle constants -----------------------
 // W and dW/dr of functions_KNL.cuh:2-144 with 1/h precomputed.
 // KT is the kernel type when the kernel instantiation fixes it (3: Wendland
-// C2, the loops then carry no type test), -1 when it is read from kt.
+// C2, 5: Wendland C6; the loops then carry no type test), -1 when it is read
+// from kt.
 template <typename R, int KT = -1>
 struct Knl {
-    static_assert(KT == -1 || KT == 3, "kernel types fixed at compile time: Wendland C2");
+    static_assert(KT == -1 || KT == 3 || KT == 5, "kernel types fixed at compile time: Wendland C2 and C6");
     int kt;
     R tA, ih, th;   // normalisation, 1/h, h
 };
@@ -300,7 +323,7 @@ __device__ __forceinline__ Knl<R, KT> knl_make(const DevParams& P, R th) {
     Knl<R, KT> k;
     k.kt = P.kernel_type;
     k.tA = knl_tmpA<R>(P.kernel_type, P.dim, th);
-    k.ih = rcp(th);
+    k.ih = (R)1 / th;
     k.th = th;
     return k;
 }
@@ -318,88 +341,49 @@ __device__ __noinline__ R knl_dw_call(int kt, R tA, R tH, R rr) {
 }
 template <typename R, int KT>
 __device__ __forceinline__ R kw(const Knl<R, KT>& k, R rr) {
-    if (KT == 3 || k.kt == 3) {
+    if (KT == 3 || (KT == -1 && k.kt == 3)) {
         R q = rr * k.ih * (R)0.5;
         if (!(q < (R)1)) return (R)0;
         R a = (R)1 - q, a2 = a * a;
         return k.tA * a2 * a2 * ((R)1 + (R)4 * q);
     }
-    if constexpr (KT == -1) {
-        if (k.kt == 5) {
+    if constexpr (KT != 3) {
+        if (KT == 5 || k.kt == 5) {
             R q = rr * k.ih * (R)0.5;
             if (!(q < (R)1)) return (R)0;
             R a = (R)1 - q, a2 = a * a, a4 = a2 * a2;
             return k.tA * a4 * a4 * ((R)1 + (R)8 * q + (R)25 * q * q + (R)32 * q * q * q);
         }
-        return knl_w_call<R>(k.kt, k.tA, k.th, rr);
+        if constexpr (KT == -1) return knl_w_call<R>(k.kt, k.tA, k.th, rr);
     }
     return (R)0;
 }
 template <typename R, int KT>
 __device__ __forceinline__ R kdw(const Knl<R, KT>& k, R rr) {
-    if (KT == 3 || k.kt == 3) {
+    if (KT == 3 || (KT == -1 && k.kt == 3)) {
         R q = rr * k.ih * (R)0.5;
         if (!(q < (R)1)) return (R)0;
         R a = (R)1 - q;
         return ((R)0.5 * k.ih) * k.tA * ((R)-20 * q * a * a * a);
     }
-    if constexpr (KT == -1) {
-        if (k.kt == 5) {
+    if constexpr (KT != 3) {
+        if (KT == 5 || k.kt == 5) {
             R q = rr * k.ih * (R)0.5;
             if (!(q < (R)1)) return (R)0;
             R a = (R)1 - q, a2 = a * a, a4 = a2 * a2;
             return ((R)0.5 * k.ih) * k.tA * ((R)-22 * q * a4 * a2 * a * ((R)16 * q * q + (R)7 * q + (R)1));
         }
-        return knl_dw_call<R>(k.kt, k.tA, k.th, rr);
+        if constexpr (KT == -1) return knl_dw_call<R>(k.kt, k.tA, k.th, rr);
     }
     return (R)0;
 }
 
-// ---- gradient correction with the matrix held in registers --------------
-template <typename R>
-struct Cm9 {
-    R c[9];
-};
-template <typename R>
-__device__ __forceinline__ Cm9<R> cm_load(const R* __restrict__ Cm, int n, int i, int on) {
-    Cm9<R> m;
-#pragma unroll
-    for (int q = 0; q < 9; q++) m.c[q] = on ? Cm[(size_t)q * n + i] : (R)((q % 4) == 0);
-    return m;
-}
-template <typename R>
-__device__ __forceinline__ void cm_apply(const Cm9<R>& m, int on, R& ax, R& ay, R& az) {
-    if (!on) return;
-    R a = ax, b = ay, c = az;
-    ax = m.c[0] * a + m.c[1] * b + m.c[2] * c;
-    ay = m.c[3] * a + m.c[4] * b + m.c[5] * c;
-    az = m.c[6] * a + m.c[7] * b + m.c[8] * c;
-}
-
 // neighbour record bundles loaded by the list passes
-template <typename R>
-struct NbQ2 {
-    PosRec<R> q;
-    V2<R> a;
-};
-template <typename R>
-struct NbQ2S {
-    PosRec<R> q;
-    V2<R> a;
-    R s;
-};
 template <typename R>
 struct NbQ44 {
     PosRec<R> q;
     V4<R> a, b;
 };
-template <typename R>
-struct NbQ24 {
-    PosRec<R> q;
-    V2<R> a;
-    V4<R> b;
-};
-
 // ---- the SPH neighbour list ---------------------------------------------
 // Blocks of 8 entries per particle: entry k of particle i at
 // ((k / 8) n + i) 8 + k % 8.  A particle's 8 consecutive entries fill one
@@ -410,6 +394,141 @@ struct NbQ24 {
 __host__ __device__ __forceinline__ size_t nb_at(int k, int n, int i) {
     return ((size_t)(k >> 3) * n + i) * 8 + (k & 7);
 }
+
+// ---- pair sums over position + volume records --------------------------------
+// the volume word: +V for the types the Shepard sum takes, -V for the
+// others, NaN for a particle of the slow path
+template <typename R>
+__device__ __forceinline__ R pv_code(R v, int tag, bool shepard) {
+    if (!(v >= (R)0) || (tag & TAG_OOR) || tag_ptype(tag) >= 1000 || tag_itype(tag) == 4)
+        return sizeof(R) == 4 ? (R)__int_as_float(0x7fffffff) : (R)__longlong_as_double(0x7fffffffffffffffll);
+    return shepard ? v : -v;
+}
+__device__ __forceinline__ int4 pv_make(const int4& q, float v) { return make_int4(q.x, q.y, q.z, __float_as_int(v)); }
+__device__ __forceinline__ Dbl4 pv_make(const QPos64& q, double v) { return Dbl4{q.x, q.y, q.z, v}; }
+__device__ __forceinline__ float pv_vol(const int4& q) { return __int_as_float(q.w); }
+__device__ __forceinline__ double pv_vol(const Dbl4& q) { return q.w; }
+__device__ __forceinline__ void pv_set_vol(int4* p, int i, float v) { reinterpret_cast<float*>(p + i)[3] = v; }
+__device__ __forceinline__ void pv_set_vol(Dbl4* p, int i, double v) { p[i].w = v; }
+__device__ __forceinline__ Disp<float> pv_disp(const DevParams& P, const int4& a, const int4& b) {
+    return Disp<float>{(float)(a.x - b.x) * P.q_step[0], (float)(a.y - b.y) * P.q_step[1],
+                       (float)(a.z - b.z) * P.q_step[2]};
+}
+__device__ __forceinline__ Disp<double> pv_disp(const DevParams&, const Dbl4& a, const Dbl4& b) {
+    return Disp<double>{a.x - b.x, a.y - b.y, a.z - b.z};
+}
+// displacement from the double positions and the plain volume of j; kept
+// out of line, the loops hold registers for the common path only
+template <typename R>
+__device__ __noinline__ V4<R> pv_slow(const double* X, const double* Y, const double* Z, const R* m, const R* rho,
+                                      int i, int j) {
+    return mk4<R>((R)(X[i] - X[j]), (R)(Y[i] - Y[j]), (R)(Z[i] - Z[j]), m[j] / rho[j]);
+}
+// 1/|d| and |d| with |d|^2 floored (the self pair: d = 0, every term of it
+// carries a component of d or a difference that is 0)
+__device__ __forceinline__ float rsq_floor(float r2) {
+    float s;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(s) : "f"(fmaxf(r2, 1e-30f)));
+    return s;
+}
+__device__ __forceinline__ double rsq_floor(double r2) { return rsqrt(fmax(r2, 1e-60)); }
+
+// Kernel values without the constant factors, which leave the sums:
+// dW/dr = gn kg r and W = wn kws.  For the Wendland kernels dW/dr is r times
+// a polynomial in q = r / 2h, so a pair needs no division by r:
+//   C2: dW/dr / r = -5 tA / h^2 (1-q)^3
+//   C6: dW/dr / r = -5.5 tA / h^2 (1-q)^7 (16 q^2 + 7 q + 1)
+// Other kernels: kg = kdw / r, gn = wn = 1.
+template <typename R>
+__device__ __forceinline__ R wl_arg(R r, R hq) {
+    const R a = (R)1 - r * hq;
+    return a > (R)0 ? a : (R)0;
+}
+template <typename R, int KT>
+struct KnlSum {
+    Knl<R, KT> k;
+    R hq, gn, wn;
+};
+template <typename R, int KT>
+__device__ __forceinline__ KnlSum<R, KT> knl_sum(const DevParams& P, R th) {
+    KnlSum<R, KT> s;
+    s.k = knl_make<R, KT>(P, th);
+    s.hq = (R)0.5 * s.k.ih;
+    const int kt = KT >= 0 ? KT : s.k.kt;
+    s.gn = kt == 3 ? (R)-5 * s.k.ih * s.k.ih * s.k.tA : kt == 5 ? (R)-5.5 * s.k.ih * s.k.ih * s.k.tA : (R)1;
+    s.wn = kt == 3 || kt == 5 ? s.k.tA : (R)1;
+    return s;
+}
+template <typename R, int KT>
+__device__ __forceinline__ R kg(const KnlSum<R, KT>& s, R r, R rinv) {
+    if (KT == 3 || (KT < 0 && s.k.kt == 3)) {
+        const R a = wl_arg(r, s.hq);
+        return a * a * a;
+    }
+    if (KT == 5 || (KT < 0 && s.k.kt == 5)) {
+        const R a = wl_arg(r, s.hq), a2 = a * a, q = r * s.hq;
+        return a2 * a2 * a2 * a * (((R)16 * q + (R)7) * q + (R)1);
+    }
+    if constexpr (KT < 0) return kdw(s.k, r) * rinv;
+    return (R)0;
+}
+template <typename R, int KT>
+__device__ __forceinline__ R kws(const KnlSum<R, KT>& s, R r) {
+    if (KT == 3 || (KT < 0 && s.k.kt == 3)) {
+        const R a = wl_arg(r, s.hq), a2 = a * a;
+        return a2 * a2 * ((R)1 + (R)4 * (r * s.hq));
+    }
+    if (KT == 5 || (KT < 0 && s.k.kt == 5)) {
+        const R a = wl_arg(r, s.hq), a2 = a * a, a4 = a2 * a2, q = r * s.hq;
+        return a4 * a4 * ((((R)32 * q + (R)25) * q + (R)8) * q + (R)1);
+    }
+    if constexpr (KT < 0) return kw(s.k, r);
+    return (R)0;
+}
+
+// the gradient correction is the inverse of a symmetric moment matrix: six
+// planes xx, xy, xz, yy, yz, zz (the identity when it is off)
+template <typename R>
+struct Cm6 {
+    R xx, xy, xz, yy, yz, zz;
+};
+template <typename R>
+__device__ __forceinline__ Cm6<R> cm6_load(const R* __restrict__ Cm, int n, int i, bool on) {
+    if (!on) return Cm6<R>{1, 0, 0, 1, 0, 1};
+    return Cm6<R>{Cm[i], Cm[(size_t)n + i], Cm[(size_t)2 * n + i], Cm[(size_t)3 * n + i], Cm[(size_t)4 * n + i],
+                  Cm[(size_t)5 * n + i]};
+}
+template <typename R>
+__device__ __forceinline__ Disp<R> cm6_mul(const Cm6<R>& c, R x, R y, R z) {
+    return Disp<R>{c.xx * x + c.xy * y + c.xz * z, c.xy * x + c.yy * y + c.yz * z, c.xz * x + c.yz * y + c.zz * z};
+}
+
+// neighbour record bundles of the position + volume passes
+template <typename R>
+struct NbP {
+    PvRec<R> q;
+};
+template <typename R>
+struct NbPS {
+    PvRec<R> q;
+    R s;
+};
+template <typename R>
+struct NbP4 {
+    PvRec<R> q;
+    V4<R> b;
+};
+template <typename R>
+struct NbP4S {
+    PvRec<R> q;
+    V4<R> b;
+    R s;
+};
+template <typename R>
+struct NbP44 {
+    PvRec<R> q;
+    V4<R> b, a;
+};
 
 // ---- batched neighbour-list walk -------------------------------------------
 // The list passes are bound by the latency of the dependent loads (list
