@@ -18,6 +18,7 @@ namespace sphdem {
 // Constants that travel with every launch.  Copied from SphdemParams plus
 // the grid computed at commit time.
 struct DevParams {
+    int c2_passes;            // Wendland C2: its own forms of the neighbour passes (records.cuh)
     int kernel_type, dim, kgc, delsph, fp, fv, fva, fg, con, xsph, open_bc, rho_type;
     int iface, fb;            // interface sharpness force, repulsive boundary force (pass B)
     int sps;                  // fv_solve with the SPS turbulence model: eddy viscosity (k_sps)

@@ -687,9 +687,10 @@ int enqueue_step(SphdemHandle* H, EngineHost<R>* EH, int flags, int64_t* nl) {
     int ns = P.ns, nd = P.nd;
     int so = E.cur_s, sn = 1 - E.cur_s, dox = E.cur_d, dn = 1 - E.cur_d;
     int r;
-    // Wendland C2 and C6 (the configurations' kernels): the neighbour passes
-    // are instantiated with the kernel type fixed
-    const bool kt3 = P.kernel_type == 3, kt5 = P.kernel_type == 5;
+    // Wendland C2 (the configurations' kernel) has its own forms of the
+    // neighbour passes; the other kernels run the general ones, whose sums
+    // keep the reference's form pair by pair
+    const bool kt3 = P.kernel_type == 3;
     const bool fork = H->concurrent && ns > 0 && nd > 0 && H->dem_stream;
     cudaStream_t sd = fork ? H->dem_stream : st;
     // event k recorded on stream a / waited for on stream b (fork only)
@@ -730,7 +731,7 @@ int enqueue_step(SphdemHandle* H, EngineHost<R>* EH, int flags, int64_t* nl) {
             CK(launch_list<R>(EH, S, EH->list_mode, st));
         }
         CK(wait(1, st));
-        { KTIME(KT_PASSA); CK((launch_pdl(kt3 ? k_passA<R, 3> : kt5 ? k_passA<R, 5> : k_passA<R, -1>, bs, TPB, 0, st, P, S, W, D, DW.rows))); }
+        { KTIME(KT_PASSA); CK((launch_pdl(kt3 ? k_passA<R> : k_passA_any<R>, bs, TPB, 0, st, P, S, W, D, DW.rows))); }
         *nl += 2;
         {
             KTIME(KT_PASSB);
@@ -738,9 +739,9 @@ int enqueue_step(SphdemHandle* H, EngineHost<R>* EH, int flags, int64_t* nl) {
                 CK((launch_pdl(kt3 ? k_sps<R, 3> : k_sps<R, -1>, bs, TPB, 0, st, P, S, W)));
                 *nl += 1;
             }
-            auto kb = P.con ? (kt3 ? k_passB<R, false, 3, true> : kt5 ? k_passB<R, false, 5, true> : k_passB<R, false, -1, true>)
-                            : (kt3 ? k_passB<R, false, 3, false> : kt5 ? k_passB<R, false, 5, false> : k_passB<R, false, -1, false>);
-            if (P.iface | P.fb | P.sps | P.ipf | P.fva) kb = P.con ? k_passB<R, true, -1, true> : k_passB<R, true, -1, false>;
+            auto kb = !kt3 ? k_passB_any<R, false> : P.con ? k_passB<R, true> : k_passB<R, false>;
+            if (P.iface | P.fb | P.sps | P.ipf) kb = k_passB_any<R, true>;
+            else if (P.fva) kb = k_passB_any<R, false>;
             CK((launch_pdl(kb, bs, TPB, 0, st, P, S, W, E.flags)));
         }
         *nl += 1;
@@ -781,7 +782,7 @@ int enqueue_step(SphdemHandle* H, EngineHost<R>* EH, int flags, int64_t* nl) {
         }
         {
             KTIME(KT_PPE);
-            if (H->p.ppe_mode == SPHDEM_PPE_REFERENCE) CK((launch_pdl(kt3 ? k_ppe<R, 3> : kt5 ? k_ppe<R, 5> : k_ppe<R, -1>, bs, TPB, 0, st, P, S, W)));
+            if (H->p.ppe_mode == SPHDEM_PPE_REFERENCE) CK((launch_pdl(kt3 ? k_ppe<R> : k_ppe_any<R>, bs, TPB, 0, st, P, S, W)));
             else if ((r = enqueue_krylov<R>(H, EH, S, W))) return r;
         }
         {
@@ -791,7 +792,7 @@ int enqueue_step(SphdemHandle* H, EngineHost<R>* EH, int flags, int64_t* nl) {
             else
                 CK((launch_pdl(k_neumann<R>, bww, TPB, 0, st, P, S, W, W.p_new, W.rows, 0)));
         }
-        { KTIME(KT_PASSC); CK((launch_pdl(kt3 ? k_passC<R, 3> : kt5 ? k_passC<R, 5> : k_passC<R, -1>, bs, TPB, 0, st, P, S, W))); }
+        { KTIME(KT_PASSC); CK((launch_pdl(kt3 ? k_passC<R> : k_passC_any<R>, bs, TPB, 0, st, P, S, W))); }
         *nl += 3;
         if (P.open_bc > 0) {
             KTIME(KT_OPENBC);
@@ -800,7 +801,7 @@ int enqueue_step(SphdemHandle* H, EngineHost<R>* EH, int flags, int64_t* nl) {
         }
         if (P.xsph) {
             KTIME(KT_XSPH);
-            CK((launch_pdl(kt3 ? k_xsph<R, 3> : kt5 ? k_xsph<R, 5> : k_xsph<R, -1>, bs, TPB, 0, st, P, S, W)));
+            CK((launch_pdl(kt3 ? k_xsph<R> : k_xsph_any<R>, bs, TPB, 0, st, P, S, W)));
             *nl += 1;
         }
     }
@@ -933,6 +934,7 @@ static int commit_t(SphdemHandle* H) {
     DevParams& P = E.P;
     std::memset(&P, 0, sizeof(P));
     P.kernel_type = p.kernel_type; P.dim = p.dim; P.kgc = p.kgc_solve; P.delsph = p.delSPH_solve;
+    P.c2_passes = p.kernel_type == 3;
     P.fp = p.fp_solve; P.fv = p.fv_solve; P.fva = p.fva_solve; P.fg = p.fg_solve; P.con = p.con_solve;
     P.iface = p.interface_solve; P.fb = p.fb_solve; P.c_repulsive = p.c_repulsive;
     P.sps = p.fv_solve == 1 && p.turbulence_model == 3;   // SPS (Parameters.cuh:111)

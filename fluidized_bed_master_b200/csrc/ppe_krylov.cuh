@@ -164,7 +164,9 @@ __global__ void __launch_bounds__(128) k_kry_assemble(DevParams P, SphState<R> S
     if (i >= n) return;
     const SphRec<R> rec = W.rec;
     int it = S.itype[i], pt = S.ptype[i], bt = S.btype[i];
-    V4<R> upi = rec.pu[i];   // {eps u*, p}
+    // {eps u*, p} (Wendland C2) or {u*, p}
+    const V4<R>* __restrict__ up = P.c2_passes ? rec.pu : rec.up;
+    V4<R> upi = up[i];
     if (!kry_solve_row(P, it, pt, bt)) {
         K.kcnt[i] = 0;
         K.wm[i] = 0.0;
@@ -185,6 +187,8 @@ __global__ void __launch_bounds__(128) k_kry_assemble(DevParams P, SphState<R> S
     V4<R> fi = rec.f1[i];
     R rhoi = fi.y, pori = fi.w;
     R irhoi = rcp(rhoi), prhoi = pori * rhoi;
+    const R ei = P.c2_passes ? (R)1 : pori;
+    const R pux = ei * upi.x, puy = ei * upi.y, puz = ei * upi.z;
     const Cm6<R> Cm = cm6_load(W.Cm, n, i, P.kgc == 1);
     int cnt = min(W.ncnt[i], P.nb_cap);
     R bx = 0, by = 0, bz = 0;
@@ -201,7 +205,7 @@ __global__ void __launch_bounds__(128) k_kry_assemble(DevParams P, SphState<R> S
             NbQ44<R> t;
             t.q = ldr(rec.pos + j);
             t.a = ldr(rec.f1 + j);
-            t.b = ldr(rec.pu + j);
+            t.b = ldr(up + j);
             return t;
         },
         [&](int j, const NbQ44<R>& t) {
@@ -220,9 +224,10 @@ __global__ void __launch_bounds__(128) k_kry_assemble(DevParams P, SphState<R> S
                 gy = cg.dy;
                 gz = cg.dz;
                 R mr = mj * irj;
-                bx += mr * (upi.x - uj.x) * gx;
-                by += mr * (upi.y - uj.y) * gy;
-                bz += mr * (upi.z - uj.z) * gz;
+                const R ej = P.c2_passes ? (R)1 : porj;
+                bx += mr * (pux - ej * uj.x) * gx;
+                by += mr * (puy - ej * uj.y) * gy;
+                bz += mr * (puz - ej * uj.z) * gz;
                 R c = -(g.dx * gx + g.dy * gy + g.dz * gz) * rinv * rinv;
                 R a = mj * ((prhoi + porj * rhoj) * irj * irhoi) * c;
                 dsum += (double)a;

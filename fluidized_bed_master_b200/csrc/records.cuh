@@ -25,6 +25,7 @@
 //                                      wall pressure by the first Neumann pass
 //   UT   {ux, uy, uz, temp}            corrector (pass C), patched by the
 //                                      open-boundary pass for buffer particles
+// Wendland C2 (the configurations' kernel), read by its own passes:
 //   PA   position + V0 = m / rho       start of step (cell gather), read by pass A
 //   PB   position + V = m' / rho'      pass A; V of walls patched by the Neumann
 //                                      pass, of buffers by the open-boundary pass
@@ -96,10 +97,10 @@ __device__ __forceinline__ float4 ldr(const float4* p) { return __ldg(p); }
 __device__ __forceinline__ float2 ldr(const float2* p) { return __ldg(p); }
 __device__ __forceinline__ int4 ldr(const int4* p) { return __ldg(p); }
 __device__ __forceinline__ double2 ldr(const double2* p) { return __ldg(p); }
-__device__ __forceinline__ Dbl4 ldr(const Dbl4* p) {
-    const double2* q = reinterpret_cast<const double2*>(p);
-    double2 a = __ldg(q), b = __ldg(q + 1);
-    return Dbl4{a.x, a.y, b.x, b.y};
+__device__ __forceinline__ Dbl4 ldr(const Dbl4* p) {   // one 32-byte load
+    Dbl4 v;
+    asm volatile("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+    return v;
 }
 __device__ __forceinline__ double ldr(const double* p) { return __ldg(p); }
 __device__ __forceinline__ float ldr(const float* p) { return __ldg(p); }
@@ -310,11 +311,10 @@ __device__ __forceinline__ double fdiv(double a, double b) { return a / b; }
 // ---- smoothing kernel with per-particle constants -----------------------
 // W and dW/dr of functions_KNL.cuh:2-144 with 1/h precomputed.
 // KT is the kernel type when the kernel instantiation fixes it (3: Wendland
-// C2, 5: Wendland C6; the loops then carry no type test), -1 when it is read
-// from kt.
+// C2, the loops then carry no type test), -1 when it is read from kt.
 template <typename R, int KT = -1>
 struct Knl {
-    static_assert(KT == -1 || KT == 3 || KT == 5, "kernel types fixed at compile time: Wendland C2 and C6");
+    static_assert(KT == -1 || KT == 3, "kernel types fixed at compile time: Wendland C2");
     int kt;
     R tA, ih, th;   // normalisation, 1/h, h
 };
@@ -323,7 +323,7 @@ __device__ __forceinline__ Knl<R, KT> knl_make(const DevParams& P, R th) {
     Knl<R, KT> k;
     k.kt = P.kernel_type;
     k.tA = knl_tmpA<R>(P.kernel_type, P.dim, th);
-    k.ih = (R)1 / th;
+    k.ih = rcp(th);
     k.th = th;
     return k;
 }
@@ -341,49 +341,90 @@ __device__ __noinline__ R knl_dw_call(int kt, R tA, R tH, R rr) {
 }
 template <typename R, int KT>
 __device__ __forceinline__ R kw(const Knl<R, KT>& k, R rr) {
-    if (KT == 3 || (KT == -1 && k.kt == 3)) {
+    if (KT == 3 || k.kt == 3) {
         R q = rr * k.ih * (R)0.5;
         if (!(q < (R)1)) return (R)0;
         R a = (R)1 - q, a2 = a * a;
         return k.tA * a2 * a2 * ((R)1 + (R)4 * q);
     }
-    if constexpr (KT != 3) {
-        if (KT == 5 || k.kt == 5) {
+    if constexpr (KT == -1) {
+        if (k.kt == 5) {
             R q = rr * k.ih * (R)0.5;
             if (!(q < (R)1)) return (R)0;
             R a = (R)1 - q, a2 = a * a, a4 = a2 * a2;
             return k.tA * a4 * a4 * ((R)1 + (R)8 * q + (R)25 * q * q + (R)32 * q * q * q);
         }
-        if constexpr (KT == -1) return knl_w_call<R>(k.kt, k.tA, k.th, rr);
+        return knl_w_call<R>(k.kt, k.tA, k.th, rr);
     }
     return (R)0;
 }
 template <typename R, int KT>
 __device__ __forceinline__ R kdw(const Knl<R, KT>& k, R rr) {
-    if (KT == 3 || (KT == -1 && k.kt == 3)) {
+    if (KT == 3 || k.kt == 3) {
         R q = rr * k.ih * (R)0.5;
         if (!(q < (R)1)) return (R)0;
         R a = (R)1 - q;
         return ((R)0.5 * k.ih) * k.tA * ((R)-20 * q * a * a * a);
     }
-    if constexpr (KT != 3) {
-        if (KT == 5 || k.kt == 5) {
+    if constexpr (KT == -1) {
+        if (k.kt == 5) {
             R q = rr * k.ih * (R)0.5;
             if (!(q < (R)1)) return (R)0;
             R a = (R)1 - q, a2 = a * a, a4 = a2 * a2;
             return ((R)0.5 * k.ih) * k.tA * ((R)-22 * q * a4 * a2 * a * ((R)16 * q * q + (R)7 * q + (R)1));
         }
-        if constexpr (KT == -1) return knl_dw_call<R>(k.kt, k.tA, k.th, rr);
+        return knl_dw_call<R>(k.kt, k.tA, k.th, rr);
     }
     return (R)0;
 }
 
+// ---- gradient correction with the matrix held in registers --------------
+template <typename R>
+struct Cm9 {
+    R c[9];
+};
+template <typename R>
+__device__ __forceinline__ Cm9<R> cm_load(const R* __restrict__ Cm, int n, int i, int on) {
+    // six stored planes (xx, xy, xz, yy, yz, zz) of the symmetric matrix
+    constexpr int plane[9] = {0, 1, 2, 1, 3, 4, 2, 4, 5};
+    Cm9<R> m;
+#pragma unroll
+    for (int q = 0; q < 9; q++) m.c[q] = on ? Cm[(size_t)plane[q] * n + i] : (R)((q % 4) == 0);
+    return m;
+}
+template <typename R>
+__device__ __forceinline__ void cm_apply(const Cm9<R>& m, int on, R& ax, R& ay, R& az) {
+    if (!on) return;
+    R a = ax, b = ay, c = az;
+    ax = m.c[0] * a + m.c[1] * b + m.c[2] * c;
+    ay = m.c[3] * a + m.c[4] * b + m.c[5] * c;
+    az = m.c[6] * a + m.c[7] * b + m.c[8] * c;
+}
+
 // neighbour record bundles loaded by the list passes
+template <typename R>
+struct NbQ2 {
+    PosRec<R> q;
+    V2<R> a;
+};
+template <typename R>
+struct NbQ2S {
+    PosRec<R> q;
+    V2<R> a;
+    R s;
+};
 template <typename R>
 struct NbQ44 {
     PosRec<R> q;
     V4<R> a, b;
 };
+template <typename R>
+struct NbQ24 {
+    PosRec<R> q;
+    V2<R> a;
+    V4<R> b;
+};
+
 // ---- the SPH neighbour list ---------------------------------------------
 // Blocks of 8 entries per particle: entry k of particle i at
 // ((k / 8) n + i) 8 + k % 8.  A particle's 8 consecutive entries fill one
@@ -433,57 +474,31 @@ __device__ __forceinline__ float rsq_floor(float r2) {
 }
 __device__ __forceinline__ double rsq_floor(double r2) { return rsqrt(fmax(r2, 1e-60)); }
 
-// Kernel values without the constant factors, which leave the sums:
-// dW/dr = gn kg r and W = wn kws.  For the Wendland kernels dW/dr is r times
-// a polynomial in q = r / 2h, so a pair needs no division by r:
-//   C2: dW/dr / r = -5 tA / h^2 (1-q)^3
-//   C6: dW/dr / r = -5.5 tA / h^2 (1-q)^7 (16 q^2 + 7 q + 1)
-// Other kernels: kg = kdw / r, gn = wn = 1.
+// Wendland C2 without its constant factors, which leave the sums:
+// dW/dr / r = gn (1-q)^3 with gn = -5 tA / h^2 and W = tA (1-q)^4 (1 + 4q),
+// q = r / 2h: a pair needs no division by r.
 template <typename R>
-__device__ __forceinline__ R wl_arg(R r, R hq) {
-    const R a = (R)1 - r * hq;
-    return a > (R)0 ? a : (R)0;
-}
-template <typename R, int KT>
-struct KnlSum {
-    Knl<R, KT> k;
-    R hq, gn, wn;
+struct C2Sum {
+    R hq, gn, wn;   // 1 / 2h, the factors of dW/dr / r and of W
 };
-template <typename R, int KT>
-__device__ __forceinline__ KnlSum<R, KT> knl_sum(const DevParams& P, R th) {
-    KnlSum<R, KT> s;
-    s.k = knl_make<R, KT>(P, th);
-    s.hq = (R)0.5 * s.k.ih;
-    const int kt = KT >= 0 ? KT : s.k.kt;
-    s.gn = kt == 3 ? (R)-5 * s.k.ih * s.k.ih * s.k.tA : kt == 5 ? (R)-5.5 * s.k.ih * s.k.ih * s.k.tA : (R)1;
-    s.wn = kt == 3 || kt == 5 ? s.k.tA : (R)1;
-    return s;
+template <typename R>
+__device__ __forceinline__ C2Sum<R> c2_sum(const DevParams& P, R th) {
+    const R ih = (R)1 / th, tA = knl_tmpA<R>(3, P.dim, th);
+    return C2Sum<R>{(R)0.5 * ih, (R)-5 * ih * ih * tA, tA};
 }
-template <typename R, int KT>
-__device__ __forceinline__ R kg(const KnlSum<R, KT>& s, R r, R rinv) {
-    if (KT == 3 || (KT < 0 && s.k.kt == 3)) {
-        const R a = wl_arg(r, s.hq);
-        return a * a * a;
-    }
-    if (KT == 5 || (KT < 0 && s.k.kt == 5)) {
-        const R a = wl_arg(r, s.hq), a2 = a * a, q = r * s.hq;
-        return a2 * a2 * a2 * a * (((R)16 * q + (R)7) * q + (R)1);
-    }
-    if constexpr (KT < 0) return kdw(s.k, r) * rinv;
-    return (R)0;
+template <typename R>
+__device__ __forceinline__ R c2_g(const C2Sum<R>& s, R r) {
+    R a = (R)1 - r * s.hq;
+    a = a > (R)0 ? a : (R)0;
+    return a * a * a;
 }
-template <typename R, int KT>
-__device__ __forceinline__ R kws(const KnlSum<R, KT>& s, R r) {
-    if (KT == 3 || (KT < 0 && s.k.kt == 3)) {
-        const R a = wl_arg(r, s.hq), a2 = a * a;
-        return a2 * a2 * ((R)1 + (R)4 * (r * s.hq));
-    }
-    if (KT == 5 || (KT < 0 && s.k.kt == 5)) {
-        const R a = wl_arg(r, s.hq), a2 = a * a, a4 = a2 * a2, q = r * s.hq;
-        return a4 * a4 * ((((R)32 * q + (R)25) * q + (R)8) * q + (R)1);
-    }
-    if constexpr (KT < 0) return kw(s.k, r);
-    return (R)0;
+template <typename R>
+__device__ __forceinline__ R c2_w(const C2Sum<R>& s, R r) {
+    const R q = r * s.hq;
+    R a = (R)1 - q;
+    a = a > (R)0 ? a : (R)0;
+    const R a2 = a * a;
+    return a2 * a2 * ((R)1 + (R)4 * q);
 }
 
 // the gradient correction is the inverse of a symmetric moment matrix: six
@@ -524,17 +539,67 @@ struct NbP4S {
     V4<R> b;
     R s;
 };
-template <typename R>
-struct NbP44 {
-    PvRec<R> q;
-    V4<R> b, a;
-};
-
 // ---- batched neighbour-list walk -------------------------------------------
 // The list passes are bound by the latency of the dependent loads (list
-// entry -> neighbour records).  Loading the records of B neighbours before
-// any of their arithmetic keeps B independent load chains in flight; the
-// sums still run in list order.  B = 2 or 4 entries come in one vector load.
+// entry -> neighbour records) and by L1 wavefronts.  The entries of a batch
+// of 4 come in one 16-byte load, requested two batches ahead, so their
+// latency (the list streams from L2 or HBM) is hidden behind the arithmetic
+// of the batches before.  The records of a batch are loaded before any of
+// its arithmetic; prep turns each into its pair (displacement, volume), fix
+// replaces those that a record does not give (rare; a branch per batch), and
+// comp runs on the four pairs without branches between them.  The sums run
+// in list order.  The last batch is padded with the particle itself at zero
+// volume, which adds nothing.
+__device__ __forceinline__ int4 nb_ld4(const int* p) {
+    int4 v;
+    asm volatile("ld.global.nc.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+template <typename T, typename PV, typename L, typename P, typename X, typename C>
+__device__ __forceinline__ void nb_sum(int cnt, const int* __restrict__ nb, int n, int i, L load, P prep, X fix,
+                                       C comp) {
+    if (cnt <= 0) return;
+    const int* p = nb + (size_t)i * 8;   // entry k of particle i: nb_at(k, n, i)
+    const size_t step = (size_t)n * 8;
+    int4 e0 = nb_ld4(p), e1 = make_int4(i, i, i, i);
+    if (cnt > 4) e1 = nb_ld4(p + 4);
+    auto batch = [&](const int4& e, int m) {
+        int j[4] = {e.x, e.y, e.z, e.w};
+        T r[4];
+        PV g[4];
+        bool bad = false;
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            if (m < 4 && u >= m) j[u] = i;
+            r[u] = load(j[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) bad |= prep(r[u], g[u]);
+        if (bad) {
+#pragma unroll
+            for (int u = 0; u < 4; u++) fix(j[u], r[u], g[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            if (m < 4 && u >= m) g[u].v = g[u].vs = 0;
+            comp(j[u], r[u], g[u]);
+        }
+    };
+    int k = 0;
+#pragma unroll 1
+    for (; k + 4 <= cnt; k += 4) {
+        // entries k+8 .. k+11 lie one block of 8 further
+        int4 e2 = e1;
+        if (k + 8 < cnt) e2 = nb_ld4(p + (size_t)((k >> 3) + 1) * step + (k & 4));
+        batch(e0, 4);
+        e0 = e1;
+        e1 = e2;
+    }
+    if (k < cnt) batch(e0, cnt - k);
+}
+
+// the same list, one entry after another in batches of B (passes that keep
+// per-pair control flow)
 template <int B, typename T, typename L, typename C>
 __device__ __forceinline__ void nb_walk(int cnt, const int* __restrict__ nb, int n, int i, L load, C comp) {
     static_assert(B == 2 || B == 4, "list walks load 2 or 4 entries at a time");

@@ -60,23 +60,31 @@ __device__ __forceinline__ R sph_volume(const DevParams& P, R th, R hd) {
     return P.dim == 2 ? (th / hd) * (th / hd) : (th / hd) * (th / hd) * (th / hd);
 }
 
-// One pair of a position + volume pass: displacement x_i - x_j and the volume
-// word of j.  True when the pair came from the slow path (i or j is not
-// usable from its record): v is then the plain volume and tag the tag of j.
+// One pair of a position + volume pass (nb_sum): displacement x_i - x_j, the
+// volume of j in the pass's sums and in its Shepard sum.
 template <typename R>
-__device__ __forceinline__ bool pv_pair(const DevParams& P, const SphState<R>& S, const PosRec<R>* pos, const R* m,
-                                        const R* rho, const PvRec<R>& qi, bool slow_i, const PvRec<R>& qj, int i, int j,
-                                        Disp<R>& d, R& v, int& tag) {
-    v = pv_vol(qj);
-    if (slow_i || v != v) {
-        const V4<R> s = pv_slow<R>(S.x, S.y, S.z, m, rho, i, j);
-        d = Disp<R>{s.x, s.y, s.z};
-        v = s.w;
-        tag = ldr(pos + j).w;
-        return true;
-    }
-    d = pv_disp(P, qi, qj);
-    return false;
+struct PairV {
+    R dx, dy, dz, v, vs;
+};
+// prep step: SHEP: the Shepard sum takes only the marked types
+template <typename R, bool SHEP>
+__device__ __forceinline__ bool pv_prep(const DevParams& P, const PvRec<R>& qi, bool slow_i, const PvRec<R>& qj,
+                                        PairV<R>& g) {
+    const R v = pv_vol(qj);
+    const Disp<R> d = pv_disp(P, qi, qj);
+    g = PairV<R>{d.dx, d.dy, d.dz, (R)fabs(v), SHEP ? (v > (R)0 ? v : (R)0) : (R)fabs(v)};
+    return slow_i || v != v;
+}
+// fix step of one pair: true when i or j is not usable from its record; the
+// pair then comes from the double positions, and tag is the tag of j
+template <typename R>
+__device__ __forceinline__ bool pv_fix(const SphState<R>& S, const PosRec<R>* pos, const R* m, const R* rho,
+                                       bool slow_i, const PvRec<R>& qj, int i, int j, PairV<R>& g, int& tag) {
+    if (!slow_i && pv_vol(qj) == pv_vol(qj)) return false;
+    const V4<R> s = pv_slow<R>(S.x, S.y, S.z, m, rho, i, j);
+    g = PairV<R>{s.x, s.y, s.z, s.w, s.w};
+    tag = ldr(pos + j).w;
+    return true;
 }
 
 // 27-cell stencil in the reference order (z,y,x), calling f(j) for every
@@ -162,7 +170,7 @@ __global__ void k_cells_gather_sph(DevParams P, SphState<R> src, SphGatherSrc<R>
     const PosRec<R> q = make_pos<R>(P, x, y, z, pt, bt, it);
     store_pos(rec.pos, i, q);
     rec.mr0[i] = mk2<R>(m, rho);
-    rec.pa[i] = pv_make(q, pv_code<R>(m / rho, q.w, pt == 1));
+    if (P.c2_passes) rec.pa[i] = pv_make(q, pv_code<R>(m / rho, q.w, pt == 1));
     rec.up[i] = mk4<R>(ux, uy, uz, pr);
     // walls and buffer particles of the step (parked slots excluded), up to
     // the launch bounds of their passes
@@ -721,9 +729,11 @@ __global__ void __launch_bounds__(DL_WARPS * 32) k_build_dlist(DevParams P, cons
 // rho_new so that no thread sees a half-updated neighbour.
 // ---------------------------------------------------------------------------
 // A pair adds V (x x^T) kg to the six moments and V kws to the Shepard sum
-// (V = m / rho of the record, constant factors after the loop).
-template <typename R, int KT>
-__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 8 : 1) k_passA(DevParams P, SphState<R> S, SphWork<R> W, DemState<double> D,
+// (V = m / rho of the record, constant factors after the loop).  Registers in
+// FP32 are held to 7 blocks per SM: 91 us on the bench bed at 8 blocks
+// (spills), 86 at 7, 92 at 6.
+template <typename R>
+__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 7 : 1) k_passA(DevParams P, SphState<R> S, SphWork<R> W, DemState<double> D,
                                                const int4* __restrict__ drows) {
     grid_dep_wait();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -742,35 +752,32 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 8 : 1) k_passA(DevParams
     W.dDEMpor_prev[i] = dprev;
     double xi = S.x[i], yi = S.y[i], zi = S.z[i], hi = S.h[i];
     R th = (R)hi;
-    const KnlSum<R, KT> K = knl_sum<R, KT>(P, th);
+    const C2Sum<R> K = c2_sum<R>(P, th);
     const PvRec<R> qi = ldr(rec.pa + i);
     const bool slow_i = pv_vol(qi) != pv_vol(qi);
     int cnt = min(W.ncnt[i], P.nb_cap);
     R txx = 0, tyy = 0, tzz = 0, txy = 0, tyz = 0, tzx = 0, sflt = 0;
     const int* __restrict__ nb = W.nbr;
     const bool kgc = P.kgc == 1;
-    nb_walk<4, NbP<R>>(
+    nb_sum<NbP<R>, PairV<R>>(
         cnt, nb, n, i,
         [&](int j) {
             NbP<R> t;
             t.q = ldr(rec.pa + j);
             return t;
         },
-        [&](int j, const NbP<R>& t) {
-            Disp<R> g;
-            R v, vs;
+        [&](const NbP<R>& t, PairV<R>& g) { return pv_prep<R, true>(P, qi, slow_i, t.q, g); },
+        [&](int j, NbP<R>& t, PairV<R>& g) {
             int tag;
-            if (pv_pair(P, S, rec.pos, S.m, S.rho, qi, slow_i, t.q, i, j, g, v, tag)) {
-                if (tag_ptype(tag) > 1000) return;
-                vs = tag_ptype(tag) == 1 ? v : (R)0;
-            } else {
-                vs = v > (R)0 ? v : (R)0;
-                v = fabs(v);
-            }
+            if (!pv_fix(S, rec.pos, S.m, S.rho, slow_i, t.q, i, j, g, tag)) return;
+            if (tag_ptype(tag) > 1000) g.v = 0;
+            if (tag_ptype(tag) != 1) g.vs = 0;
+        },
+        [&](int, const NbP<R>&, const PairV<R>& g) {
             const R r2 = g.dx * g.dx + g.dy * g.dy + g.dz * g.dz;
             const R rinv = rsq_floor(r2), r = r2 * rinv;
-            sflt += vs * kws(K, r);
-            const R w = v * kg(K, r, rinv);
+            sflt += g.vs * c2_w(K, r);
+            const R w = g.v * c2_g(K, r);
             const R wx = w * g.dx, wy = w * g.dy, wz = w * g.dz;
             txx += wx * g.dx;
             txy += wx * g.dy;
@@ -819,14 +826,15 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 8 : 1) k_passA(DevParams
     double Rr = P.kappa * hi;
     R por = 0, dfx = 0, dfy = 0, dfz = 0;
     if (P.nd > 0) {
+        const Knl<R, 3> Kd = knl_make<R, 3>(P, th);
         float r2l = r2_lo(Rr), r2h = r2_hi(Rr);
         auto dem = [&](int j) {
             if (D.ptype[j] <= 1000) return;
             PairT<R> g = pair_test<R>(xi, yi, zi, D.x[j], D.y[j], D.z[j], Rr, 1e-20, r2l, r2h);
             if (!g.in) return;
             R r = g.r + (R)1e-20, ir = rcp(r);
-            R w = kw(K.k, r);
-            R dw = kdw(K.k, r);
+            R w = kw(Kd, r);
+            R dw = kdw(Kd, r);
             R rj = (R)D.rad[j];
             R v = dem_measure(P, rj);
             por += w * v;
@@ -1057,11 +1065,10 @@ __global__ void __launch_bounds__(128) k_sps(DevParams P, SphState<R> S, SphWork
 // du; heat conduction and advection share T_i - T_j the same way.  (The
 // reference multiplies C into every pair's gradient and divides by r; that
 // form took 118 instructions per pair, this one about 60.)
-// FULL: a force that needs m_j and rho_j themselves is on (interface
-// sharpness, repulsive boundary, SPS eddy viscosity, inter-particle surface
-// tension, artificial viscosity); a separate instantiation, so that the
-// default pass keeps its registers.  HEAT: conduction (con_solve).
-template <typename R, bool FULL, int KT, bool HEAT>
+// The forces that need m_j and rho_j themselves (interface sharpness,
+// repulsive boundary, SPS eddy viscosity, inter-particle surface tension,
+// artificial viscosity) run in k_passB_any.  HEAT: conduction (con_solve).
+template <typename R, bool HEAT>
 __global__ void __launch_bounds__(128) k_passB(DevParams P, SphState<R> S, SphWork<R> W, const DevFlags* F) {
     grid_dep_wait();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1078,52 +1085,65 @@ __global__ void __launch_bounds__(128) k_passB(DevParams P, SphState<R> S, SphWo
     bool adv = !(P.open_bc > 0 && bt > 0) && pt < 1000 && pt > 0;
     if (!filt && !adv) return;
     R th = (R)S.h[i];
-    const KnlSum<R, KT> K = knl_sum<R, KT>(P, th);
+    const C2Sum<R> K = c2_sum<R>(P, th);
     const PvRec<R> qi = ldr(rec.pb + i);
     const bool slow_i = pv_vol(qi) != pv_vol(qi);
     V4<R> upi = rec.up[i];
     V4<R> fi = rec.f1[i];
     R uxi = upi.x, uyi = upi.y, uzi = upi.z, pi = upi.w;
-    R rhoi = fi.y, tempi = fi.z, pori = fi.w, mi = fi.x;
+    R rhoi = fi.y, tempi = fi.z, pori = fi.w;
     R irhoi = rcp(rhoi);
     const Cm6<R> C = cm6_load(W.Cm, n, i, P.kgc == 1);
-    R vis = (R)P.mu_gas, vis_h = (vis * vis) / (vis + vis);
-    R kc = (R)P.k_sph;
+    const R vis = (R)P.mu_gas, vis_h = (vis * vis) / (vis + vis), kc = (R)P.k_sph;
     // per-particle factors of the pair terms
     const R cv_i = P.fv ? vis_h * (R)4 * pori * irhoi : (R)0;
-    R visi = vis;
-    if (FULL && P.sps) visi += W.vist[i];   // viscosity + P3.vis_t (functions_PPE2.cuh:1323)
     const R ch_i = (R)4 * pori * kc * kc * irhoi / (kc + kc) / (R)P.cp_sph * (R)(pt != -1);
     Disp<R> w = cm6_mul(C, uxi, uyi, uzi);
     if (P.sph_lagrangian) w = Disp<R>{0, 0, 0};
     int cnt = min(W.ncnt[i], P.nb_cap);
     R flt = 0, tx = 0, ty = 0, tz = 0, px = 0, py = 0, pz = 0, et = 0;
-    // FULL: artificial viscosity (corrected after the loop) and the raw forces
-    R vx = 0, vy = 0, vz = 0, fx = 0, fy = 0, fz = 0;
     const int* __restrict__ nb = W.nbr;
-    using Rec = std::conditional_t<FULL, NbP44<R>, std::conditional_t<HEAT, NbP4S<R>, NbP4<R>>>;
-    nb_walk<4, Rec>(
+    using Rec = std::conditional_t<HEAT, NbP4S<R>, NbP4<R>>;
+    if (!adv) {   // a filter step of a row without forces: the Shepard sum alone
+        nb_sum<NbP<R>, PairV<R>>(
+            cnt, nb, n, i, [&](int j) { return NbP<R>{ldr(rec.pb + j)}; },
+            [&](const NbP<R>& t, PairV<R>& g) { return pv_prep<R, false>(P, qi, slow_i, t.q, g); },
+            [&](int j, NbP<R>& t, PairV<R>& g) {
+                int tag;
+                pv_fix(S, rec.pos, W.m_new, W.rho_new, slow_i, t.q, i, j, g, tag);
+            },
+            [&](int, const NbP<R>&, const PairV<R>& g) {
+                const R r2 = g.dx * g.dx + g.dy * g.dy + g.dz * g.dz;
+                flt += g.vs * c2_w(K, r2 * rsq_floor(r2));
+            });
+        S.flt_s[i] = flt * K.wn;
+        return;
+    }
+    nb_sum<Rec, PairV<R>>(
         cnt, nb, n, i,
         [&](int j) {
             Rec t;
             t.q = ldr(rec.pb + j);
             t.b = ldr(rec.up + j);
-            if constexpr (FULL) t.a = ldr(rec.f1 + j);
-            else if constexpr (HEAT) t.s = ldr(S.temp + j);
+            if constexpr (HEAT) t.s = ldr(S.temp + j);
             return t;
         },
-        [&](int j, const Rec& t) {
+        [&](const Rec& t, PairV<R>& g) { return pv_prep<R, false>(P, qi, slow_i, t.q, g); },
+        [&](int j, Rec& t, PairV<R>& g) {
+            int tag;
+            if (!pv_fix(S, rec.pos, W.m_new, W.rho_new, slow_i, t.q, i, j, g, tag) || tag_ptype(tag) < 1000) return;
+            // not a neighbour of the forces; the filter counts its volume
+            g.v = 0;
+            t.b = mk4<R>(uxi, uyi, uzi, pi);
+            if constexpr (HEAT) t.s = tempi;
+        },
+        [&](int, const Rec& t, const PairV<R>& g) {
             const V4<R>& uj = t.b;
-            Disp<R> g;
-            R v;
-            int tag = 0;
-            const bool sl = pv_pair(P, S, rec.pos, W.m_new, W.rho_new, qi, slow_i, t.q, i, j, g, v, tag);
-            if (!sl) v = fabs(v);
+            const R v = g.v;
             const R r2 = g.dx * g.dx + g.dy * g.dy + g.dz * g.dz;
             const R rinv = rsq_floor(r2), r = r2 * rinv;
-            if (filt) flt += v * kws(K, r);
-            if (!adv || (sl && tag_ptype(tag) >= 1000)) return;
-            const R G = kg(K, r, rinv), vg = v * G;
+            if (filt) flt += g.vs * c2_w(K, r);
+            const R G = c2_g(K, r), vg = v * G;
             const R s = vg * (pi + uj.w);
             px += s * g.dx;
             py += s * g.dy;
@@ -1131,89 +1151,17 @@ __global__ void __launch_bounds__(128) k_passB(DevParams P, SphState<R> S, SphWo
             const R dux = uxi - uj.x, duy = uyi - uj.y, duz = uzi - uj.z;
             const Disp<R> y = cm6_mul(C, g.dx, g.dy, g.dz);
             const R quad = g.dx * y.dx + g.dy * y.dy + g.dz * y.dz;
-            R cv = cv_i;
-            if constexpr (FULL) {
-                if (P.sps && P.fv) {
-                    // harmonic mean of the two particles' viscosity + vis_t
-                    const R visj = vis + W.vist[j];
-                    cv = visi * visj / (visi + visj) * (R)4 * pori * irhoi;
-                }
-            }
             const R wd = w.dx * g.dx + w.dy * g.dy + w.dz * g.dz;
-            const R a = vg * (cv * quad * rinv * rinv + wd);
+            const R a = vg * (cv_i * quad * rinv * rinv + wd);
             tx += a * dux;
             ty += a * duy;
             tz += a * duz;
-            if constexpr (HEAT) {
-                R tj;
-                if constexpr (FULL) tj = t.a.z;
-                else tj = t.s;
-                et += vg * (ch_i * r * rcp(r + (R)1e-10) + wd) * (tempi - tj);
-            }
-            if constexpr (FULL) {
-                const R mj = t.a.x, rhoj = t.a.y, Gn = G * K.gn;
-                if (P.fva) {
-                    R uij = dux * g.dx + duy * g.dy + duz * g.dz;
-                    if (uij < (R)0) {
-                        R hij = (th + th) * (R)0.5;
-                        R phi = hij * uij / (r * r + (R)0.01 * hij * hij);
-                        R Pij = mi * phi * ((R)-0.1 * (R)P.soundspeed + (R)0.02 * phi) / (rhoi + rhoj) * (R)0.5;
-                        vx += -Pij * Gn * g.dx;
-                        vy += -Pij * Gn * g.dy;
-                        vz += -Pij * Gn * g.dz;
-                    }
-                }
-                const int ptj = tag_ptype(ldr(rec.pos + j).w);
-                R ax = 0, ay = 0, az = 0;
-                if (P.iface) {
-                    // interface sharpness force (functions_PPE2.cuh:1450-1464): raw
-                    // kernel slope; the neighbour's pressure only across a fluid-fluid
-                    // interface (wall 0 and moving 9 excluded)
-                    const bool flag = (pt != 0) && (pt != 9) && (ptj != 0) && (ptj != 9) && (pt != ptj);
-                    const R mri = mi * irhoi, mrj = v;
-                    R Ci = fabs(pi) * mri * mri + fabs(uj.w) * mrj * mrj * (R)flag;
-                    Ci *= ((R)0.08 / mi) * Gn;
-                    ax += Ci * -g.dx;
-                    ay += Ci * -g.dy;
-                    az += Ci * -g.dz;
-                }
-                if (P.fb && pt == 1 && ptj != 1) {
-                    // repulsive force of non-fluid neighbours (functions_PPE2.cuh:1465-1472)
-                    const R rr = r + (R)1e-10;
-                    const R fb = (R)P.c_repulsive / rr / rr * kw(K.k, r) * ((R)2 * mj / (mi + mj));
-                    ax += fb * g.dx;
-                    ay += fb * g.dy;
-                    az += fb * g.dz;
-                }
-                if (P.ipf && pt == 1 && ptj == 1) {
-                    // inter-particle surface tension (functions_PPE2.cuh:1490-1542): of the
-                    // pair strengths of Parameters.cuh:134-148 only fluid-fluid (s_ff1 =
-                    // 1.1e-6) is non-zero and every A is zero, so
-                    // Cs = -s_ff1 w_ipf / (m_i (r + 1e-10)) with the cosine kernel
-                    // w_ipf = -cos(3 pi / 4 r / h) for r < 2h (functions_INTERACTION.cuh:1-33)
-                    const R tR = r * rcp(th);
-                    const R wipf = tR < (R)2 ? -cos((R)(3.0 * 3.141592653 / 4.0) * tR) : (R)0;
-                    const R Cs = -((R)1.1e-6 * (wipf / (mi * (r + (R)1e-10))));
-                    ax += Cs * g.dx;
-                    ay += Cs * g.dy;
-                    az += Cs * g.dz;
-                }
-                fx += ax;
-                fy += ay;
-                fz += az;
-            }
+            if constexpr (HEAT) et += vg * (ch_i * r * rcp(r + (R)1e-10) + wd) * (tempi - t.s);
         });
     if (filt) S.flt_s[i] = flt * K.wn;
-    if (!adv) return;
     tx *= K.gn;
     ty *= K.gn;
     tz *= K.gn;
-    if constexpr (FULL) {
-        const Disp<R> a = cm6_mul(C, vx, vy, vz);
-        tx += a.dx + fx;
-        ty += a.dy + fy;
-        tz += a.dz + fz;
-    }
     if (P.fg) tz += -(R)P.g_sph;
     W.ftx[i] = tx;
     W.fty[i] = ty;
@@ -1829,25 +1777,33 @@ __global__ void __launch_bounds__(128) k_sph_coupling(DevParams P, SphState<R> S
         usz = uzi + ftz * b * dt;
     }
     S.ux[i] = usx; S.uy[i] = usy; S.uz[i] = usz;
-    const R pori = W.DEMpor[i];
-    W.rec.pu[i] = mk4<R>(pori * usx, pori * usy, pori * usz, S.pres[i]);
+    if (P.c2_passes) {
+        const R pori = W.DEMpor[i];
+        W.rec.pu[i] = mk4<R>(pori * usx, pori * usy, pori * usz, S.pres[i]);
+    } else {
+        W.rec.up[i] = mk4<R>(usx, usy, usz, S.pres[i]);
+    }
     if (time_zero) W.rho_ref[i] = W.rho_new[i];
     if (P.con && pt > 0) W.temp0[i] = S.temp[i];
 }
 
 // a wall's pressure and density into the state and the records of the passes
-// that follow (its pressure into {eps u*, p} before the pressure equation)
+// that follow (patch_p: its pressure too, before the pressure equation)
 template <typename R>
-__device__ __forceinline__ void wall_store(const SphState<R>& S, const SphWork<R>& W, R* pres, int i, R pw, R rw,
-                                           int patch_pu) {
+__device__ __forceinline__ void wall_store(const DevParams& P, const SphWork<R>& W, R* pres, int i, R pw, R rw,
+                                           int patch_p) {
     const SphRec<R> rec = W.rec;
     pres[i] = pw;
     W.rho_new[i] = rw;
     *comp<R>(rec.f1, i, 1) = rw;
-    pv_set_vol(rec.pb, i, pv_code<R>(*comp<R>(rec.f1, i, 0) / rw, ldr(rec.pos + i).w, false));
-    if (patch_pu) {
-        rec.rp[i] = rec.f1[i].w * rw;
-        *comp<R>(rec.pu, i, 3) = pw;
+    if (P.c2_passes) {
+        pv_set_vol(rec.pb, i, pv_code<R>(*comp<R>(rec.f1, i, 0) / rw, ldr(rec.pos + i).w, false));
+        if (patch_p) {
+            rec.rp[i] = rec.f1[i].w * rw;
+            *comp<R>(rec.pu, i, 3) = pw;
+        }
+    } else if (patch_p) {
+        *comp<R>(rec.up, i, 3) = pw;
     }
 }
 
@@ -1912,7 +1868,7 @@ __global__ void __launch_bounds__(128) k_neumann(DevParams P, SphState<R> S, Sph
         S.temp[i] = tt / flt;
         rw = rec.f1[i].w * tr / flt;
     }
-    wall_store<R>(S, W, pres, i, pw, rw, patch_up);
+    wall_store<R>(P, W, pres, i, pw, rw, patch_up);
 }
 
 // Cell-tiled Neumann pass (FP32 build): one warp per cell that holds wall
@@ -2109,7 +2065,7 @@ __device__ __forceinline__ void neumann_cell(int c, DevParams P, SphState<float>
             S.temp[i] = tt / flt;
             rw = rec.f1[i].w * tr / flt;
         }
-        wall_store<float>(S, W, pres, i, pw, rw, patch_up);
+        wall_store<float>(P, W, pres, i, pw, rw, patch_up);
     }
 }
 
@@ -2145,8 +2101,8 @@ __global__ void __launch_bounds__(NT_WARPS * 32, 8) k_neumann_tiled(DevParams P,
 // gradient correction: A_ij = -(eps_i rho_i + eps_j rho_j) / rho_i V G (d . C d) / r^2
 // and the divergence sum takes V G (eps_i u_i - eps_j u_j) . C d; eps u*, p and
 // eps rho come from their records, G's factor and 1 / rho_i leave the sums.
-template <typename R, int KT>
-__global__ void __launch_bounds__(128) k_ppe(DevParams P, SphState<R> S, SphWork<R> W) {
+template <typename R>
+__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 5 : 1) k_ppe(DevParams P, SphState<R> S, SphWork<R> W) {
     grid_dep_wait();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     int n = P.ns;
@@ -2160,7 +2116,7 @@ __global__ void __launch_bounds__(128) k_ppe(DevParams P, SphState<R> S, SphWork
     }
     const V4<R> pui = rec.pu[i];
     R th = (R)S.h[i];
-    const KnlSum<R, KT> K = knl_sum<R, KT>(P, th);
+    const C2Sum<R> K = c2_sum<R>(P, th);
     const PvRec<R> qi = ldr(rec.pb + i);
     const bool slow_i = pv_vol(qi) != pv_vol(qi);
     const R prhoi = rec.rp[i];
@@ -2168,7 +2124,7 @@ __global__ void __launch_bounds__(128) k_ppe(DevParams P, SphState<R> S, SphWork
     int cnt = min(W.ncnt[i], P.nb_cap);
     R b = 0, A = 0, AP = 0;
     const int* __restrict__ nb = W.nbr;
-    nb_walk<4, NbP4S<R>>(
+    nb_sum<NbP4S<R>, PairV<R>>(
         cnt, nb, n, i,
         [&](int j) {
             NbP4S<R> t;
@@ -2177,18 +2133,21 @@ __global__ void __launch_bounds__(128) k_ppe(DevParams P, SphState<R> S, SphWork
             t.s = ldr(rec.rp + j);
             return t;
         },
-        [&](int j, const NbP4S<R>& t) {
-            Disp<R> g;
-            R v;
+        [&](const NbP4S<R>& t, PairV<R>& g) { return pv_prep<R, false>(P, qi, slow_i, t.q, g); },
+        [&](int j, NbP4S<R>& t, PairV<R>& g) {
             int tag;
-            if (pv_pair(P, S, rec.pos, W.m_new, W.rho_new, qi, slow_i, t.q, i, j, g, v, tag)) {
-                if (tag_ptype(tag) >= 1000 || tag_itype(tag) == 4) return;
-            } else {
-                v = fabs(v);
+            if (!pv_fix(S, rec.pos, W.m_new, W.rho_new, slow_i, t.q, i, j, g, tag)) return;
+            if (tag_ptype(tag) >= 1000 || tag_itype(tag) == 4) {   // no neighbour of this sum
+                g.v = 0;
+                t.b = pui;
+                t.s = prhoi;
             }
+        },
+        [&](int, const NbP4S<R>& t, const PairV<R>& g) {
             const R r2 = g.dx * g.dx + g.dy * g.dy + g.dz * g.dz;
             const R rinv = rsq_floor(r2), r = r2 * rinv;
-            const R vg = v * kg(K, r, rinv);
+            const R v = g.v;
+            const R vg = v * c2_g(K, r);
             const Disp<R> y = cm6_mul(C, g.dx, g.dy, g.dz);
             b += vg * ((pui.x - t.b.x) * y.dx + (pui.y - t.b.y) * y.dy + (pui.z - t.b.z) * y.dz);
             const R quad = g.dx * y.dx + g.dy * y.dy + g.dz * y.dz;
@@ -2205,8 +2164,8 @@ __global__ void __launch_bounds__(128) k_ppe(DevParams P, SphState<R> S, SphWork
 // pass C: KERNEL_pressureforce3D_sph (functions_PPE2.cuh:2154-2335) and
 // KERNEL_time_update_projection_sph (functions_TIME_ISPH2.cuh:467-620).
 // ---------------------------------------------------------------------------
-template <typename R, int KT>
-__global__ void __launch_bounds__(128) k_passC(DevParams P, SphState<R> S, SphWork<R> W) {
+template <typename R>
+__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 7 : 1) k_passC(DevParams P, SphState<R> S, SphWork<R> W) {
     grid_dep_wait();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     int n = P.ns;
@@ -2223,14 +2182,14 @@ __global__ void __launch_bounds__(128) k_passC(DevParams P, SphState<R> S, SphWo
     if (pf && P.fp) {
         // sum of V (p_i + p_j) G d; the gradient correction and the factors after it
         R th = (R)S.h[i];
-        const KnlSum<R, KT> K = knl_sum<R, KT>(P, th);
+        const C2Sum<R> K = c2_sum<R>(P, th);
         const PvRec<R> qi = ldr(rec.pb + i);
         const bool slow_i = pv_vol(qi) != pv_vol(qi);
         const R pi = W.p_new[i];
         int cnt = min(W.ncnt[i], P.nb_cap);
         const int* __restrict__ nb = W.nbr;
         const R* __restrict__ pn = W.p_new;
-        nb_walk<4, NbPS<R>>(
+        nb_sum<NbPS<R>, PairV<R>>(
             cnt, nb, n, i,
             [&](int j) {
                 NbPS<R> t;
@@ -2238,18 +2197,20 @@ __global__ void __launch_bounds__(128) k_passC(DevParams P, SphState<R> S, SphWo
                 t.s = ldr(pn + j);
                 return t;
             },
-            [&](int j, const NbPS<R>& t) {
-                Disp<R> g;
-                R v;
+            [&](const NbPS<R>& t, PairV<R>& g) { return pv_prep<R, false>(P, qi, slow_i, t.q, g); },
+            [&](int j, NbPS<R>& t, PairV<R>& g) {
                 int tag;
-                if (pv_pair(P, S, rec.pos, W.m_new, W.rho_new, qi, slow_i, t.q, i, j, g, v, tag)) {
-                    if (tag_ptype(tag) >= 1000) return;
-                } else {
-                    v = fabs(v);
+                if (!pv_fix(S, rec.pos, W.m_new, W.rho_new, slow_i, t.q, i, j, g, tag)) return;
+                if (tag_ptype(tag) >= 1000) {   // no neighbour of this sum
+                    g.v = 0;
+                    t.s = pi;
                 }
+            },
+            [&](int, const NbPS<R>& t, const PairV<R>& g) {
+                const R v = g.v;
                 const R r2 = g.dx * g.dx + g.dy * g.dy + g.dz * g.dz;
                 const R rinv = rsq_floor(r2), r = r2 * rinv;
-                const R s = v * kg(K, r, rinv) * (pi + t.s);
+                const R s = v * c2_g(K, r) * (pi + t.s);
                 fx += s * g.dx;
                 fy += s * g.dy;
                 fz += s * g.dz;
@@ -2518,7 +2479,7 @@ __global__ void __launch_bounds__(128) k_open_bc(DevParams P, SphState<R> S, Sph
     // the XSPH pass reads buffer particles through the records
     *comp<R>(W.rec.f1, i, 0) = mn;
     *comp<R>(W.rec.f1, i, 1) = rn;
-    pv_set_vol(W.rec.pb, i, pv_code<R>(mn / rn, ldr(W.rec.pos + i).w, S.ptype[i] == 1 || S.ptype[i] == 3));
+    if (P.c2_passes) pv_set_vol(W.rec.pb, i, pv_code<R>(mn / rn, ldr(W.rec.pos + i).w, S.ptype[i] == 1 || S.ptype[i] == 3));
     W.rec.ut[i] = mk4<R>(ux, uy, uz, tn);
 }
 
@@ -2527,7 +2488,7 @@ __global__ void __launch_bounds__(128) k_open_bc(DevParams P, SphState<R> S, Sph
 // Writes the smoothed velocity/temperature of every particle (or a copy)
 // into u_tmp/temp_tmp; the next reorder reads them.
 // ---------------------------------------------------------------------------
-template <typename R, int KT>
+template <typename R>
 __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 6 : 1) k_xsph(DevParams P, SphState<R> S, SphWork<R> W) {
     grid_dep_wait();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2542,7 +2503,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 6 : 1) k_xsph(DevParams 
         return;
     }
     R th = (R)S.h[i];
-    const KnlSum<R, KT> K = knl_sum<R, KT>(P, th);
+    const C2Sum<R> K = c2_sum<R>(P, th);
     const PvRec<R> qi = ldr(rec.pb + i);
     const bool slow_i = pv_vol(qi) != pv_vol(qi);
     R c = (R)P.c_xsph;
@@ -2550,7 +2511,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 6 : 1) k_xsph(DevParams 
     // the kernel's normalisation leaves the ratios below
     R tx = 0, ty = 0, tz = 0, tt = 0, flt = 0;
     const int* __restrict__ nb = W.nbr;
-    nb_walk<4, NbP4<R>>(
+    nb_sum<NbP4<R>, PairV<R>>(
         cnt, nb, n, i,
         [&](int j) {
             NbP4<R> t;
@@ -2558,22 +2519,25 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 6 : 1) k_xsph(DevParams 
             t.b = ldr(rec.ut + j);
             return t;
         },
-        [&](int j, const NbP4<R>& t) {
-            Disp<R> g;
-            R v;
+        [&](const NbP4<R>& t, PairV<R>& g) { return pv_prep<R, true>(P, qi, slow_i, t.q, g); },
+        [&](int j, NbP4<R>& t, PairV<R>& g) {
             int tag;
-            if (pv_pair(P, S, rec.pos, W.m_new, W.rho_new, qi, slow_i, t.q, i, j, g, v, tag)) {
-                if (tag_ptype(tag) != 1 && tag_ptype(tag) != 3) return;
-            } else if (!(v > (R)0)) {
-                return;
+            if (!pv_fix(S, rec.pos, W.m_new, W.rho_new, slow_i, t.q, i, j, g, tag)) return;
+            if (tag_ptype(tag) != 1 && tag_ptype(tag) != 3) {   // no neighbour of this sum
+                g.vs = 0;
+                t.b = ui;
             }
+        },
+        [&](int, const NbP4<R>& t, const PairV<R>& g) {
+            const R v = g.vs;
+            const bool in = v > (R)0;   // a wall's fields stay out of the sums
             const R r2 = g.dx * g.dx + g.dy * g.dy + g.dz * g.dz;
             const R r = r2 * rsq_floor(r2);
-            const R m = v * kws(K, r);
-            tx += m * (t.b.x - uxi);
-            ty += m * (t.b.y - uyi);
-            tz += m * (t.b.z - uzi);
-            tt += m * (t.b.w - ti);
+            const R m = v * c2_w(K, r);
+            tx += m * (in ? t.b.x - uxi : (R)0);
+            ty += m * (in ? t.b.y - uyi : (R)0);
+            tz += m * (in ? t.b.z - uzi : (R)0);
+            tt += m * (in ? t.b.w - ti : (R)0);
             flt += m;
         });
     R on = (R)(pt > 0);
@@ -2582,6 +2546,503 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 6 : 1) k_xsph(DevParams 
     W.u_tmpy[i] = (uyi + ty * iflt) * on;
     W.u_tmpz[i] = (uzi + tz * iflt) * on;
     W.temp_tmp[i] = (ti + (R)0.01 * tt * iflt) * on;
+}
+
+// ---------------------------------------------------------------------------
+// The neighbour passes for any kernel and switch set (the passes above their
+// own Wendland C2 forms).
+// ---------------------------------------------------------------------------
+// the planes xx, xy, xz, yy, yz, zz of the symmetric 3 x 3 matrix C
+template <typename R>
+__device__ __forceinline__ void cm_store(R* Cm, int n, int i, const R* C) {
+    Cm[i] = C[0];
+    Cm[(size_t)n + i] = C[1];
+    Cm[(size_t)2 * n + i] = C[2];
+    Cm[(size_t)3 * n + i] = C[4];
+    Cm[(size_t)4 * n + i] = C[5];
+    Cm[(size_t)5 * n + i] = C[8];
+}
+template <typename R>
+__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 8 : 1) k_passA_any(DevParams P, SphState<R> S, SphWork<R> W, DemState<double> D,
+                                               const int4* __restrict__ drows) {
+    grid_dep_wait();
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    int n = P.ns;
+    if (i >= n) return;
+    const SphRec<R> rec = W.rec;
+    int it = S.itype[i], pt = S.ptype[i];
+    R mo = S.m[i], ro = S.rho[i];
+    if (it > 2) {
+        W.m_new[i] = mo;
+        W.rho_new[i] = ro;
+        rec.f1[i] = mk4<R>(mo, ro, S.temp[i], W.DEMpor[i]);
+        return;
+    }
+    R dprev = S.dDEMpor[i];
+    W.dDEMpor_prev[i] = dprev;
+    double xi = S.x[i], yi = S.y[i], zi = S.z[i], hi = S.h[i];
+    R th = (R)hi;
+    Knl<R> K = knl_make<R>(P, th);
+    PosRec<R> qi = ldr(rec.pos + i);
+    int cnt = min(W.ncnt[i], P.nb_cap);
+    R txx = 0, tyy = 0, tzz = 0, txy = 0, tyz = 0, tzx = 0, sflt = 0;
+    const int* __restrict__ nb = W.nbr;
+    const bool kgc = (P.kgc == 1);
+    nb_walk<4, NbQ2<R>>(
+        cnt, nb, n, i,
+        [&](int j) {
+            NbQ2<R> t;
+            t.q = ldr(rec.pos + j);
+            t.a = ldr(rec.mr0 + j);
+            return t;
+        },
+        [&](int j, const NbQ2<R>& t) {
+            int ptj = tag_ptype(t.q.w);
+            if (ptj > 1000) return;
+            Disp<R> g = disp(P, qi, t.q, S.x, S.y, S.z, i, j);
+            R r2 = g.dx * g.dx + g.dy * g.dy + g.dz * g.dz, r, rinv;
+            rdist(r2, r, rinv);
+            R irj = rcp(t.a.y);
+            if (ptj == 1) sflt += t.a.x * irj * kw(K, r);
+            if (kgc && r2 > (R)0) {
+                R dw = kdw(K, r);
+                R c = -t.a.x * dw * irj * rinv;
+                txx += c * g.dx * g.dx;
+                txy += c * g.dy * g.dx;
+                tyy += c * g.dy * g.dy;
+                tzx += c * g.dx * g.dz;
+                tyz += c * g.dy * g.dz;
+                tzz += c * g.dz * g.dz;
+            }
+        });
+    if (kgc && P.dim == 2) {
+        // a bed in a plane y = const: the x-z block of the moment matrix
+        const R det = txx * tzz - tzx * tzx;
+        R C[9] = {1, 0, 0, 0, 1, 0, 0, 0, 1};
+        if (fabs(det) > (R)1e-4) {
+            const R rr = (R)1 / det;
+            C[0] = tzz * rr;
+            C[2] = -tzx * rr;
+            C[6] = -tzx * rr;
+            C[8] = txx * rr;
+        }
+        cm_store(W.Cm, n, i, C);
+    } else if (kgc) {
+        R det = txx * (tyy * tzz - tyz * tyz);
+        det -= txy * (txy * tzz - tyz * tzx);
+        det += tzx * (txy * tyz - tyy * tzx);
+        R C[9];
+        if (fabs(det) > (R)1e-4) {
+            R rr = (R)1 / det;
+            C[0] = (tyy * tzz - tyz * tyz) * rr;
+            C[1] = (tzx * tyz - txy * tzz) * rr;
+            C[2] = (txy * tyz - tzx * tyy) * rr;
+            C[3] = (tzx * tyz - txy * tzz) * rr;
+            C[4] = (txx * tzz - tzx * tzx) * rr;
+            C[5] = (tzx * txy - txx * tyz) * rr;
+            C[6] = (txy * tyz - tzx * tyy) * rr;
+            C[7] = (tzx * txy - txx * tyz) * rr;
+            C[8] = (txx * tyy - txy * txy) * rr;
+        } else {
+            C[0] = 1; C[1] = 0; C[2] = 0; C[3] = 0; C[4] = 1; C[5] = 0; C[6] = 0; C[7] = 0; C[8] = 1;
+        }
+        cm_store(W.Cm, n, i, C);
+    }
+    // SPH-DEM porosity over the SPH -> DEM list (DEM arrays are small and
+    // L2-resident: plain loads)
+    double Rr = P.kappa * hi;
+    R por = 0, dfx = 0, dfy = 0, dfz = 0;
+    if (P.nd > 0) {
+        float r2l = r2_lo(Rr), r2h = r2_hi(Rr);
+        auto dem = [&](int j) {
+            if (D.ptype[j] <= 1000) return;
+            PairT<R> g = pair_test<R>(xi, yi, zi, D.x[j], D.y[j], D.z[j], Rr, 1e-20, r2l, r2h);
+            if (!g.in) return;
+            R r = g.r + (R)1e-20, ir = rcp(r);
+            R w = kw(K, r);
+            R dw = kdw(K, r);
+            R rj = (R)D.rad[j];
+            R v = dem_measure(P, rj);
+            por += w * v;
+            dfx += dw * g.dx * ir * (R)D.ux[j] * v;
+            dfy += dw * g.dy * ir * (R)D.uy[j] * v;
+            dfz += dw * g.dz * ir * (R)D.uz[j] * v;
+        };
+        const int cd = W.ncntd[i];
+        if (cd <= P.nbd_cap) {
+            for (int k = 0; k < cd; k++) dem(W.nbrd[(size_t)k * n + i]);
+        } else {
+            int ic, jc, kc;
+            cell_ijk(P, xi, yi, zi, ic, jc, kc);
+            for_stencil_j(P, ic, jc, kc, drows, make_cull(xi, yi, zi, Rr), dem);
+        }
+    }
+    R isf = rcp(sflt + (R)1e-20);
+    R pori = (R)1 - por * isf;
+    W.DEMpor[i] = pori;
+    S.dDEMpor[i] = (dfx + dfy + dfz) * isf;
+    // prep_sph
+    R hd = (R)P.h_over_dx;
+    R v = sph_volume(P, th, hd);
+    R mref;
+    if (pt == 9) mref = (R)P.rho_liquid * v * pori;
+    else if (pt == -3 || pt == 0 || pt == 3 || pt == 1) mref = (R)P.rho_gas * v * pori;
+    else mref = (R)P.rho_liquid * v * pori;
+    if (pt == 9 && zi < 0.05) mref = (R)P.rho_gas * v * pori;
+    R rref = (P.dim == 2) ? mref / ((th / hd) * (th / hd)) : mref / v;
+    W.rho_ref[i] = rref;
+    R mn = mo, rn = ro;
+    if (P.rho_type == 1) {
+        rn = mref / v;
+        mn = mref;
+    }
+    W.rho_new[i] = rn;
+    W.m_new[i] = mn;
+    rec.f1[i] = mk4<R>(mn, rn, S.temp[i], pori);
+}
+
+template <typename R, bool FORCES>
+__global__ void __launch_bounds__(128) k_passB_any(DevParams P, SphState<R> S, SphWork<R> W, const DevFlags* F) {
+    grid_dep_wait();
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    int n = P.ns;
+    if (i >= n) return;
+    const SphRec<R> rec = W.rec;
+    // Shepard filter every freq_filt*decouple_stride steps (functions_PREP2.cuh:2120)
+    const int filt = (F->step_count % P.filt_period) == 0;
+    int it = S.itype[i], pt = S.ptype[i], bt = S.btype[i];
+    W.ftx[i] = 0; W.fty[i] = 0; W.ftz[i] = 0; W.ftot[i] = 0;
+    W.pgfx[i] = 0; W.pgfy[i] = 0; W.pgfz[i] = 0;
+    W.dtemp[i] = 0;
+    if (it > 2 || pt > 1000) return;
+    bool adv = !(P.open_bc > 0 && bt > 0) && pt < 1000 && pt > 0;
+    if (!filt && !adv) return;
+    R th = (R)S.h[i];
+    Knl<R> K = knl_make<R>(P, th);
+    PosRec<R> qi = ldr(rec.pos + i);
+    V4<R> upi = rec.up[i];
+    V4<R> fi = rec.f1[i];
+    R uxi = upi.x, uyi = upi.y, uzi = upi.z, pi = upi.w;
+    R rhoi = fi.y, tempi = fi.z, pori = fi.w, mi = fi.x;
+    R irhoi = rcp(rhoi);
+    const bool kgc = (P.kgc == 1);
+    Cm9<R> Cm = cm_load(W.Cm, n, i, kgc);
+    R vis = (R)P.mu_gas, vis_h = (vis * vis) / (vis + vis);
+    R kc = (R)P.k_sph;
+    R eli = (P.sph_lagrangian != 0) ? (R)1 : (R)0;
+    // per-particle factors of the pair terms
+    R cp_i = -pori * irhoi * (rhoi / pori);      // rho_i/eps_i * (-eps_i / rho_i)
+    R cv_i = vis_h * (R)4 * pori * irhoi;
+    R visi = vis;
+    if (FORCES && P.sps) visi += W.vist[i];   // viscosity + P3.vis_t (functions_PPE2.cuh:1323)
+    R ch_i = (R)4 * pori * kc * kc * irhoi / (kc + kc);
+    int cnt = min(W.ncnt[i], P.nb_cap);
+    R flt = 0, tx = 0, ty = 0, tz = 0, px = 0, py = 0, pz = 0, Rc = 0, ex = 0, ey = 0, ez = 0, et = 0;
+    const int* __restrict__ nb = W.nbr;
+    nb_walk<4, NbQ44<R>>(
+        cnt, nb, n, i,
+        [&](int j) {
+            NbQ44<R> t;
+            t.q = ldr(rec.pos + j);
+            t.a = ldr(rec.f1 + j);
+            t.b = ldr(rec.up + j);
+            return t;
+        },
+        [&](int j, const NbQ44<R>& t) {
+            const V4<R>& fj = t.a;
+            const V4<R>& uj = t.b;
+            Disp<R> g = disp(P, qi, t.q, S.x, S.y, S.z, i, j);
+            R r2 = g.dx * g.dx + g.dy * g.dy + g.dz * g.dz, r, rinv;
+            rdist(r2, r, rinv);
+            R mj = fj.x, irj = rcp(fj.y);
+            if (filt) flt += mj * irj * kw(K, r);
+            if (!adv || tag_ptype(t.q.w) >= 1000) return;
+            R dw = kdw(K, r);
+            R gx = dw * g.dx * rinv, gy = dw * g.dy * rinv, gz = dw * g.dz * rinv;
+            cm_apply(Cm, kgc, gx, gy, gz);
+            R tj = fj.z;
+            if ((P.fp != 0)) {
+                R s = cp_i * mj * (pi + uj.w) * irj;
+                px += s * gx;
+                py += s * gy;
+                pz += s * gz;
+            }
+            if ((P.fv != 0)) {
+                R cv = cv_i;
+                if (FORCES && P.sps) {
+                    // harmonic mean of the two particles' viscosity + vis_t
+                    const R visj = vis + W.vist[j];
+                    cv = visi * visj / (visi + visj) * (R)4 * pori * irhoi;
+                }
+                R Cv = (g.dx * gx + g.dy * gy + g.dz * gz) * cv * mj * irj * rinv * rinv;
+                tx += Cv * (uxi - uj.x);
+                ty += Cv * (uyi - uj.y);
+                tz += Cv * (uzi - uj.z);
+            }
+            if ((P.fva != 0)) {
+                R uij = (uxi - uj.x) * g.dx + (uyi - uj.y) * g.dy + (uzi - uj.z) * g.dz;
+                if (uij < (R)0) {
+                    R hij = (th + th) * (R)0.5;
+                    R phi = hij * uij / (r * r + (R)0.01 * hij * hij);
+                    R Pij = mi * phi * ((R)-0.1 * (R)P.soundspeed + (R)0.02 * phi) / (rhoi + fj.y) * (R)0.5;
+                    tx += -Pij * gx;
+                    ty += -Pij * gy;
+                    tz += -Pij * gz;
+                }
+            }
+            if (FORCES) {
+                const int ptj = tag_ptype(t.q.w);
+                if (P.iface) {
+                    // interface sharpness force (functions_PPE2.cuh:1450-1464): raw
+                    // kernel slope; the neighbour's pressure only across a fluid-fluid
+                    // interface (wall 0 and moving 9 excluded)
+                    const bool flag = (pt != 0) && (pt != 9) && (ptj != 0) && (ptj != 9) && (pt != ptj);
+                    const R mri = mi * irhoi, mrj = mj * irj;
+                    R Ci = fabs(pi) * mri * mri + fabs(uj.w) * mrj * mrj * (R)flag;
+                    Ci *= ((R)0.08 / mi) * dw * rinv;
+                    tx += Ci * -g.dx;
+                    ty += Ci * -g.dy;
+                    tz += Ci * -g.dz;
+                }
+                if (P.fb && pt == 1 && ptj != 1) {
+                    // repulsive force of non-fluid neighbours (functions_PPE2.cuh:1465-1472)
+                    const R rr = r + (R)1e-10;
+                    const R fb = (R)P.c_repulsive / rr / rr * kw(K, r) * ((R)2 * mj / (mi + mj));
+                    tx += fb * g.dx;
+                    ty += fb * g.dy;
+                    tz += fb * g.dz;
+                }
+                if (P.ipf && pt == 1 && ptj == 1) {
+                    // inter-particle surface tension (functions_PPE2.cuh:1490-1542): of the
+                    // pair strengths of Parameters.cuh:134-148 only fluid-fluid (s_ff1 =
+                    // 1.1e-6) is non-zero and every A is zero, so
+                    // Cs = -s_ff1 w_ipf / (m_i (r + 1e-10)) with the cosine kernel
+                    // w_ipf = -cos(3 pi / 4 r / h) for r < 2h (functions_INTERACTION.cuh:1-33)
+                    const R tR = r * rcp(th);
+                    const R wipf = tR < (R)2 ? -cos((R)(3.0 * 3.141592653 / 4.0) * tR) : (R)0;
+                    const R Cs = -((R)1.1e-6 * (wipf / (mi * (r + (R)1e-10))));
+                    tx += Cs * g.dx;
+                    ty += Cs * g.dy;
+                    tz += Cs * g.dz;
+                }
+            }
+            if (eli < (R)1) {
+                R mr = mj * irj * ((R)1 - eli);
+                R ug = uxi * gx + uyi * gy + uzi * gz;
+                ex += (uj.x - uxi) * ug * mr;
+                ey += (uj.y - uyi) * ug * mr;
+                ez += (uj.z - uzi) * ug * mr;
+                if ((P.con != 0)) et += (tj - tempi) * ug * mr;
+            }
+            if ((P.con != 0)) Rc += ch_i * mj * (tempi - tj) * dw * irj * rcp(r + (R)1e-10);
+        });
+    if (filt) S.flt_s[i] = flt;
+    if (!adv) return;
+    if (P.fg) tz += -(R)P.g_sph;
+    W.ftx[i] = tx - ex;
+    W.fty[i] = ty - ey;
+    W.ftz[i] = tz - ez;
+    W.ftot[i] = sqrt(tx * tx + ty * ty + tz * tz);
+    W.pgfx[i] = px;
+    W.pgfy[i] = py;
+    W.pgfz[i] = pz;
+    if ((P.con != 0)) W.dtemp[i] = Rc / (R)P.cp_sph * (R)(pt != -1) - et;
+}
+
+template <typename R>
+__global__ void __launch_bounds__(128) k_ppe_any(DevParams P, SphState<R> S, SphWork<R> W) {
+    grid_dep_wait();
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    int n = P.ns;
+    if (i >= n) return;
+    const SphRec<R> rec = W.rec;
+    int it = S.itype[i], pt = S.ptype[i], bt = S.btype[i];
+    V4<R> upi = rec.up[i];
+    bool solve = it <= 2 && !(P.open_bc > 0 && bt > 0) && pt < 1000 && pt > 0;
+    if (!solve) {
+        W.p_new[i] = upi.w;
+        return;
+    }
+    R th = (R)S.h[i];
+    Knl<R> K = knl_make<R>(P, th);
+    PosRec<R> qi = ldr(rec.pos + i);
+    V4<R> fi = rec.f1[i];
+    R uxi = upi.x, uyi = upi.y, uzi = upi.z, rhoi = fi.y, pori = fi.w;
+    R irhoi = rcp(rhoi), prhoi = pori * rhoi;
+    R pux = pori * uxi, puy = pori * uyi, puz = pori * uzi;
+    const bool kgc = (P.kgc == 1);
+    Cm9<R> Cm = cm_load(W.Cm, n, i, kgc);
+    int cnt = min(W.ncnt[i], P.nb_cap);
+    R bx = 0, by = 0, bz = 0, A = 0, AP = 0;
+    const int* __restrict__ nb = W.nbr;
+    nb_walk<4, NbQ44<R>>(
+        cnt, nb, n, i,
+        [&](int j) {
+            NbQ44<R> t;
+            t.q = ldr(rec.pos + j);
+            t.a = ldr(rec.f1 + j);
+            t.b = ldr(rec.up + j);
+            return t;
+        },
+        [&](int j, const NbQ44<R>& t) {
+            int tj = t.q.w;
+            if (tag_ptype(tj) >= 1000 || tag_itype(tj) == 4) return;
+            const V4<R>& fj = t.a;
+            const V4<R>& uj = t.b;
+            Disp<R> g = disp(P, qi, t.q, S.x, S.y, S.z, i, j);
+            R r2 = g.dx * g.dx + g.dy * g.dy + g.dz * g.dz, r, rinv;
+            rdist(r2, r, rinv);
+            R mj = fj.x, rhoj = fj.y, porj = fj.w, irj = rcp(rhoj);
+            R dw = kdw(K, r);
+            R gx = dw * g.dx * rinv, gy = dw * g.dy * rinv, gz = dw * g.dz * rinv;
+            cm_apply(Cm, kgc, gx, gy, gz);
+            R mr = mj * irj;
+            bx += mr * (pux - porj * uj.x) * gx;
+            by += mr * (puy - porj * uj.y) * gy;
+            bz += mr * (puz - porj * uj.z) * gz;
+            R c = -(g.dx * gx + g.dy * gy + g.dz * gz) * rinv * rinv;
+            R a = mj * ((prhoi + porj * rhoj) * irj * irhoi) * c;
+            A += a;
+            AP += a * uj.w;
+        });
+    R b = (R)P.rho_gas * (bx + by + bz + (R)2 * S.dDEMpor[i] - W.dDEMpor_prev[i]) / (R)P.sdt;
+    W.p_new[i] = (b + AP) / A;
+}
+
+template <typename R>
+__global__ void __launch_bounds__(128) k_passC_any(DevParams P, SphState<R> S, SphWork<R> W) {
+    grid_dep_wait();
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    int n = P.ns;
+    if (i >= n) return;
+    const SphRec<R> rec = W.rec;
+    int it = S.itype[i], pt = S.ptype[i], bt = S.btype[i];
+    W.fpx[i] = 0; W.fpy[i] = 0; W.fpz[i] = 0;
+    if (it > 2) {
+        rec.ut[i] = mk4<R>(S.ux[i], S.uy[i], S.uz[i], S.temp[i]);
+        return;
+    }
+    R fx = 0, fy = 0, fz = 0;
+    bool pf = !(P.open_bc > 0 && bt > 0) && pt < 1000 && pt > 0;
+    if (pf && (P.fp != 0)) {
+        R th = (R)S.h[i];
+        Knl<R> K = knl_make<R>(P, th);
+        PosRec<R> qi = ldr(rec.pos + i);
+        R pi = W.p_new[i], rhoi = W.rho_new[i], pori = rec.f1[i].w;
+        R cpi = -pori * rcp(rhoi);
+        const bool kgc = (P.kgc == 1);
+        Cm9<R> Cm = cm_load(W.Cm, n, i, kgc);
+        int cnt = min(W.ncnt[i], P.nb_cap);
+        const int* __restrict__ nb = W.nbr;
+        const R* __restrict__ pn = W.p_new;
+        nb_walk<4, NbQ2S<R>>(
+            cnt, nb, n, i,
+            [&](int j) {
+                NbQ2S<R> t;
+                t.q = ldr(rec.pos + j);
+                t.a = ldr(reinterpret_cast<const V2<R>*>(rec.f1 + j));
+                t.s = __ldg(pn + j);
+                return t;
+            },
+            [&](int j, const NbQ2S<R>& t) {
+                if (tag_ptype(t.q.w) >= 1000) return;
+                Disp<R> g = disp(P, qi, t.q, S.x, S.y, S.z, i, j);
+                R r2 = g.dx * g.dx + g.dy * g.dy + g.dz * g.dz, r, rinv;
+                rdist(r2, r, rinv);
+                R dw = kdw(K, r);
+                R gx = dw * g.dx * rinv, gy = dw * g.dy * rinv, gz = dw * g.dz * rinv;
+                cm_apply(Cm, kgc, gx, gy, gz);
+                R Cp = cpi * t.a.x * (pi + t.s) * rcp(t.a.y);
+                fx += Cp * gx;
+                fy += Cp * gy;
+                fz += Cp * gz;
+            });
+        W.fpx[i] = fx; W.fpy[i] = fy; W.fpz[i] = fz;
+    }
+    if (pt == 9) {
+        rec.ut[i] = mk4<R>(S.ux[i], S.uy[i], S.uz[i], S.temp[i]);
+        return;
+    }
+    R ux0, uy0, uz0, ax, ay, az;
+    if (pt > 0) {
+        ux0 = S.ux[i]; uy0 = S.uy[i]; uz0 = S.uz[i];
+        R b = (R)(bt == 0);
+        ax = fx * b; ay = fy * b; az = fz * b;
+    } else {
+        ux0 = W.ux0[i]; uy0 = W.uy0[i]; uz0 = W.uz0[i];
+        ax = ay = az = (R)0;
+    }
+    R dt = (R)P.sdt;
+    R uxc = ux0 + ax * dt, uyc = uy0 + ay * dt, uzc = uz0 + az * dt;
+    R lim = (R)P.u_limit;
+    if ((uxc * uxc + uyc * uyc + uzc * uzc) >= lim * lim) {
+        uxc = ux0; uyc = uy0; uzc = uz0;
+    }
+    if (!P.xsph && (P.sph_lagrangian != 0) && pt > 0) {
+        S.x[i] += ((double)W.ux0[i] + (double)uxc) / 2.0 * P.sdt;
+        S.y[i] += ((double)W.uy0[i] + (double)uyc) / 2.0 * P.sdt;
+        S.z[i] += ((double)W.uz0[i] + (double)uzc) / 2.0 * P.sdt;
+    }
+    S.ux[i] = uxc; S.uy[i] = uyc; S.uz[i] = uzc;
+    R tn = S.temp[i];
+    if ((P.con != 0) && pt > 0) {
+        tn = W.temp0[i] + W.dtemp[i] * dt * (R)(pt != -1);
+        S.temp[i] = tn;
+    }
+    rec.ut[i] = mk4<R>(uxc, uyc, uzc, tn);
+}
+
+template <typename R>
+__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 6 : 1) k_xsph_any(DevParams P, SphState<R> S, SphWork<R> W) {
+    grid_dep_wait();
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    int n = P.ns;
+    if (i >= n) return;
+    const SphRec<R> rec = W.rec;
+    int it = S.itype[i], pt = S.ptype[i];
+    V4<R> ui = rec.ut[i];
+    R uxi = ui.x, uyi = ui.y, uzi = ui.z, ti = ui.w;
+    if (it != 1 || pt > 1000 || pt == 0 || pt == 9) {
+        W.u_tmpx[i] = uxi; W.u_tmpy[i] = uyi; W.u_tmpz[i] = uzi; W.temp_tmp[i] = ti;
+        return;
+    }
+    R th = (R)S.h[i];
+    Knl<R> K = knl_make<R>(P, th);
+    PosRec<R> qi = ldr(rec.pos + i);
+    R c = (R)P.c_xsph;
+    int cnt = min(W.ncnt[i], P.nb_cap);
+    R tx = 0, ty = 0, tz = 0, tt = 0, flt = 0;
+    const int* __restrict__ nb = W.nbr;
+    nb_walk<4, NbQ24<R>>(
+        cnt, nb, n, i,
+        [&](int j) {
+            NbQ24<R> t;
+            t.q = ldr(rec.pos + j);
+            t.a = ldr(reinterpret_cast<const V2<R>*>(rec.f1 + j));
+            t.b = ldr(rec.ut + j);
+            return t;
+        },
+        [&](int j, const NbQ24<R>& t) {
+            int ptj = tag_ptype(t.q.w);
+            if (ptj != 1 && ptj != 3) return;
+            Disp<R> g = disp(P, qi, t.q, S.x, S.y, S.z, i, j);
+            R r2 = g.dx * g.dx + g.dy * g.dy + g.dz * g.dz, r, rinv;
+            rdist(r2, r, rinv);
+            R w = kw(K, r);
+            R m = t.a.x * rcp(t.a.y) * w;
+            R cm = c * m;
+            tx += cm * (t.b.x - uxi);
+            ty += cm * (t.b.y - uyi);
+            tz += cm * (t.b.z - uzi);
+            tt += (R)0.01 * cm * (t.b.w - ti);
+            flt += m;
+        });
+    R on = (R)(pt > 0);
+    R iflt = rcp(flt);
+    W.u_tmpx[i] = (uxi + tx * iflt) * on;
+    W.u_tmpy[i] = (uyi + ty * iflt) * on;
+    W.u_tmpz[i] = (uzi + tz * iflt) * on;
+    W.temp_tmp[i] = (ti + tt * iflt) * on;
 }
 
 // end of a step: the host loop's count++ (ISPH_Calc_seperate.cuh:925)
