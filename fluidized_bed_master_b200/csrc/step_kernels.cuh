@@ -186,6 +186,32 @@ __global__ void k_cells_gather_sph(DevParams P, SphState<R> src, SphGatherSrc<R>
     }
 }
 
+// The same hand-over without NNPS, in place: the steps of one sphdem_step call
+// after its first.  The step is Eulerian (SPH particles keep their positions
+// and types), so the set is already in cell order and its grid, wall and
+// buffer slots and neighbour list are those of the call's first step; only
+// the end-of-step values become the state and the records are rebuilt.
+template <typename R>
+__global__ void k_refresh_sph(DevParams P, SphGatherSrc<R> g, SphState<R> S, SphRec<R> rec) {
+    grid_dep_wait();
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= P.ns) return;
+    const R ux = g.ux[i], uy = g.uy[i], uz = g.uz[i], m = g.m[i], rho = g.rho[i], pr = g.pres[i];
+    S.ux[i] = ux;
+    S.uy[i] = uy;
+    S.uz[i] = uz;
+    S.m[i] = m;
+    S.rho[i] = rho;
+    S.pres[i] = pr;
+    S.temp[i] = g.temp[i];
+    rec.mr0[i] = mk2<R>(m, rho);
+    rec.up[i] = mk4<R>(ux, uy, uz, pr);
+    if (P.c2_passes) {
+        const PosRec<R> q = ldr(rec.pos + i);
+        rec.pa[i] = pv_make(q, pv_code<R>(m / rho, q.w, tag_ptype(q.w) == 1));
+    }
+}
+
 template <typename R>
 __global__ void k_cells_gather_dem(DevParams P, DemState<R> src, DemState<R> dst, const int* __restrict__ perm) {
     grid_dep_wait();
