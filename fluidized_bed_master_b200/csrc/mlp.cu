@@ -23,7 +23,8 @@ static int num_sms() {
 
 int mlp_alloc(MlpNet& m) {
     std::memset(&m, 0, sizeof(m));
-    m.nparts = num_sms();
+    m.sms = num_sms();
+    m.nparts = MLP_GRAD_CTAS * m.sms;
     auto al = [&](void** p, size_t b) { return cudaMalloc(p, b) == cudaSuccess; };
     bool ok = al((void**)&m.W1, sizeof(__nv_bfloat16) * MLP_H * MLP_IN) &&
               al((void**)&m.W2, sizeof(__nv_bfloat16) * MLP_H * MLP_H) &&
@@ -74,7 +75,7 @@ int mlp_set_params(MlpNet& m, const float* params_dev, cudaStream_t st) {
 int mlp_forward(const MlpNet& m, const void* feat, int n, float* out, cudaStream_t st, int stall) {
     if (n <= 0) return SPHDEM_OK;
     int tiles = (n + MLP_TILE - 1) / MLP_TILE;
-    int grid = std::min(tiles, 2 * m.nparts);   // two CTAs per SM overlap their MMA waits
+    int grid = std::min(tiles, MLP_INFER_CTAS * m.sms);   // the CTAs of an SM overlap their MMA waits
     k_mlp_infer<<<grid, 128, SM_INFER_END + SM_ALIGN, st>>>(n, (const __nv_bfloat16*)feat, dev_view(m), out, m.err,
                                                             stall);
     return cudaGetLastError() == cudaSuccess ? SPHDEM_OK : SPHDEM_E_CUDA;
@@ -84,11 +85,12 @@ int mlp_forward(const MlpNet& m, const void* feat, int n, float* out, cudaStream
 // of CTAs that did not run are zeroed so the sum stays over m.nparts rows)
 int mlp_grad(const MlpNet& m, const void* feat, const float* target, const float* weight, int n, float inv_wsum,
              cudaStream_t st) {
-    if (cudaMemsetAsync(m.part, 0, sizeof(float) * MLP_PART * (size_t)m.nparts, st) != cudaSuccess)
+    const int tiles = n > 0 ? (n + MLP_TILE - 1) / MLP_TILE : 0;
+    const int grid = std::min(tiles, m.nparts);
+    if (grid < m.nparts && cudaMemsetAsync(m.part + (size_t)grid * MLP_PART, 0,
+                                           sizeof(float) * MLP_PART * (size_t)(m.nparts - grid), st) != cudaSuccess)
         return SPHDEM_E_CUDA;
     if (n <= 0) return SPHDEM_OK;
-    int tiles = (n + MLP_TILE - 1) / MLP_TILE;
-    int grid = std::min(tiles, m.nparts);
     k_mlp_grad<<<grid, 128, SM_TRAIN_END + SM_ALIGN, st>>>(n, (const __nv_bfloat16*)feat, target, weight, inv_wsum,
                                                             dev_view(m), m.part, m.err);
     return cudaGetLastError() == cudaSuccess ? SPHDEM_OK : SPHDEM_E_CUDA;
@@ -144,6 +146,7 @@ int mlp_put_params(MlpNet& m, const float* host, cudaStream_t st) {
 __global__ void k_mlp_sum(int nparts, const float* __restrict__ part, float* out) {
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < MLP_NPARAM + 2; p += gridDim.x * blockDim.x) {
         float g = 0.f;
+#pragma unroll 8
         for (int c = 0; c < nparts; c++) g += part[(size_t)c * MLP_PART + p];
         out[p] = g;
     }
@@ -214,7 +217,7 @@ extern "C" int sphdem_mlp_grad(const void* feat, const float* target, const floa
     if (!r) r = mlp_grad(m, feat, target, weight, n, (float)(1.0 / weight_sum), st);
     tm.stop(st);
     if (!r) {
-        k_mlp_sum<<<(MLP_NPARAM + 2 + 255) / 256, 256, 0, st>>>(m.nparts, m.part, grad);
+        k_mlp_sum<<<(MLP_NPARAM + 2 + 63) / 64, 64, 0, st>>>(m.nparts, m.part, grad);
         if (cudaGetLastError() != cudaSuccess) r = SPHDEM_E_CUDA;
     }
     int err = 0;

@@ -13,7 +13,8 @@ struct MlpNet {
     float* part;                    // per-CTA partial gradients
     float* loss;                    // [sum w e^2, sum w] of the last gradient pass
     int* err;                       // bounded-wait failures of the MMA kernels
-    int nparts;                     // CTAs of the gradient kernel (= SMs)
+    int sms;                        // multiprocessors of the device
+    int nparts;                     // most CTAs of the gradient kernel, rows of part
 };
 
 int mlp_alloc(MlpNet& m);

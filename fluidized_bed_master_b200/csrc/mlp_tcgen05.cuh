@@ -108,6 +108,12 @@ __device__ __forceinline__ void tc_ld16(uint32_t taddr, float* v) {
     for (int q = 0; q < 16; q++) v[q] = __uint_as_float(r[q]);
 }
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// 64 columns, one wait
+__device__ __forceinline__ void tc_ld64(uint32_t taddr, float* v) {
+#pragma unroll
+    for (int c = 0; c < 64; c += 16) tc_ld16(taddr + c, v + c);
+    tc_wait_ld();
+}
 
 __device__ __forceinline__ void mbar_init(uint64_t* m, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(m)), "r"(count) : "memory");
@@ -116,7 +122,7 @@ __device__ __forceinline__ void mbar_fence_init() { asm volatile("fence.mbarrier
 // bounded wait for the phase with the given parity; false on timeout
 __device__ __forceinline__ bool mbar_wait(uint64_t* m, uint32_t parity) {
     uint32_t addr = smem_u32(m);
-    uint64_t t0 = global_ns();
+    uint64_t t0 = 0;
     while (true) {
         uint32_t done;
         asm volatile(
@@ -126,7 +132,9 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* m, uint32_t parity) {
             : "r"(addr), "r"(parity)
             : "memory");
         if (done) return true;
-        if (global_ns() - t0 > MLP_WAIT_NS) return false;
+        const uint64_t t = global_ns();   // read only once a first try has failed
+        if (t0 == 0) t0 = t;
+        else if (t - t0 > MLP_WAIT_NS) return false;
     }
 }
 
@@ -176,13 +184,20 @@ constexpr int SM_W2 = SM_W1 + 2048;             // W2  [64 x 64]        8 KB
 constexpr int SM_H1 = SM_W2 + 8192;             // H1  [128 x 64]      16 KB
 constexpr int SM_VEC = SM_H1 + 16384;           // b1, b2, w3 (FP32)   768 B
 constexpr int SM_INFER_END = SM_VEC + 1024;     // inference total    ~31 KB
+// The gradient's tile: delta2 takes H1's place (the second MMA has read H1,
+// the weight gradient reads H1^T), and delta1^T takes delta2^T's.  The
+// weight-gradient MMAs have M = 128 with 64 rows in use; rows 64..127 of
+// their A operand are whatever follows delta^T in this plan (H1^T), and only
+// give accumulator lanes that nothing reads.  84 KB, so two CTAs share an SM
+// and one's MMA waits hide behind the other's epilogues.
 constexpr int SM_W2T = SM_INFER_END;            // W2T [64 x 64]        8 KB
 constexpr int SM_XT = SM_W2T + 8192;            // [X^T; 1; 0] [32 x 128]   8 KB
-constexpr int SM_H1T = SM_XT + 8192;            // [H1^T; 1; 0] [80 x 128] 20 KB
-constexpr int SM_D2 = SM_H1T + 20480;           // delta2 [128 x 64]   16 KB
-constexpr int SM_D2T = SM_D2 + 16384;           // delta2^T [128 x 128], rows 64.. zero  32 KB
-constexpr int SM_D1T = SM_D2T + 32768;          // delta1^T [128 x 128], rows 64.. zero  32 KB
-constexpr int SM_TRAIN_END = SM_D1T + 32768;    // training total     ~167 KB
+constexpr int SM_D2 = SM_H1;                    // delta2 [128 x 64]
+constexpr int SM_DT = SM_XT + 8192;             // delta2^T, then delta1^T [64 x 128]  16 KB
+constexpr int SM_H1T = SM_DT + 16384;           // [H1^T; 1; 0] [80 x 128] 20 KB
+constexpr int SM_TRAIN_END = SM_H1T + 20480;    // training total     ~84 KB
+static_assert(SM_TRAIN_END - SM_DT >= 128 * 128 * 2, "rows 64..127 of delta^T stay inside the plan");
+constexpr int MLP_GRAD_CTAS = 2, MLP_INFER_CTAS = 4;   // resident CTAs per SM (TMEM: 2 x 256, 4 x 128 columns)
 constexpr int SM_ALIGN = 1024;
 // TMEM columns of the gradient kernel
 constexpr int TM_D1 = 0, TM_D2 = 64, TM_GW2 = 128, TM_GW1 = 208;
@@ -203,27 +218,22 @@ __device__ __forceinline__ void load_vectors(float* v, const MlpDev& net) {
     }
 }
 
-// X tile row `tid` (zero past n); returns the row's features as float
-__device__ __forceinline__ void load_x_row(unsigned char* sm, const __nv_bfloat16* feat, int n, int row, int tid,
-                                           float* x) {
+// a row's features as loaded (zero past n), and its place in the X tile
+struct XRow {
+    uint4 a, b;
+};
+__device__ __forceinline__ XRow ld_x_row(const __nv_bfloat16* feat, int n, int row) {
+    XRow x{make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
     if (row < n) {
         const uint4* src = reinterpret_cast<const uint4*>(feat + (size_t)row * MLP_IN);
-        uint4 a = src[0], b = src[1];
-        *reinterpret_cast<uint4*>(sm + SM_X + cm_off(tid, 0, MLP_IN)) = a;
-        *reinterpret_cast<uint4*>(sm + SM_X + cm_off(tid, 8, MLP_IN)) = b;
-        const __nv_bfloat16* pa = reinterpret_cast<const __nv_bfloat16*>(&a);
-        const __nv_bfloat16* pb = reinterpret_cast<const __nv_bfloat16*>(&b);
-#pragma unroll
-        for (int q = 0; q < 8; q++) {
-            x[q] = __bfloat162float(pa[q]);
-            x[8 + q] = __bfloat162float(pb[q]);
-        }
-    } else {
-#pragma unroll
-        for (int q = 0; q < 16; q++) x[q] = 0.f;
-        st_row8(sm + SM_X, tid, 0, MLP_IN, x);
-        st_row8(sm + SM_X, tid, 8, MLP_IN, x + 8);
+        x.a = __ldg(src);
+        x.b = __ldg(src + 1);
     }
+    return x;
+}
+__device__ __forceinline__ void st_x_row(unsigned char* sm, int tid, const XRow& x) {
+    *reinterpret_cast<uint4*>(sm + SM_X + cm_off(tid, 0, MLP_IN)) = x.a;
+    *reinterpret_cast<uint4*>(sm + SM_X + cm_off(tid, 8, MLP_IN)) = x.b;
 }
 
 // one MMA group + commit by thread 0, bounded wait by all.  A thread whose
@@ -263,7 +273,7 @@ __device__ __forceinline__ void load_x_row(unsigned char* sm, const __nv_bfloat1
 // stall != 0 is the failure drill of the bounded waits: the first MMA group
 // is not issued, its wait runs out after MLP_WAIT_NS, and the kernel must
 // report through *err, free its TMEM and return (no MMA is in flight).
-__global__ void __launch_bounds__(128, 1) k_mlp_infer(int n, const __nv_bfloat16* __restrict__ feat, MlpDev net,
+__global__ void __launch_bounds__(128, MLP_INFER_CTAS) k_mlp_infer(int n, const __nv_bfloat16* __restrict__ feat, MlpDev net,
                                                       float* __restrict__ out, int* err, int stall) {
     extern __shared__ unsigned char smem_raw[];
     __shared__ uint64_t mbar;
@@ -293,35 +303,29 @@ __global__ void __launch_bounds__(128, 1) k_mlp_infer(int n, const __nv_bfloat16
     const uint32_t id64 = idesc_bf16(MLP_TILE, MLP_H);
     uint32_t phase = 0, fparity = 0;
     const int ntiles = (n + MLP_TILE - 1) / MLP_TILE;
+    XRow x = ld_x_row(feat, n, blockIdx.x * MLP_TILE + tid);
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const int row = tile * MLP_TILE + tid;
-        float x[16];
-        load_x_row(sm, feat, n, row, tid, x);
+        st_x_row(sm, tid, x);
         MLP_SYNC_ISSUE(tc_mma(tm + TM_D1, smem_desc(sm + SM_X, 128, 256), smem_desc(sm + SM_W1, 128, 256), id64, 0));
+        x = ld_x_row(feat, n, row + gridDim.x * MLP_TILE);   // the next tile's, while this one is worked on
         // H1 = relu(D1 + b1) -> BF16 operand
+        float v[MLP_H];
+        tc_ld64(tm + lane_off + TM_D1, v);
 #pragma unroll
-        for (int c0 = 0; c0 < MLP_H; c0 += 16) {
-            float v[16];
-            tc_ld16(tm + lane_off + TM_D1 + c0, v);
-            tc_wait_ld();
+        for (int c0 = 0; c0 < MLP_H; c0 += 8) {
 #pragma unroll
-            for (int q = 0; q < 16; q++) v[q] = fmaxf(v[q] + vec[c0 + q], 0.f);
-            st_row8(sm + SM_H1, tid, c0, MLP_H, v);
-            st_row8(sm + SM_H1, tid, c0 + 8, MLP_H, v + 8);
+            for (int q = 0; q < 8; q++) v[c0 + q] = fmaxf(v[c0 + q] + vec[c0 + q], 0.f);
+            st_row8(sm + SM_H1, tid, c0, MLP_H, v + c0);
         }
         MLP_SYNC_ISSUE(for (int kk = 0; kk < MLP_H / 16; kk++) tc_mma(
             tm + TM_D2, smem_desc(sm + SM_H1 + kk * 256, 128, 1024), smem_desc(sm + SM_W2 + kk * 256, 128, 1024),
             id64, kk > 0));
         // y = relu(D2 + b2) . w3 + b3
         float y = b3;
+        tc_ld64(tm + lane_off + TM_D2, v);
 #pragma unroll
-        for (int c0 = 0; c0 < MLP_H; c0 += 16) {
-            float v[16];
-            tc_ld16(tm + lane_off + TM_D2 + c0, v);
-            tc_wait_ld();
-#pragma unroll
-            for (int q = 0; q < 16; q++) y += fmaxf(v[q] + vec[MLP_H + c0 + q], 0.f) * vec[2 * MLP_H + c0 + q];
-        }
+        for (int q = 0; q < MLP_H; q++) y += fmaxf(v[q] + vec[MLP_H + q], 0.f) * vec[2 * MLP_H + q];
         if (row < n) out[row] = fail ? 0.f : y;
         tc_fence_before();
         __syncthreads();
@@ -344,7 +348,7 @@ __global__ void __launch_bounds__(128, 1) k_mlp_infer(int n, const __nv_bfloat16
 // weight-gradient MMAs through a row of ones appended to H1^T and X^T.
 // Rounding points (kept by the oracle): H1, delta2 and delta1 are BF16 where
 // an MMA reads them; the masks, y and dL/dy are FP32.
-__global__ void __launch_bounds__(128, 1) k_mlp_grad(int n, const __nv_bfloat16* __restrict__ feat,
+__global__ void __launch_bounds__(128, MLP_GRAD_CTAS) k_mlp_grad(int n, const __nv_bfloat16* __restrict__ feat,
                                                      const float* __restrict__ target,
                                                      const float* __restrict__ weight, float inv_wsum, MlpDev net,
                                                      float* __restrict__ part, int* err) {
@@ -369,12 +373,7 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad(int n, const __nv_bfloat16*
     load_operand(sm + SM_W2, net.W2, MLP_H, MLP_H);
     load_operand(sm + SM_W2T, net.W2T, MLP_H, MLP_H);
     load_vectors(vec, net);
-    // rows that stay zero: delta^T padding (64..127), H1^T 65..79, X^T 17..31
-    for (int q = tid; q < 64 * 16; q += blockDim.x) {
-        int r = 64 + q / 16, k0 = (q % 16) * 8;
-        *reinterpret_cast<uint4*>(sm + SM_D2T + cm_off(r, k0, 128)) = make_uint4(0, 0, 0, 0);
-        *reinterpret_cast<uint4*>(sm + SM_D1T + cm_off(r, k0, 128)) = make_uint4(0, 0, 0, 0);
-    }
+    // rows that stay zero: H1^T 65..79, X^T 17..31
     for (int q = tid; q < 15 * 16; q += blockDim.x) {
         int r = q / 16, k0 = (q % 16) * 8;
         *reinterpret_cast<uint4*>(sm + SM_H1T + cm_off(65 + r, k0, 128)) = make_uint4(0, 0, 0, 0);
@@ -396,50 +395,59 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad(int n, const __nv_bfloat16*
     const int stall = 0;
     int first = 1;
     const int ntiles = (n + MLP_TILE - 1) / MLP_TILE;
+    int row = blockIdx.x * MLP_TILE + tid;
+    XRow x = ld_x_row(feat, n, row);
+    float wn = row < n ? __ldg(weight + row) : 0.f, tn = row < n ? __ldg(target + row) : 0.f;
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const int row = tile * MLP_TILE + tid;
         const bool valid = row < n;
-        float x[16];
-        load_x_row(sm, feat, n, row, tid, x);
+        const float wi = wn, ti = tn;
+        st_x_row(sm, tid, x);
+        {
+            const __nv_bfloat16* pa = reinterpret_cast<const __nv_bfloat16*>(&x.a);
+            const __nv_bfloat16* pb = reinterpret_cast<const __nv_bfloat16*>(&x.b);
 #pragma unroll
-        for (int q = 0; q < 16; q++) st_bf16(sm + SM_XT, q, tid, 128, x[q]);
+            for (int q = 0; q < 8; q++) {
+                *reinterpret_cast<__nv_bfloat16*>(sm + SM_XT + cm_off(q, tid, 128)) = pa[q];
+                *reinterpret_cast<__nv_bfloat16*>(sm + SM_XT + cm_off(8 + q, tid, 128)) = pb[q];
+            }
+        }
         st_bf16(sm + SM_XT, 16, tid, 128, valid ? 1.f : 0.f);
         st_bf16(sm + SM_H1T, 64, tid, 128, valid ? 1.f : 0.f);
-        const float wi = valid ? weight[row] : 0.f, ti = valid ? target[row] : 0.f;
         MLP_SYNC_ISSUE(tc_mma(tm + TM_D1, smem_desc(sm + SM_X, 128, 256), smem_desc(sm + SM_W1, 128, 256), id64, 0));
+        // the next tile's row, while this one is worked on
+        row += gridDim.x * MLP_TILE;
+        x = ld_x_row(feat, n, row);
+        wn = row < n ? __ldg(weight + row) : 0.f;
+        tn = row < n ? __ldg(target + row) : 0.f;
         uint32_t m1lo = 0, m1hi = 0;   // ReLU masks of layer 1 (bit c: z1_c > 0)
+        float v[MLP_H];
+        tc_ld64(tm + lane_off + TM_D1, v);
 #pragma unroll
-        for (int c0 = 0; c0 < MLP_H; c0 += 16) {
-            float v[16];
-            tc_ld16(tm + lane_off + TM_D1 + c0, v);
-            tc_wait_ld();
+        for (int c0 = 0; c0 < MLP_H; c0 += 8) {
 #pragma unroll
-            for (int q = 0; q < 16; q++) {
+            for (int q = 0; q < 8; q++) {
                 const int c = c0 + q;
-                float z = v[q] + vec[c];
+                float z = v[c] + vec[c];
                 bool on = z > 0.f;
                 if (on) {
                     if (c < 32) m1lo |= 1u << c;
                     else m1hi |= 1u << (c - 32);
                 }
-                v[q] = on ? z : 0.f;
-                st_bf16(sm + SM_H1T, c, tid, 128, v[q]);
+                v[c] = on ? z : 0.f;
+                st_bf16(sm + SM_H1T, c, tid, 128, v[c]);
             }
-            st_row8(sm + SM_H1, tid, c0, MLP_H, v);
-            st_row8(sm + SM_H1, tid, c0 + 8, MLP_H, v + 8);
+            st_row8(sm + SM_H1, tid, c0, MLP_H, v + c0);
         }
         MLP_SYNC_ISSUE(for (int kk = 0; kk < MLP_H / 16; kk++) tc_mma(
             tm + TM_D2, smem_desc(sm + SM_H1 + kk * 256, 128, 1024), smem_desc(sm + SM_W2 + kk * 256, 128, 1024),
             id64, kk > 0));
-        // y (first read of D2), then dL/dy, w3 gradient and delta2 (second read)
+        // y, then dL/dy, w3 gradient and delta2
         float y = b3;
+        tc_ld64(tm + lane_off + TM_D2, v);
 #pragma unroll
-        for (int c0 = 0; c0 < MLP_H; c0 += 16) {
-            float v[16];
-            tc_ld16(tm + lane_off + TM_D2 + c0, v);
-            tc_wait_ld();
-#pragma unroll
-            for (int q = 0; q < 16; q++) y += fmaxf(v[q] + vec[MLP_H + c0 + q], 0.f) * vec[2 * MLP_H + c0 + q];
+        for (int q = 0; q < MLP_H; q++) {
+            v[q] = fmaxf(v[q] + vec[MLP_H + q], 0.f);
+            y += v[q] * vec[2 * MLP_H + q];
         }
         const float e = y - ti;
         const float g3 = 2.f * wi * e * inv_wsum;
@@ -447,23 +455,16 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad(int n, const __nv_bfloat16*
         wsum += wi;
         gb3 += g3;
 #pragma unroll
-        for (int c0 = 0; c0 < MLP_H; c0 += 16) {
-            float v[16];
-            tc_ld16(tm + lane_off + TM_D2 + c0, v);
-            tc_wait_ld();
+        for (int c0 = 0; c0 < MLP_H; c0 += 8) {
+            float d[8];
 #pragma unroll
-            for (int h = 0; h < 16; h += 8) {
-                float d[8];
-#pragma unroll
-                for (int q = 0; q < 8; q++) {
-                    const int c = c0 + h + q;
-                    float h2 = fmaxf(v[h + q] + vec[MLP_H + c], 0.f);
-                    gw3[c] += g3 * h2;
-                    d[q] = h2 > 0.f ? g3 * vec[2 * MLP_H + c] : 0.f;
-                    st_bf16(sm + SM_D2T, c, tid, 128, d[q]);
-                }
-                st_row8(sm + SM_D2, tid, c0 + h, MLP_H, d);
+            for (int q = 0; q < 8; q++) {
+                const int c = c0 + q;
+                gw3[c] += g3 * v[c];
+                d[q] = v[c] > 0.f ? g3 * vec[2 * MLP_H + c] : 0.f;
+                st_bf16(sm + SM_DT, c, tid, 128, d[q]);
             }
+            st_row8(sm + SM_D2, tid, c0, MLP_H, d);
         }
         // D3 = delta2 W2 (B operand W2^T); [dW2 | db2] += delta2^T [H1 | 1]
         MLP_SYNC_ISSUE({
@@ -471,25 +472,19 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad(int n, const __nv_bfloat16*
                 tc_mma(tm + TM_D1, smem_desc(sm + SM_D2 + kk * 256, 128, 1024),
                        smem_desc(sm + SM_W2T + kk * 256, 128, 1024), id64, kk > 0);
             for (int kk = 0; kk < MLP_TILE / 16; kk++)
-                tc_mma(tm + TM_GW2, smem_desc(sm + SM_D2T + kk * 256, 128, 2048),
+                tc_mma(tm + TM_GW2, smem_desc(sm + SM_DT + kk * 256, 128, 2048),
                        smem_desc(sm + SM_H1T + kk * 256, 128, 2048), idw2, (first == 0 || kk > 0));
         });
         // delta1 = D3 (z1 > 0)
+        tc_ld64(tm + lane_off + TM_D1, v);
 #pragma unroll
-        for (int c0 = 0; c0 < MLP_H; c0 += 16) {
-            float v[16];
-            tc_ld16(tm + lane_off + TM_D1 + c0, v);
-            tc_wait_ld();
-#pragma unroll
-            for (int q = 0; q < 16; q++) {
-                const int c = c0 + q;
-                bool on = (c < 32) ? ((m1lo >> c) & 1u) : ((m1hi >> (c - 32)) & 1u);
-                st_bf16(sm + SM_D1T, c, tid, 128, on ? v[q] : 0.f);
-            }
+        for (int c = 0; c < MLP_H; c++) {
+            bool on = (c < 32) ? ((m1lo >> c) & 1u) : ((m1hi >> (c - 32)) & 1u);
+            st_bf16(sm + SM_DT, c, tid, 128, on ? v[c] : 0.f);
         }
         // [dW1 | db1] += delta1^T [X | 1]
         MLP_SYNC_ISSUE(for (int kk = 0; kk < MLP_TILE / 16; kk++) tc_mma(
-            tm + TM_GW1, smem_desc(sm + SM_D1T + kk * 256, 128, 2048), smem_desc(sm + SM_XT + kk * 256, 128, 2048),
+            tm + TM_GW1, smem_desc(sm + SM_DT + kk * 256, 128, 2048), smem_desc(sm + SM_XT + kk * 256, 128, 2048),
             idw1, (first == 0 || kk > 0)));
         first = 0;
         tc_fence_before();
@@ -582,6 +577,7 @@ __global__ void k_mlp_adam(int nparts, const float* __restrict__ part, MlpOpt o,
                            float beta2, float eps, int t, int apply) {
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < MLP_NPARAM + 2; p += gridDim.x * blockDim.x) {
         float g = 0.f;
+#pragma unroll 8
         for (int c = 0; c < nparts; c++) g += part[(size_t)c * MLP_PART + p];
         if (p >= MLP_NPARAM) {
             if (p == MLP_NPARAM) o.loss[0] = g;   // sum w e^2 (divided by the weight sum on the host)
