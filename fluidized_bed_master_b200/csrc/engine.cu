@@ -1465,6 +1465,36 @@ struct WEngineHost {
 };
 
 // launch KERN<R, L> with L lanes per particle (n L threads in blocks of TPB)
+// the settings whose step runs the fused pass (k_w_pair)
+static bool w_fused(const DevParams& P, const WParams& Q) {
+    return P.kernel_type == 3 && P.kgc != 1 && Q.delsph == 0;
+}
+
+template <typename R, int L>
+static cudaError_t w_launch_list(const DevParams& P, const WState<R>& S, const WWork<R>& W, int* nbr, DevFlags* F,
+                                 cudaStream_t st) {
+    return launch_pdl(k_w_list<R, L>, nblocks(P.ns * L, TPB), TPB, 0, st, P, S, W, nbr, W.ncnt, F);
+}
+template <typename R>
+static cudaError_t w_list(int L, const DevParams& P, const WState<R>& S, const WWork<R>& W, DevFlags* F,
+                          cudaStream_t st) {
+    switch (L) {
+    case 1: return w_launch_list<R, 1>(P, S, W, W.nbr, F, st);
+    case 2: return w_launch_list<R, 2>(P, S, W, W.nbr, F, st);
+    case 4: return w_launch_list<R, 4>(P, S, W, W.nbr, F, st);
+    case 8: return w_launch_list<R, 8>(P, S, W, W.nbr, F, st);
+    default: return w_launch_list<R, 16>(P, S, W, W.nbr, F, st);
+    }
+}
+template <typename R, bool CORR>
+static cudaError_t w_pairs(int L, const DevParams& P, const WParams& Q, const WState<R>& S, const WWork<R>& W,
+                           DevFlags* F, cudaStream_t st) {
+    auto k = L == 1 ? k_w_pair<R, 1, CORR> : L == 2 ? k_w_pair<R, 2, CORR> : L == 4 ? k_w_pair<R, 4, CORR>
+             : L == 8 ? k_w_pair<R, 8, CORR> : k_w_pair<R, 16, CORR>;
+    const int l = L == 1 || L == 2 || L == 4 || L == 8 ? L : 16;
+    return launch_pdl(k, nblocks(P.ns * l, TPB), TPB, 0, st, P, Q, S, W, (const DevFlags*)F);
+}
+
 #define W_LAUNCH(L, KERN, n, st, ...)                                                                      \
     do {                                                                                                   \
         switch (L) {                                                                                       \
@@ -1499,8 +1529,10 @@ static int w_nnps(SphdemHandle* H, WEngineHost<R>* EH, int src, int dst, bool ha
     WState<R>& S = EH->S[src];
     if (!hashed) k_w_hash<R><<<nblocks(n, TPB), TPB, 0, st>>>(P, S, W.key_in, EH->cs.cnt);
     CK(cell_sort(EH->cs, n, W.key_in, W.val_out, W.key_out, W.g_str, W.g_end, st));
-    k_w_gather<R><<<nblocks(n, TPB), TPB, 0, st>>>(P, S, EH->S[dst], W.val_out);
-    k_rows<<<nblocks(P.NI * P.NJ * P.NK, TPB), TPB, 0, st>>>(P, W.g_str, W.g_end, W.rows);
+    CK((launch_pdl(k_w_gather<R>, nblocks(n, TPB), TPB, 0, st, P, EH->Q, S, EH->S[dst], W,
+                   hashed && w_fused(P, EH->Q) ? 1 : 0, EH->flags)));
+    CK((launch_pdl(k_rows, nblocks(P.NI * P.NJ * P.NK, TPB), TPB, 0, st, P, (const int*)W.g_str,
+                   (const int*)W.g_end, W.rows)));
     CK(cudaGetLastError());
     return SPHDEM_OK;
 }
@@ -1514,7 +1546,10 @@ static int w_enqueue(SphdemHandle* H, WEngineHost<R>* EH, int64_t* nl) {
     cudaStream_t st = H->stream;
     int n = P.ns, so = EH->cur, sn = 1 - EH->cur;
     int bs = nblocks(n, TPB);
-    { KTIME(KT_W_PRED); k_w_predictor<R><<<bs, TPB, 0, st>>>(P, Q, EH->S[so], W, W.key_in, EH->cs.cnt); }
+    {
+        KTIME(KT_W_PRED);
+        CK((launch_pdl(k_w_predictor<R>, bs, TPB, 0, st, P, Q, EH->S[so], W, W.key_in, EH->cs.cnt)));
+    }
     {
         KTIME(KT_W_NNPS);
         int r = w_nnps<R>(H, EH, so, sn, true);
@@ -1522,14 +1557,32 @@ static int w_enqueue(SphdemHandle* H, WEngineHost<R>* EH, int64_t* nl) {
     }
     WState<R>& S = EH->S[sn];
     const int L = EH->lanes;
-    { KTIME(KT_W_LIST); W_LAUNCH(L, k_w_list, n, st, P, S, W.rows, W.nbr, W.ncnt, EH->flags); }
+    { KTIME(KT_W_LIST); CK(w_list<R>(L, P, S, W, EH->flags, st)); }
+    if (w_fused(P, Q)) {
+        // predictor (+ keys), the sort's four passes, gather (+ EOS), rows, list,
+        // pair pass (+ corrector; with XSPH corrector, XSPH and finish follow)
+        *nl += 9;
+        {
+            KTIME(KT_W_INTER);
+            if (!P.xsph) CK((w_pairs<R, true>(L, P, Q, S, W, EH->flags, st)));
+            else CK((w_pairs<R, false>(L, P, Q, S, W, EH->flags, st)));
+        }
+        if (P.xsph) {
+            { KTIME(KT_W_CORR); CK((launch_pdl(k_w_corrector<R>, bs, TPB, 0, st, P, Q, S, W, (DevFlags*)nullptr))); }
+            { KTIME(KT_W_XSPH); W_LAUNCH(L, k_w_xsph, n, st, P, S, W); }
+            { KTIME(KT_W_FINISH); k_w_finish<R><<<bs, TPB, 0, st>>>(P, S, W); }
+            *nl += 3;
+        }
+        CK(cudaGetLastError());
+        return SPHDEM_OK;
+    }
     // gradient_correction() runs for kgc_solve > 0 or Antuono, but only the
     // KGC case fills Cm, and only KGC reads it (apply_gradient_correction_2D)
     if (P.kgc == 1) { KTIME(KT_W_KGC); W_LAUNCH(L, k_w_kgc, n, st, P, S, W); }
     { KTIME(KT_W_PREP); W_LAUNCH(L, k_w_prep, n, st, P, Q, S, W, EH->flags); }
     { KTIME(KT_W_CONT); W_LAUNCH(L, k_w_continuity, n, st, P, Q, S, W); }   // + EOS
     { KTIME(KT_W_INTER); W_LAUNCH(L, k_w_interaction, n, st, P, Q, S, W); }
-    { KTIME(KT_W_CORR); k_w_corrector<R><<<bs, TPB, 0, st>>>(P, Q, S, W, EH->flags); }
+    { KTIME(KT_W_CORR); CK((launch_pdl(k_w_corrector<R>, bs, TPB, 0, st, P, Q, S, W, EH->flags))); }
     if (P.xsph) {
         { KTIME(KT_W_XSPH); W_LAUNCH(L, k_w_xsph, n, st, P, S, W); }
         { KTIME(KT_W_FINISH); k_w_finish<R><<<bs, TPB, 0, st>>>(P, S, W); }
@@ -1602,7 +1655,12 @@ static int w_tune_lanes(SphdemHandle* H, WEngineHost<R>* EH) {
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));
     auto pass = [&](int L) {
-        W_LAUNCH(L, k_w_list, n, st, P, S, W.rows, W.nbr, W.ncnt, EH->flags);
+        w_list<R>(L, P, S, W, EH->flags, st);
+        if (w_fused(P, Q)) {
+            w_pairs<R, false>(L, P, Q, S, W, EH->flags, st);
+            if (P.xsph) W_LAUNCH(L, k_w_xsph, n, st, P, S, W);
+            return;
+        }
         if (P.kgc == 1) W_LAUNCH(L, k_w_kgc, n, st, P, S, W);
         W_LAUNCH(L, k_w_prep, n, st, P, Q, S, W, EH->flags);
         W_LAUNCH(L, k_w_continuity, n, st, P, Q, S, W);
@@ -1768,6 +1826,9 @@ static int w_commit_t(SphdemHandle* H) {
     W.g_str = A.get<int>(P.num_cells + 1); W.g_end = A.get<int>(P.num_cells + 1);
     W.rows = A.get<int4>(NI * NJ * NK);
     W.ncnt = A.get<int>(ns);
+    W.rp = A.get<V4<R>>(ns);
+    W.rb = A.get<V4<R>>(ns);
+    W.rc = sizeof(R) == 4 ? A.get<V2<R>>(ns) : nullptr;
     W.nbr = nullptr;
     EH->flags = A.get<DevFlags>(1);
     EH->red_buf = A.get<double>(4);
@@ -1811,7 +1872,7 @@ static int w_commit_t(SphdemHandle* H) {
     if (r) return SPHDEM_E_CUDA;
     // neighbour-list capacity from an exact count on the sorted input
     if ((r = w_nnps<R>(H, EH, 0, 1))) return r;
-    k_w_list<R, 1><<<nblocks(ns, TPB), TPB, 0, st>>>(P, EH->S[1], W.rows, nullptr, W.ncnt, EH->flags);
+    CK((w_launch_list<R, 1>(P, EH->S[1], W, nullptr, EH->flags, st)));
     CK(cudaGetLastError());
     DevFlags f;
     CK(cudaMemcpyAsync(&f, EH->flags, sizeof(f), cudaMemcpyDeviceToHost, st));

@@ -100,6 +100,7 @@ struct DevFlags {
     int max_ncnt;
     int step_count; // the reference's count (vii[43]), advanced by k_tick at the end of a step
     int max_ncntd;  // largest SPH -> DEM list count seen
+    int filt_now;   // the 2-D WCSPH step under way sums the Shepard filter (k_w_gather)
 };
 
 template <typename R>

@@ -16,6 +16,13 @@
 //   k_w_xsph        KERNEL_xsph2D (functions_TIME.cuh:1520-1605)
 //   k_w_finish      (XSPH on) corrected positions and density become the state
 //
+// With Wendland C2 and neither gradient correction nor delta-SPH (w_fused)
+// the gather also forms the reference density and the EOS pressure of the
+// predicted state, which need no neighbour, and packs the neighbour records
+// (WWork::rp, rb, rc); one pass over the list (k_w_pair) then sums the
+// continuity, the forces and, on a filter step, the Shepard filter, and
+// corrects the state.  Other settings run the kernels above one by one.
+//
 // The reference's stock 2-D driver cannot run a moving fluid: it sets the
 // ALE flags to Eulerian (KERNEL_set_alpha, functions_ALE.cuh:2-20), runs
 // NNPS only at count 0 (WCSPH_Calc.cuh:34) and has KERNEL_interaction2D
@@ -74,7 +81,35 @@ struct WWork {
     double* rhon;                // corrected density
     int *key_in, *key_out, *val_in, *val_out, *g_str, *g_end, *nbr, *ncnt;
     int4* rows;
+    // neighbour records of the sorted, predicted state (k_w_gather):
+    //   FP32: rp {x_hi, x_lo, y_hi, y_lo} (x = x_hi + x_lo to 2^-48), rc {rho, +-h}
+    //   FP64: rp {x, y, rho, +-h}
+    // rb {ux, uy, m / rho, p}; h negative for p_type <= 0
+    V4<R>*rp, *rb;
+    V2<R>* rc;
 };
+
+__device__ __forceinline__ float4 w_pos_rec(double x, double y, float, float) {
+    const float xh = (float)x, yh = (float)y;
+    return make_float4(xh, (float)(x - (double)xh), yh, (float)(y - (double)yh));
+}
+__device__ __forceinline__ Dbl4 w_pos_rec(double x, double y, double rho, double h) { return Dbl4{x, y, rho, h}; }
+// displacement x_i - x_j: FP32 differences of the high parts are exact for
+// neighbours, so it is rounded once, like (float)(x_i - x_j)
+__device__ __forceinline__ float2 w_disp(const float4& a, const float4& b) {
+    return make_float2((a.x - b.x) + (a.y - b.y), (a.z - b.z) + (a.w - b.w));
+}
+__device__ __forceinline__ double2 w_disp(const Dbl4& a, const Dbl4& b) { return make_double2(a.x - b.x, a.y - b.y); }
+// {rho, +-h} of slot j
+__device__ __forceinline__ float2 w_rho_h(const float4&, const float2* rc, int j) { return ldr(rc + j); }
+__device__ __forceinline__ double2 w_rho_h(const Dbl4& p, const double2*, int) { return make_double2(p.z, p.w); }
+// the width (relative to Rr^2) of the band around the list radius that the
+// exact predicate decides: r^2 of w_disp is within 4 roundings (2.4e-7 in
+// FP32) plus the records' 2^-48 of the coordinates (FP64: 4 x 1.1e-16)
+__device__ __forceinline__ double w_band(float, double x, double y, double Rr) {
+    return 1e-6 + 1.5e-14 * (fabs(x) + fabs(y) + Rr) / Rr;
+}
+__device__ __forceinline__ double w_band(double, double, double, double) { return 4e-15; }
 
 struct WParams {
     double alpha, beta, delta;   // artificial viscosity, delta-SPH
@@ -96,6 +131,7 @@ __device__ __forceinline__ int w_predict(const DevParams& P, const WParams& Q, W
 
 template <typename R>
 __global__ void k_w_predictor(DevParams P, WParams Q, WState<R> S, WWork<R> W, int* key, int* cnt) {
+    grid_dep_wait();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     int k = -1;
     if (i < P.ns) {
@@ -162,39 +198,73 @@ struct Grp {
     }
 };
 
-// neighbour list: sqrt(dx^2+dy^2) + 1e-20 < kappa h_i, FP64, exact
+// neighbour list: sqrt(dx^2+dy^2) + 1e-20 < kappa h_i, exact.  The three
+// stencil rows of the particle's cell (its sort key) are slot ranges; r^2 from
+// the records decides outside the band around the radius, the FP64 predicate
+// inside it.  Every candidate's FP64 square root, the cell index by FP64
+// divisions and one atomic per particle for the largest count took 571 us on
+// the 64-bed batch (1.08 M particles).
 template <typename R, int L>
-__global__ void __launch_bounds__(128) k_w_list(DevParams P, WState<R> S, const int4* __restrict__ rows, int* nbr,
-                                                int* ncnt, DevFlags* F) {
+__global__ void __launch_bounds__(128) k_w_list(DevParams P, WState<R> S, WWork<R> W, int* nbr, int* ncnt,
+                                                DevFlags* F) {
+    grid_dep_wait();
     const Grp<L> g;
     const int i = g.i;
     if (i >= P.ns) return;   // the whole group
-    double xi = S.x[i], yi = S.y[i];
-    double Rr = __dmul_rn(P.kappa, S.h[i]);
-    int ic, jc, kc;
-    const double2 o = w_cell_off(S, i);
-    cell_ijk(P, xi + o.x, yi + o.y, 0.0, ic, jc, kc);
-    int c = 0, cap = P.nb_cap, n = P.ns;
-    const Cull cu = make_cull(xi + o.x, yi + o.y, 0.0, Rr);
-    const unsigned low = (1u << g.lane) - 1u;
-    for_rows(P, ic, jc, kc, rows, cu, [&](int a, int b) {
-        for (int j0 = a; j0 < b; j0 += L) {
-            const int j = j0 + g.lane;
-            bool hit = false;
-            if (j < b && S.ptype[j] <= 1000) hit = __dadd_rn(w_dist(xi, yi, S.x[j], S.y[j]), 1e-20) < Rr;
-            unsigned grp = (__ballot_sync(g.mask, hit) & g.mask) >> g.base;
-            if (hit) {
-                int pos = c + __popc(grp & low);
-                if (nbr && pos < cap) nbr[(size_t)pos * n + i] = j;
+    const int key = W.key_out[i];
+    int c = 0;
+    const int cap = P.nb_cap, n = P.ns;
+    if (key < P.NI * P.NJ) {
+        const int jc = key / P.NI, ic = key - jc * P.NI;
+        const double xi = S.x[i], yi = S.y[i], Rr = __dmul_rn(P.kappa, S.h[i]);
+        const double bd = w_band((R)0, xi, yi, Rr), R2 = Rr * Rr;
+        const R lo = (R)(R2 * (1.0 - bd)), hi = (R)(R2 * (1.0 + bd));
+        const V4<R> pi = ldr(W.rp + i);
+        auto test = [&](const V4<R>& pj, int j) {
+            const V2<R> d = w_disp(pi, pj);
+            const R r2 = d.x * d.x + d.y * d.y;
+            if (r2 < lo) return true;
+            if (r2 > hi) return false;
+            return __dadd_rn(w_dist(xi, yi, S.x[j], S.y[j]), 1e-20) < Rr;
+        };
+        const unsigned low = (1u << g.lane) - 1u;
+        for (int jy = max(jc - 1, 0); jy <= min(jc + 1, P.NJ - 1); jy++) {
+            const int4 r = __ldg(W.rows + ic + P.NI * jy);
+            if constexpr (L == 1) {
+                for (int j0 = r.x; j0 < r.w; j0 += 4) {
+                    V4<R> q[4];
+#pragma unroll
+                    for (int u = 0; u < 4; u++) q[u] = ldr(W.rp + min(j0 + u, r.w - 1));
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        if (j0 + u < r.w && test(q[u], j0 + u)) {
+                            if (nbr && c < cap) nbr[(size_t)c * n + i] = j0 + u;
+                            c++;
+                        }
+                    }
+                }
+            } else {
+                for (int j0 = r.x; j0 < r.w; j0 += L) {
+                    const int j = j0 + g.lane;
+                    const bool hit = j < r.w && test(ldr(W.rp + min(j, r.w - 1)), j);
+                    const unsigned grp = (__ballot_sync(g.mask, hit) & g.mask) >> g.base;
+                    if (hit) {
+                        const int pos = c + __popc(grp & low);
+                        if (nbr && pos < cap) nbr[(size_t)pos * n + i] = j;
+                    }
+                    c += __popc(grp);
+                }
             }
-            c += __popc(grp);
         }
-    });
+    }
     if (g.lane == 0) {
         ncnt[i] = c;
         if (c > cap) atomicOr(&F->overflow, 1);
-        atomicMax(&F->max_ncnt, c);
     }
+    // one atomic per converged group of threads for the largest count
+    const unsigned am = __activemask();
+    const int wmax = __reduce_max_sync(am, c);
+    if ((threadIdx.x & 31) == __ffs(am) - 1) atomicMax(&F->max_ncnt, wmax);
 }
 
 template <typename R>
@@ -266,7 +336,7 @@ __global__ void __launch_bounds__(128) k_w_prep(DevParams P, WParams Q, WState<R
     R th = (R)S.h[i], tA = knl_tmpA<R>(P.kernel_type, 2, th);
     const double rhoi = S.rho[i];
     const bool filt = (count % Q.freq_filt) == 0, anto = Q.delsph == 2, kgc = P.kgc == 1;
-    int cnt = min(W.ncnt[i], P.nb_cap);
+    const int cnt = filt || anto ? min(W.ncnt[i], P.nb_cap) : 0;   // nothing to sum on the other steps
     R flt = 0, gx = 0, gy = 0;
     for (int k = g.lane; k < cnt; k += L) {
         int j = W.nbr[(size_t)k * n + i];
@@ -295,6 +365,11 @@ __global__ void __launch_bounds__(128) k_w_prep(DevParams P, WParams Q, WState<R
         W.grx[i] = gx;
         W.gry[i] = gy;
     }
+}
+
+// Tait pressure of one particle (KERNEL_EOS, functions_PROP.cuh:7-28)
+__device__ __forceinline__ double w_eos(const WParams& Q, double rho, double rho_ref) {
+    return Q.eos_B * (pow(rho / rho_ref, Q.gamma) - 1.0);
 }
 
 // KERNEL_clc_continuity_norm2D
@@ -344,9 +419,147 @@ __global__ void __launch_bounds__(128) k_w_continuity(DevParams P, WParams Q, WS
     // buffer_type 0: it reads only row i's density and reference density,
     // and nothing in this pass reads a pressure
     if (S.btype[i] == 0) {
-        double tP = pow(rhoi_d / W.rho_ref[i], Q.gamma);
-        S.pres[i] = (R)(Q.eos_B * (tP - 1.0));
+        S.pres[i] = (R)w_eos(Q, rhoi_d, W.rho_ref[i]);
     }
+}
+
+// the corrected state of slot i from its force and density rate
+// (KERNEL_time_update_single without XSPH)
+template <typename R>
+__device__ __forceinline__ void w_correct(const DevParams& P, const WParams& Q, WState<R>& S, WWork<R>& W, int i,
+                                          R ftx, R fty, R drho, bool direct) {
+    const int pt = S.ptype[i], bt = S.btype[i];
+    R ux0 = S.ux0[i], uy0 = S.uy0[i], ax = 0, ay = 0;
+    if (pt > 0) {
+        R b = (R)(bt == 0);
+        ax = ftx * b;
+        ay = fty * b;
+    }
+    R dt = (R)P.dt;
+    R uxc = ux0 + ax * dt, uyc = uy0 + ay * dt;
+    R lim = (R)P.u_limit;
+    if ((uxc * uxc + uyc * uyc) >= lim * lim) {
+        uxc = ux0;
+        uyc = uy0;
+    }
+    if (direct) {
+        S.x[i] = S.x0[i] + (double)uxc * P.dt * (double)(pt > 0);
+        S.y[i] = S.y0[i] + (double)uyc * P.dt * (double)(pt > 0);
+    }
+    S.ux[i] = uxc;
+    S.uy[i] = uyc;
+    if (Q.rho_cont && pt > 0) {
+        double rn = S.rho0[i] + (double)drho * P.dt;
+        if (direct) S.rho[i] = rn;
+        else W.rhon[i] = rn;
+    }
+}
+
+// Continuity, forces and Shepard filter in one pass over the list (w_fused);
+// CORR: the corrector too (without XSPH).  Neighbours are read through the
+// records only, so the corrected state can go straight into the state.
+// With g = G d, G = dW/dr / r (C2Sum), V = m_j / rho_j, du = u_i - u_j:
+//   drho   rho_i V G du . d             (walls' velocities 0 there)
+//   force  -V G (p_i + p_j) / rho_i d   pressure
+//          4 V G nu / rho_i du          viscous: (d . g) / r^2 = G
+//          -P_ij G d                    artificial viscosity
+// It is bound by the list -> record loads (40 bytes per pair in FP32), so L
+// lanes share a particle's list where the particles alone do not fill the
+// machine (w_lanes).
+template <typename R, int L, bool CORR>
+__global__ void __launch_bounds__(128) k_w_pair(DevParams P, WParams Q, WState<R> S, WWork<R> W, const DevFlags* F) {
+    grid_dep_wait();
+    const Grp<L> g;
+    const int i = g.i, n = P.ns;
+    if (i >= n || S.itype[i] > 2) return;
+    const bool force = S.itype[i] == 1, filt = F->filt_now != 0;
+    const C2Sum<R> K = c2_sum<R>(P, (R)S.h[i]);
+    const V4<R> pi = ldr(W.rp + i), bi = ldr(W.rb + i);
+    const V2<R> ci = w_rho_h(pi, W.rc, i);
+    const R hi = fabs(ci.y), rhoi = ci.x, mi = (R)S.m[i];
+    const bool mov = ci.y > (R)0;   // p_type > 0
+    const R irhoi = (R)1 / rhoi, vis = (R)P.mu_gas;
+    const R cv = P.fv ? (R)4 * irhoi * ((vis * vis) / (vis + vis)) : (R)0;
+    const R cp = P.fp ? (R)1 : (R)0;
+    const R al = -(R)Q.alpha * (R)P.soundspeed, be = (R)Q.beta;
+    const R mux = mov ? bi.x : (R)0, muy = mov ? bi.y : (R)0;
+    const int cnt = min(W.ncnt[i], P.nb_cap);
+    R dr = 0, tx = 0, ty = 0, px = 0, py = 0, flt = 0;
+    auto pair = [&](const V4<R>& pj, const V4<R>& bj, const V2<R>& cj) {
+        const V2<R> d = w_disp(pi, pj);
+        const R r2 = d.x * d.x + d.y * d.y;
+        const R r = sqrt(r2);
+        if (filt) flt += bj.z * c2_w(K, r);
+        const R G = c2_g(K, r), vg = bj.z * G;
+        const bool mj = cj.y > (R)0;
+        dr += vg * ((mux - (mj ? bj.x : (R)0)) * d.x + (muy - (mj ? bj.y : (R)0)) * d.y);
+        const R dux = bi.x - bj.x, duy = bi.y - bj.y;
+        const R s = vg * (bi.w + bj.w);
+        px += s * d.x;
+        py += s * d.y;
+        R a = cv * vg;
+        tx += a * dux;
+        ty += a * duy;
+        if (P.fva) {
+            const R uij = dux * d.x + duy * d.y;
+            if (uij < (R)0) {
+                const R hij = (hi + fabs(cj.y)) * (R)0.5;
+                const R phi = hij * uij / (r2 + (R)0.01 * hij * hij);
+                const R q = -mi * phi * (al + be * phi) / (rhoi + cj.x) * (R)0.5 * G;
+                tx += q * d.x;
+                ty += q * d.y;
+            }
+        }
+    };
+    constexpr int U = 4;   // records of U entries in flight
+    int k = g.lane;
+    for (; k + (U - 1) * L < cnt; k += U * L) {
+        int j[U];
+        V4<R> pj[U], bj[U];
+        V2<R> cj[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) j[u] = __ldg(W.nbr + (size_t)(k + u * L) * n + i);
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            pj[u] = ldr(W.rp + j[u]);
+            bj[u] = ldr(W.rb + j[u]);
+            cj[u] = w_rho_h(pj[u], W.rc, j[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) pair(pj[u], bj[u], cj[u]);
+    }
+    for (; k < cnt; k += L) {
+        const int j = __ldg(W.nbr + (size_t)k * n + i);
+        const V4<R> pj = ldr(W.rp + j);
+        pair(pj, ldr(W.rb + j), w_rho_h(pj, W.rc, j));
+    }
+    dr = g.sum(dr);
+    tx = g.sum(tx);
+    ty = g.sum(ty);
+    px = g.sum(px);
+    py = g.sum(py);
+    if (filt) flt = g.sum(flt);
+    if (g.lane) return;
+    const R drho = dr * K.gn * rhoi * (R)(S.rho[i] / W.rho_ref[i]);
+    W.drho[i] = drho;
+    if (filt) S.flt_s[i] = flt * K.wn;
+    R fx = 0, fy = 0;
+    if (force) {
+        px *= -cp * K.gn;
+        py *= -cp * K.gn;
+        fx = tx * K.gn + px * irhoi;
+        fy = ty * K.gn + py * irhoi;
+        if (P.fg) fy += -(R)P.g_sph;
+        W.ftx[i] = fx;
+        W.fty[i] = fy;
+        W.ftot[i] = sqrt(fx * fx + fy * fy);
+        W.pgfx[i] = px;
+        W.pgfy[i] = py;
+    } else {
+        fx = W.ftx[i];
+        fy = W.fty[i];
+    }
+    if constexpr (CORR) w_correct(P, Q, S, W, i, fx, fy, drho, true);
 }
 
 // KERNEL_interaction2D (i_type 1): pressure, viscous and artificial-viscosity
@@ -421,11 +634,12 @@ __global__ void __launch_bounds__(128) k_w_interaction(DevParams P, WParams Q, W
 // Without XSPH no later pass reads the predicted positions and density, so
 // the corrected ones go straight into the state; with XSPH they wait in
 // xn, yn, rhon for k_w_finish.  Thread 0 also advances the device step
-// counter (read by the next step's prep).
+// counter (F; null where the gather has done that).
 template <typename R>
 __global__ void k_w_corrector(DevParams P, WParams Q, WState<R> S, WWork<R> W, DevFlags* F) {
+    grid_dep_wait();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i == 0) F->step_count += 1;
+    if (i == 0 && F) F->step_count += 1;
     if (i >= P.ns) return;
     const bool direct = !P.xsph;
     if (!direct) {
@@ -434,31 +648,7 @@ __global__ void k_w_corrector(DevParams P, WParams Q, WState<R> S, WWork<R> W, D
         W.rhon[i] = S.rho[i];
     }
     if (S.itype[i] == 3) return;
-    int pt = S.ptype[i], bt = S.btype[i];
-    R ux0 = S.ux0[i], uy0 = S.uy0[i], ax = 0, ay = 0;
-    if (pt > 0) {
-        R b = (R)(bt == 0);
-        ax = W.ftx[i] * b;
-        ay = W.fty[i] * b;
-    }
-    R dt = (R)P.dt;
-    R uxc = ux0 + ax * dt, uyc = uy0 + ay * dt;
-    R lim = (R)P.u_limit;
-    if ((uxc * uxc + uyc * uyc) >= lim * lim) {
-        uxc = ux0;
-        uyc = uy0;
-    }
-    if (direct) {
-        S.x[i] = S.x0[i] + (double)uxc * P.dt * (double)(pt > 0);
-        S.y[i] = S.y0[i] + (double)uyc * P.dt * (double)(pt > 0);
-    }
-    S.ux[i] = uxc;
-    S.uy[i] = uyc;
-    if (Q.rho_cont && pt > 0) {
-        double rn = S.rho0[i] + (double)W.drho[i] * P.dt;
-        if (direct) S.rho[i] = rn;
-        else W.rhon[i] = rn;
-    }
+    w_correct(P, Q, S, W, i, W.ftx[i], W.fty[i], W.drho[i], direct);
 }
 
 // KERNEL_xsph2D: positions from the corrected velocity plus the XSPH term
@@ -500,20 +690,40 @@ __global__ void k_w_finish(DevParams P, WState<R> S, WWork<R> W) {
     S.rho[i] = W.rhon[i];
 }
 
-// cell gather of the WCSPH state
+// cell gather of the WCSPH state, and the neighbour records.  fused: a step
+// of the w_fused path: reference density and EOS pressure of the predicted
+// state, and the step counter with the step's filter decision.
 template <typename R>
-__global__ void k_w_gather(DevParams P, WState<R> src, WState<R> dst, const int* __restrict__ perm) {
+__global__ void k_w_gather(DevParams P, WParams Q, WState<R> src, WState<R> dst, WWork<R> W, int fused, DevFlags* F) {
+    grid_dep_wait();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     int n = P.ns;
+    if (fused && i == 0) {
+        F->filt_now = (F->step_count % Q.freq_filt) == 0;
+        F->step_count += 1;
+    }
     if (i >= n) return;
-    int p = perm[i];
-    dst.x[i] = src.x[p]; dst.y[i] = src.y[p]; dst.z[i] = src.z[p]; dst.h[i] = src.h[p];
-    dst.ux[i] = src.ux[p]; dst.uy[i] = src.uy[p]; dst.m[i] = src.m[p]; dst.rho[i] = src.rho[p];
-    dst.pres[i] = src.pres[p]; dst.temp[i] = src.temp[p]; dst.flt_s[i] = src.flt_s[p];
+    int p = W.val_out[i];
+    const double x = src.x[p], y = src.y[p], h = src.h[p], m = src.m[p], rho = src.rho[p];
+    const R ux = src.ux[p], uy = src.uy[p];
+    const int pt = src.ptype[p], bt = src.btype[p], it = src.itype[p];
+    R pres = src.pres[p];
+    if (fused && it <= 2) {
+        const double v = h / 1.6, ref = m / (v * v);
+        W.rho_ref[i] = ref;
+        if (bt == 0) pres = (R)w_eos(Q, rho, ref);
+    }
+    dst.x[i] = x; dst.y[i] = y; dst.z[i] = src.z[p]; dst.h[i] = h;
+    dst.ux[i] = ux; dst.uy[i] = uy; dst.m[i] = m; dst.rho[i] = rho;
+    dst.pres[i] = pres; dst.temp[i] = src.temp[p]; dst.flt_s[i] = src.flt_s[p];
     dst.x0[i] = src.x0[p]; dst.y0[i] = src.y0[p];
     dst.ux0[i] = src.ux0[p]; dst.uy0[i] = src.uy0[p]; dst.rho0[i] = src.rho0[p];
-    dst.ptype[i] = src.ptype[p]; dst.btype[i] = src.btype[p]; dst.itype[i] = src.itype[p]; dst.pid[i] = src.pid[p];
+    dst.ptype[i] = pt; dst.btype[i] = bt; dst.itype[i] = it; dst.pid[i] = src.pid[p];
     if (src.bed) dst.bed[i] = src.bed[p];
+    const R hs = pt > 0 ? (R)h : -(R)h;
+    W.rp[i] = w_pos_rec(x, y, (R)rho, hs);
+    W.rb[i] = mk4<R>(ux, uy, (R)(m / rho), pres);
+    if (W.rc) W.rc[i] = mk2<R>((R)rho, hs);
 }
 
 // cell key of the state as it stands (the first NNPS at commit; in a step
