@@ -202,6 +202,8 @@ void alloc_work(Alloc& A, SphWork<R>& W, DemWork<double>& DW, int ns, int nd, in
     DW.rows = A.get<int4>(ncells);
     DW.nbs = A.get<int>((size_t)nd * DEM_SPH_CAP);
     DW.ncs = A.get<int>(nd);
+    DW.nbd = A.get<int>((size_t)nd * DEM_DEM_CAP);
+    DW.ncd = A.get<int>(nd);
     DW.dcs = A.get<double>((size_t)nd * 14);
     DW.dcf = A.get<int>(nd);
 }
@@ -737,7 +739,11 @@ int enqueue_step(SphdemHandle* H, EngineHost<R>* EH, int flags, int64_t* nl) {
         {
             KTIME_ON(KT_DEMCONTACT, sd);
             if (dem_thread_per_sphere(P)) CK((launch_pdl(k_dem_contact<R, 1>, bd, TPB, 0, sd, P, D, DW, DW.rows, E.flags)));
-            else CK((launch_pdl(k_dem_contact<R, 32>, bdw, TPB, 0, sd, P, D, DW, DW.rows, E.flags)));
+            else {
+                CK((launch_pdl(k_dem_near, bdw, TPB, 0, sd, P, D, DW, (const int4*)DW.rows)));
+                CK((launch_pdl(k_dem_contact<R, 8>, nblocks(nd * 8, TPB), TPB, 0, sd, P, D, DW, DW.rows, E.flags)));
+                *nl += 1;
+            }
         }
         {
             KTIME_ON(KT_DEMPREP, sd);   // see dem_thread_per_sphere

@@ -1205,36 +1205,76 @@ __global__ void __launch_bounds__(128) k_passB(DevParams P, SphState<R> S, SphWo
 }
 
 // ---------------------------------------------------------------------------
+// The spheres within the search range of each sphere (r_search r_i, the
+// candidates of KERNEL_DEM_interaction3D_dem), in visit order, for
+// k_dem_contact.  A warp per sphere scans the stencil's ~160 slots and keeps
+// ~18: the contact pass then runs its pair terms (about 450 instructions) over
+// the short list only, with 8 lanes per sphere; scanning and summing in one
+// warp-per-sphere kernel ran them with 11 of 32 lanes busy at 128 registers.
+// The squared distance decides outside a band of 4e-15 around the range (its
+// FP64 rounding is below 1e-15), the reference's square root inside it.
+// ncd holds the exact count; a sphere with more than the list holds is walked
+// by its stencil.
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(128) k_dem_near(DevParams P, DemState<double> D, DemWork<double> DW,
+                                                  const int4* __restrict__ drows) {
+    grid_dep_wait();
+    const int i = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    __shared__ int s_rows[4][20];
+    if (i >= P.nd || D.itype[i] != 1 || D.ptype[i] <= 1000) return;
+    const double xi = D.x[i], yi = D.y[i], zi = D.z[i], R = P.r_search * D.rad[i];
+    const double lo = R * R * (1.0 - 4e-15), hi = R * R * (1.0 + 4e-15);
+    int ic, jc, kc;
+    cell_ijk(P, xi, yi, zi, ic, jc, kc);
+    const unsigned lt = (1u << lane) - 1u;
+    int c = 0;
+    for_rows_warp_all(P, ic, jc, kc, drows, make_cull(xi, yi, zi, R), s_rows[threadIdx.x >> 5], lane, [&](int j) {
+        bool in = false;
+        if (j >= 0 && __ldg(D.ptype + j) > 1000) {
+            const double xj = __ldg(D.x + j), yj = __ldg(D.y + j), zj = __ldg(D.z + j);
+            const double dx = xi - xj, dy = yi - yj, dz = zi - zj, d2 = dx * dx + dy * dy + dz * dz;
+            in = d2 < lo;
+            if (!in && !(d2 > hi)) in = pair_dist(xi, yi, zi, xj, yj, zj) < R;
+            in = in && d2 > 0.0;
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, in);
+        if (in) {
+            const int pos = c + __popc(m & lt);
+            if (pos < DEM_DEM_CAP) DW.nbd[(size_t)i * DEM_DEM_CAP + pos] = j;
+        }
+        c += __popc(m);
+    });
+    if (lane == 0) DW.ncd[i] = c;
+}
+
+// ---------------------------------------------------------------------------
 // DEM contact: KERNEL_DEM_interaction3D_dem (functions_DEM_INTERACTION2.cuh:
 // 888-1766).  The history lookup compares against the start-of-step slot
 // ids held in registers; inserts pick the first slot that was free at the
 // start of the step (so two new partners in one step share a slot, as in
 // the reference).  Spring increments and overlap are FP64.
 // ---------------------------------------------------------------------------
-// G = 32: one warp per sphere (3-D beds: ~160 stencil candidates each);
-// G = 1: one thread per sphere over its candidates in visit order (2-D beds
-// with many spheres: a few candidates, which a warp would leave mostly
-// idle).  The launch picks G from the configuration (dem_thread_per_sphere
-// in engine.cu), so a bed always runs one form.
+// G = 8: eight lanes per sphere over the list of k_dem_near; G = 1: one
+// thread per sphere over its stencil in visit order (2-D beds with many
+// spheres: a few candidates, which a warp would leave mostly idle).  The
+// launch picks G from the configuration (dem_thread_per_sphere in engine.cu),
+// so a bed always runs one form.
 template <typename R, int G>
-// 4 blocks of 128 per SM (128 registers, a few spilled): 0.145 -> 0.124 ms on
-// the bench bed against the unbounded 162-register build
+// 4 blocks of 128 per SM (128 registers)
 __global__ void __launch_bounds__(128, 4) k_dem_contact(DevParams P, DemState<double> D, DemWork<double> DW,
                                                      const int4* __restrict__ drows,
                                                      DevFlags* F) {
-    static_assert(G == 32 || G == 1, "a warp or a thread per sphere");
+    static_assert(G == 8 || G == 1, "eight lanes or a thread per sphere");
     grid_dep_wait();
-    // G = 32: lanes take candidates l, l+32, ... of the stencil in visit
-    // order (for_rows_warp) and the pair terms are reduced with shuffles.
+    // G = 8: lanes take entries l, l+8, ... of the list, which is in visit
+    // order, and the pair terms are reduced with shuffles.
     // History writes keep the sequential semantics: lookups use the
     // start-of-step ids, a release clears only the partner's own slot, and
     // every new contact targets the first slot free at the start of the
     // step, so the new contact visited last wins that slot.
-    const int i = G == 32 ? (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5)
-                          : (int)(blockIdx.x * blockDim.x + threadIdx.x);
-    const int lane = G == 32 ? (int)(threadIdx.x & 31) : 0;
-    __shared__ int s_rows[4][20];
-    int* sm = s_rows[threadIdx.x >> 5];
+    const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x) / G;
+    const int lane = (int)(threadIdx.x % G);
+    const unsigned gm = G == 1 ? 0u : ((1u << G) - 1u) << (threadIdx.x & 31 & ~(G - 1));   // the group's lanes
     const int n = P.nd;
     if (i >= n) return;
     if (lane == 0) {
@@ -1270,17 +1310,14 @@ __global__ void __launch_bounds__(128, 4) k_dem_contact(DevParams P, DemState<do
         oid[s] = D.hid[s * n + i];
         if (free_slot < 0 && oid[s] < 1) free_slot = s;
     }
-    int ic, jc, kc;
-    cell_ijk(P, xi, yi, zi, ic, jc, kc);
     Q tx = 0, ty = 0, tz = 0, tqx = 0, tqy = 0, tqz = 0, dtr = 0, dtc = 0;
     const double kdt = P.dt;
     // this lane's last new contact (visit order t) and its spring
     int new_t = -1, new_id = 0;
     double new_dx = 0, new_dy = 0, new_dz = 0;
-    int t_visit = lane - G;
-    const Cull cu = make_cull(xi, yi, zi, P.r_search * radi);
+    int t_visit = -1;   // place of the pair in visit order
     auto pair = [&](int j) {
-        t_visit += G;
+        if (G == 1) t_visit++;
         if (D.ptype[j] <= 1000) return;
         double xj = D.x[j], yj = D.y[j], zj = D.z[j], radj = D.rad[j];
         double td = pair_dist(xi, yi, zi, xj, yj, zj);
@@ -1415,13 +1452,33 @@ __global__ void __launch_bounds__(128, 4) k_dem_contact(DevParams P, DemState<do
             D.hid[slot * n + i] = 0;
         }
     };
-    if constexpr (G == 32) for_rows_warp(P, ic, jc, kc, drows, cu, sm, lane, pair);
-    else for_stencil_j(P, ic, jc, kc, drows, cu, pair);
+    const int cd = G == 1 ? 0 : DW.ncd[i];
+    if (G > 1 && cd <= DEM_DEM_CAP) {
+        const int* __restrict__ nbd = DW.nbd + (size_t)i * DEM_DEM_CAP;
+        for (int k = lane; k < cd; k += G) {
+            t_visit = k;
+            pair(__ldg(nbd + k));
+        }
+    } else {
+        int ic, jc, kc, t = 0;
+        cell_ijk(P, xi, yi, zi, ic, jc, kc);
+        for_stencil_j(P, ic, jc, kc, drows, make_cull(xi, yi, zi, P.r_search * radi), [&](int j) {
+            if constexpr (G == 1) {
+                pair(j);
+            } else {
+                if (t % G == lane) {
+                    t_visit = t;
+                    pair(j);
+                }
+                t++;
+            }
+        });
+    }
     // the new contact visited last takes the first slot free at the start
     int last_t = new_t;
-    if constexpr (G == 32) {
+    if constexpr (G > 1) {
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) last_t = max(last_t, __shfl_xor_sync(0xffffffffu, last_t, o));
+        for (int o = G / 2; o > 0; o >>= 1) last_t = max(last_t, __shfl_xor_sync(gm, last_t, o));
     }
     if (last_t >= 0 && new_t == last_t) {
         // no free slot (a 17th partner): flag it; the new contact acted this
@@ -1437,10 +1494,13 @@ __global__ void __launch_bounds__(128, 4) k_dem_contact(DevParams P, DemState<do
             D.hds[(slot * 3 + 2) * n + i] = new_dz;
         }
     }
-    if constexpr (G == 32) {
-        tx = warp_sum(tx); ty = warp_sum(ty); tz = warp_sum(tz);
-        tqx = warp_sum(tqx); tqy = warp_sum(tqy); tqz = warp_sum(tqz);
-        dtr = warp_sum(dtr); dtc = warp_sum(dtc);
+    if constexpr (G > 1) {
+#pragma unroll
+        for (int o = G / 2; o > 0; o >>= 1) {
+            tx += __shfl_xor_sync(gm, tx, o); ty += __shfl_xor_sync(gm, ty, o); tz += __shfl_xor_sync(gm, tz, o);
+            tqx += __shfl_xor_sync(gm, tqx, o); tqy += __shfl_xor_sync(gm, tqy, o); tqz += __shfl_xor_sync(gm, tqz, o);
+            dtr += __shfl_xor_sync(gm, dtr, o); dtc += __shfl_xor_sync(gm, dtc, o);
+        }
     }
     if (lane != 0) return;
     if (P.fg) tz += -(Q)P.g_dem;
