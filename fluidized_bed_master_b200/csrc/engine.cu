@@ -748,7 +748,7 @@ int enqueue_step(SphdemHandle* H, EngineHost<R>* EH, int flags, int64_t* nl) {
         {
             KTIME_ON(KT_DEMPREP, sd);   // see dem_thread_per_sphere
             if (dem_thread_per_sphere(P)) CK((launch_pdl(k_dem_prep<R, 1>, bd, TPB, 0, sd, P, S, W.rec, D, DW, W.rows, DW.rows)));
-            else CK((launch_pdl(k_dem_prep<R, 32>, bdw, TPB, 0, sd, P, S, W.rec, D, DW, W.rows, DW.rows)));
+            else CK((launch_pdl(kt3 ? k_dem_prep_c2<R> : k_dem_prep<R, 32>, bdw, TPB, 0, sd, P, S, W.rec, D, DW, W.rows, DW.rows)));
         }
         *nl += 2;
     }

@@ -1023,6 +1023,107 @@ __global__ void __launch_bounds__(128) k_dem_prep(DevParams P, SphState<R> S, Sp
     }
 }
 
+// The same for Wendland C2, a warp per sphere: the scan of the ~620 SPH
+// stencil candidates only lists the ~60 within the radius, and the Shepard sums
+// run over that list (two rounds of the warp); summing inside the scan ran the
+// kernel in nearly every round with a few lanes on.  The porosity sum takes
+// the spheres from k_dem_near's list where the kernel's radius lies inside its
+// range.  78 -> 40 us on the bench bed.
+template <typename R>
+__global__ void __launch_bounds__(128) k_dem_prep_c2(DevParams P, SphState<R> S, SphRec<R> rec, DemState<double> D,
+                                                     DemWork<double> DW, const int4* __restrict__ srows,
+                                                     const int4* __restrict__ drows) {
+    grid_dep_wait();
+    const int i = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    __shared__ int s_rows[4][20];
+    __shared__ int s_list[4][DEM_SPH_CAP];
+    int* sm = s_rows[threadIdx.x >> 5];
+    int* list = s_list[threadIdx.x >> 5];
+    if (i >= P.nd) return;
+    const int it = D.itype[i];
+    if (it > 2) return;
+    const int pti = D.ptype[i];
+    const double xi = D.x[i], yi = D.y[i], zi = D.z[i], hi = D.h[i], Rr = P.kappa * hi;
+    const Knl<R, 3> K = knl_make<R, 3>(P, (R)hi);
+    const Band bd = make_band(P, Rr);
+    const PosRec<R> qp = make_pos<R>(P, xi, yi, zi, 0, 0, 0);
+    int ic, jc, kc;
+    cell_ijk(P, xi, yi, zi, ic, jc, kc);
+    const Cull cu = make_cull(xi, yi, zi, Rr);
+    const unsigned lt = (1u << lane) - 1u;
+    // the sphere's SPH neighbours (p_type <= 1000, the add = 0 form of the
+    // predicate, which k_dem_coupling_c2 uses), in visit order
+    int cs = 0;
+    for_rows_warp_all(P, ic, jc, kc, srows, cu, sm, lane, [&](int j) {
+        bool in = false;
+        if (j >= 0) {
+            const PosRec<R> qj = ldr(rec.pos + j);
+            Disp<R> d;
+            R r2;
+            in = tag_ptype(qj.w) <= 1000 && test_pair(P, qp, qj, xi, yi, zi, S.x, S.y, S.z, j, Rr, 0.0, bd, d, r2);
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, in);
+        if (in) {
+            const int pos = cs + __popc(m & lt);
+            if (pos < DEM_SPH_CAP) list[pos] = j;
+        }
+        cs += __popc(m);
+    });
+    if (lane == 0) DW.ncs[i] = cs;
+    __syncwarp();
+    R f1 = 0, f3 = 0, por = 0;
+    auto shep = [&](int j) {   // p_type 1 and 3, the 1e-20 form (add = 0 admits no other pair of non-zero weight)
+        const PosRec<R> qj = ldr(rec.pos + j);
+        const V2<R> mr = ldr(rec.mr0 + j);
+        const int ptj = tag_ptype(qj.w);
+        const Disp<R> d = disp_pt(P, qp, qj, xi, yi, zi, S.x, S.y, S.z, j);
+        R r, rinv;
+        rdist(d.dx * d.dx + d.dy * d.dy + d.dz * d.dz, r, rinv);
+        const R c = mr.x * rcp(mr.y) * kw(K, r);
+        f1 += ptj == 1 ? c : (R)0;
+        f3 += ptj == 3 ? c : (R)0;
+    };
+    if (cs <= DEM_SPH_CAP) {
+        int* __restrict__ nbs = DW.nbs + (size_t)i * DEM_SPH_CAP;
+        for (int k = lane; k < cs; k += 32) {
+            const int j = list[k];
+            nbs[k] = j;
+            shep(j);
+        }
+    } else {   // more than the list holds: the stencil again
+        for_rows_warp(P, ic, jc, kc, srows, cu, sm, lane, [&](int j) {
+            const PosRec<R> qj = ldr(rec.pos + j);
+            Disp<R> d;
+            R r2;
+            if (tag_ptype(qj.w) <= 1000 && test_pair(P, qp, qj, xi, yi, zi, S.x, S.y, S.z, j, Rr, 0.0, bd, d, r2)) shep(j);
+        });
+    }
+    const float r2l = r2_lo(Rr), r2h = r2_hi(Rr);
+    auto dem_por = [&](int j) {
+        if (D.ptype[j] <= 1000) return;
+        const PairT<R> g = pair_test<R>(xi, yi, zi, D.x[j], D.y[j], D.z[j], Rr, 1e-20, r2l, r2h);
+        if (g.in) por += kw(K, g.r) * dem_measure(P, (R)D.rad[j]);
+    };
+    const int cd = it == 1 && pti > 1000 && Rr <= P.r_search * D.rad[i] ? DW.ncd[i] : DEM_DEM_CAP + 1;
+    if (cd <= DEM_DEM_CAP) {
+        // the list leaves out the sphere itself (and any at its very centre)
+        const int* __restrict__ nbd = DW.nbd + (size_t)i * DEM_DEM_CAP;
+        for (int k = lane; k < cd; k += 32) dem_por(__ldg(nbd + k));
+        if (lane == 0) dem_por(i);
+    } else {
+        for_rows_warp(P, ic, jc, kc, drows, cu, sm, lane, dem_por);
+    }
+    f1 = warp_sum(f1);
+    f3 = warp_sum(f3);
+    por = warp_sum(por);
+    if (lane == 0 && pti > 1000) {
+        DW.flt_s[i] = f3;
+        DW.flt_sd[i] = f1;
+        DW.flt_sd2[i] = f1;
+        DW.DEMpor[i] = (R)1 - (por / (f3 + f1 + (R)1.0e-20));
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Sub-particle-scale eddy viscosity, the strain-rate branch of
 // KERNEL_clc_prep3D_sph (functions_PREP2.cuh:2113-2118, 2166-2171), run
@@ -1548,6 +1649,34 @@ struct DcSums {
 // kappa h_i test): Shepard sums of fluid/air velocity, temperature and
 // porosity, and the pressure-gradient force
 template <typename R, int KT>
+__device__ __forceinline__ void dc_pair_at(const Knl<R, KT>& K, R ff, R fa, R pgc, const V4<R>& fj, const V4<R>& uj,
+                                           R gx, R gy, R gz, int ptj, R r, DcSums<R>& a) {
+    const R porj = fj.w;
+    if (!(porj < (R)1)) return;
+    R w = kw(K, r);
+    R mj = fj.x, rhoj = fj.y, c = mj * w * rcp(rhoj);
+    if ((ptj == 1 && ff > (R)0.000001) || (ptj == 3 && fa > (R)0.000001)) {
+        if (ptj == 1) {
+            a.has_f = 1;
+            a.ufx += uj.x * c; a.ufy += uj.y * c; a.ufz += uj.z * c;
+            a.ttf += fj.z * c;
+            a.wtf += c;
+        } else {
+            a.has_a = 1;
+            a.uax += uj.x * c; a.uay += uj.y * c; a.uaz += uj.z * c;
+            a.tta += fj.z * c;
+            a.wta += c;
+        }
+        a.por += porj * c;
+    }
+    if (ptj != 0 && ptj != 9 && ptj != -3 && ptj != 3 && ff > (R)0.01) {
+        R q = c * pgc;
+        a.tx += gx * q;
+        a.ty += gy * q;
+        a.tz += gz * q;
+    }
+}
+template <typename R, int KT>
 __device__ __forceinline__ void dc_pair(const SphWork<R>& W, const Knl<R, KT>& K, R ff, R fa, R pgc, int j, int ptj, R r,
                                         DcSums<R>& a) {
     const V4<R> fj = ldr(W.rec.f1 + j);
@@ -1743,7 +1872,22 @@ __global__ void __launch_bounds__(128) k_dem_coupling(DevParams P, SphState<R> S
         // the neighbours k_dem_prep listed (same positions, same predicate);
         // a sphere with more than the list holds walks its stencil
         const int cs = DW.ncs[i];
-        if (cs <= DEM_SPH_CAP) {
+        if (KT == 3 && G == 32 && cs <= DEM_SPH_CAP) {
+            // the listed pairs are inside: all of a pair's records load
+            // together instead of one after another's test (54 -> 38 us on the
+            // bench bed, where the pass waits on loads)
+            const int* __restrict__ nbs = DW.nbs + (size_t)i * DEM_SPH_CAP;
+            for (int k = lane; k < cs; k += G) {
+                const int j = __ldg(nbs + k);
+                const PosRec<R> qj = ldr(rec.pos + j);
+                const V4<R> fj = ldr(rec.f1 + j), uj = ldr(rec.up + j);
+                const R gx = ldr(W.pgfx + j), gy = ldr(W.pgfy + j), gz = ldr(W.pgfz + j);
+                const Disp<R> d = disp_pt(P, qp, qj, xi, yi, zi, S.x, S.y, S.z, j);
+                R r, rinv;
+                rdist(d.dx * d.dx + d.dy * d.dy + d.dz * d.dz, r, rinv);
+                dc_pair_at(K, ff, fa, pgc, fj, uj, gx, gy, gz, tag_ptype(qj.w), r, a);
+            }
+        } else if (cs <= DEM_SPH_CAP) {
             const int* __restrict__ nbs = DW.nbs + (size_t)i * DEM_SPH_CAP;
             for (int k = lane; k < cs; k += G) pair(__ldg(nbs + k));
         } else {
