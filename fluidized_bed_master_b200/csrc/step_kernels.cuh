@@ -1028,7 +1028,8 @@ __global__ void __launch_bounds__(128) k_dem_prep(DevParams P, SphState<R> S, Sp
 // run over that list (two rounds of the warp); summing inside the scan ran the
 // kernel in nearly every round with a few lanes on.  The porosity sum takes
 // the spheres from k_dem_near's list where the kernel's radius lies inside its
-// range.  78 -> 40 us on the bench bed.
+// range.  78 -> 66 us on the bench bed, 0.66 -> 0.57 ms on
+// 200,000 spheres: bound by the scan.
 template <typename R>
 __global__ void __launch_bounds__(128) k_dem_prep_c2(DevParams P, SphState<R> S, SphRec<R> rec, DemState<double> D,
                                                      DemWork<double> DW, const int4* __restrict__ srows,
@@ -1874,7 +1875,7 @@ __global__ void __launch_bounds__(128) k_dem_coupling(DevParams P, SphState<R> S
         const int cs = DW.ncs[i];
         if (KT == 3 && G == 32 && cs <= DEM_SPH_CAP) {
             // the listed pairs are inside: all of a pair's records load
-            // together instead of one after another's test (54 -> 38 us on the
+            // together instead of one after another's test (56 -> 48 us on the
             // bench bed, where the pass waits on loads)
             const int* __restrict__ nbs = DW.nbs + (size_t)i * DEM_SPH_CAP;
             for (int k = lane; k < cs; k += G) {
