@@ -545,6 +545,27 @@ inline cudaError_t launch_neumann_tiled(Engine<float>& E, const SphState<float>&
                       (const int*)nullptr, (const int*)nullptr);
 }
 
+// the wall pass: tiled in FP32 and, for Wendland C2, in FP64; else a warp per wall
+template <typename R>
+cudaError_t launch_neumann(Engine<R>& E, const SphState<R>& S, R* pres, int patch_p, cudaStream_t st) {
+    const DevParams& P = E.P;
+    SphWork<R>& W = E.sw;
+    if constexpr (std::is_same<R, float>::value) {
+        return launch_neumann_tiled(E, S, pres, patch_p, st);
+    } else {
+        if (!P.c2_passes)
+            return launch_pdl(k_neumann<R>, nblocks(P.nwall * 32, TPB), TPB, 0, st, P, S, W, pres, (const int4*)W.rows,
+                              patch_p);
+        if (cell_sort_sparse(E.cs_s, P.ns))
+            return launch_pdl(k_neumann_tiled64<true>, (occ_warps(P) + 1) / 2, 64, 0, st, P, S, W, pres,
+                              (const int*)W.g_str, (const int*)W.g_end, (const int4*)W.rows, patch_p,
+                              (const int*)E.cs_s.occ, (const int*)E.cs_s.occ_n);
+        return launch_pdl(k_neumann_tiled64<false>, (P.NI * P.NJ * P.NK + 1) / 2, 64, 0, st, P, S, W, pres,
+                          (const int*)W.g_str, (const int*)W.g_end, (const int4*)W.rows, patch_p,
+                          (const int*)nullptr, (const int*)nullptr);
+    }
+}
+
 template <typename R>
 cudaError_t launch_list(EngineHost<R>* EH, const SphState<R>& S, int mode, cudaStream_t st) {
     Engine<R>& E = EH->E;
@@ -719,7 +740,7 @@ int enqueue_step(SphdemHandle* H, EngineHost<R>* EH, int flags, int64_t* nl) {
     SphState<R>& S = E.S[sn];
     DemState<double>& D = E.D[dn];
     int bs = nblocks(ns, TPB), bd = nblocks(nd, TPB);
-    int bdw = nblocks(nd * 32, TPB), bww = nblocks(P.nwall * 32, TPB), bbw = nblocks(P.nbuf * 32, TPB);
+    int bdw = nblocks(nd * 32, TPB), bbw = nblocks(P.nbuf * 32, TPB);
     if (!keep) {
         if ((r = nnps_sph<R>(H, EH, so, sn, nl))) return r;
     } else if (ns > 0) {
@@ -802,10 +823,7 @@ int enqueue_step(SphdemHandle* H, EngineHost<R>* EH, int flags, int64_t* nl) {
     if (ns > 0) {
         if (flags & F_COUNT0) {
             KTIME(KT_NEUMANN0);
-            if constexpr (std::is_same<R, float>::value)
-                CK(launch_neumann_tiled(E, S, S.pres, 1, st));
-            else
-                CK((launch_pdl(k_neumann<R>, bww, TPB, 0, st, P, S, W, S.pres, W.rows, 1)));
+            CK(launch_neumann<R>(E, S, S.pres, 1, st));
             *nl += 1;
         }
         {
@@ -815,10 +833,7 @@ int enqueue_step(SphdemHandle* H, EngineHost<R>* EH, int flags, int64_t* nl) {
         }
         {
             KTIME(KT_NEUMANN);
-            if constexpr (std::is_same<R, float>::value)
-                CK(launch_neumann_tiled(E, S, W.p_new, 0, st));
-            else
-                CK((launch_pdl(k_neumann<R>, bww, TPB, 0, st, P, S, W, W.p_new, W.rows, 0)));
+            CK(launch_neumann<R>(E, S, W.p_new, 0, st));
         }
         { KTIME(KT_PASSC); CK((launch_pdl(kt3 ? k_passC<R> : k_passC_any<R>, bs, TPB, 0, st, P, S, W))); }
         *nl += 3;

@@ -218,6 +218,9 @@ __device__ __forceinline__ Disp<double> disp_pt(const DevParams&, const QPos64&,
 struct Band {
     float lo, hi;
 };
+// FP64 build: a squared distance (rounded by less than 1e-15 of itself) that
+// decides the predicate without the square root
+__device__ __forceinline__ bool far64(double r2, double Rr) { return r2 > Rr * Rr * (1.0 + 4e-15); }
 __device__ __forceinline__ Band make_band(const DevParams& P, double Rr) {
     double b = 2e-6 + P.q_abs / Rr;
     double r2 = Rr * Rr;
@@ -269,8 +272,9 @@ __device__ __forceinline__ void test_pair2(const DevParams&, const QPos64&, cons
     d.dx = ax - b.x;
     d.dy = ay - b.y;
     d.dz = az - b.z;
-    const double r = pair_dist(ax, ay, az, b.x, b.y, b.z);
     r2 = d.dx * d.dx + d.dy * d.dy + d.dz * d.dz;
+    if (far64(r2, Rr)) { in0 = in20 = false; return; }
+    const double r = pair_dist(ax, ay, az, b.x, b.y, b.z);
     in0 = __dadd_rn(r, 0.0) < Rr;
     in20 = __dadd_rn(r, 1e-20) < Rr;
 }
@@ -280,9 +284,10 @@ __device__ __forceinline__ bool test_pair(const DevParams&, const QPos64&, const
     d.dx = ax - b.x;
     d.dy = ay - b.y;
     d.dz = az - b.z;
-    double r = pair_dist(ax, ay, az, b.x, b.y, b.z);
     r2 = d.dx * d.dx + d.dy * d.dy + d.dz * d.dz;
-    return __dadd_rn(r, add) < Rr;
+    if (far64(r2, Rr)) return false;
+    if (r2 < Rr * Rr * (1.0 - 4e-15) && add < 1e-17 * Rr) return true;
+    return __dadd_rn(pair_dist(ax, ay, az, b.x, b.y, b.z), add) < Rr;
 }
 
 // ---- pair distance, reciprocal ----------------------------------------------

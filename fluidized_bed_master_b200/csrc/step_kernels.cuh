@@ -2323,6 +2323,130 @@ __global__ void __launch_bounds__(NT_WARPS * 32, 8) k_neumann_tiled(DevParams P,
     }
 }
 
+// The tiled pass in double (Wendland C2): a warp per cell that holds walls,
+// the fluid candidates staged with their factors, a lane per wall.  The squared
+// distance decides outside a band of 4e-15 around the radius (its rounding is
+// below 1e-15), the reference's square root inside it.  A warp per wall
+// (k_neumann) evaluated a square root per candidate and reduced four sums per
+// wall: 331 -> 143 us on the bench bed.
+constexpr int N64_CH = 96;
+__device__ __forceinline__ void neumann_cell64(int c, const DevParams& P, SphState<double>& S, SphWork<double>& W,
+                                               double* pres, const int* __restrict__ gs, const int* __restrict__ ge,
+                                               const int4* __restrict__ rows, int patch_p, double2 (*sa)[4], int* sj,
+                                               int* srw, int lane) {
+    const int a0 = __ldg(gs + c);
+    if (a0 < 0) return;
+    const int e0 = __ldg(ge + c);
+    const SphRec<double> rec = W.rec;
+    bool any_wall = false;
+    for (int i = a0 + lane; i < e0; i += 32) any_wall |= S.ptype[i] <= 0;
+    if (!__any_sync(0xffffffffu, any_wall)) return;
+    const int ic = c % P.NI, jc = (c / P.NI) % P.NJ, kc = c / (P.NI * P.NJ);
+    const int tot = stage_rows(P, ic, jc, kc, rows, srw, lane);
+    const unsigned lt = (1u << lane) - 1u;
+    for (int p0 = a0; p0 < e0; p0 += 32) {
+        const int i = p0 + lane;
+        const bool act = i < e0 && S.ptype[i] <= 0;
+        if (!__any_sync(0xffffffffu, act)) continue;
+        double xi = 0, yi = 0, zi = 0, R2 = 0, hq = 0, scale = 1;
+        if (act) {
+            xi = S.x[i];
+            yi = S.y[i];
+            zi = S.z[i];
+            const double hi = S.h[i];
+            R2 = 2.0 * (P.kappa * hi);
+            hq = 0.25 / hi;   // 1 / (2 (2h))
+            scale = knl_tmpA<double>(3, P.dim, hi);
+        }
+        const double lo = R2 * R2 * (1.0 - 4e-15), hi2 = R2 * R2 * (1.0 + 4e-15);
+        double tp = 0, flt = 0, tt = 0, tr = 0;
+        int t = 0;
+        while (t < tot) {
+            int ns = 0;
+            while (t < tot && ns <= N64_CH - 32) {
+                const int tl = t + lane;
+                bool keep = false;
+                int j = 0;
+                if (tl < tot) {
+                    j = row_slot(srw, tl);
+                    const int ptj = S.ptype[j];
+                    keep = ptj >= 1 && ptj < 1000;
+                }
+                const unsigned m = __ballot_sync(0xffffffffu, keep);
+                if (keep) {
+                    const int pos = ns + __popc(m & lt);
+                    const Dbl4 fj = ldr(rec.f1 + j);
+                    sa[pos][0] = make_double2(S.x[j], S.y[j]);
+                    sa[pos][1] = make_double2(S.z[j], fj.x / fj.y);
+                    sa[pos][2] = make_double2(pres[j], fj.z);
+                    sa[pos][3] = make_double2(fj.x / fj.w, 0.0);
+                    sj[pos] = j;
+                }
+                ns += __popc(m);
+                t += 32;
+            }
+            __syncwarp();
+            if (act) {
+#pragma unroll 2
+                for (int u = 0; u < ns; u++) {
+                    const double2 xy = sa[u][0], zm = sa[u][1];
+                    const double dx = xi - xy.x, dy = yi - xy.y, dz = zi - zm.x;
+                    const double r2 = dx * dx + dy * dy + dz * dz;
+                    if (r2 > hi2) continue;
+                    if (!(r2 < lo)) {
+                        const int j = sj[u];
+                        if (!(__dadd_rn(pair_dist(xi, yi, zi, S.x[j], S.y[j], S.z[j]), 1e-20) < R2)) continue;
+                    }
+                    const double q = r2 * rsq_floor(r2) * hq;
+                    if (!(q < 1.0)) continue;
+                    const double a = 1.0 - q, a2 = a * a, wk = a2 * a2 * (1.0 + 4.0 * q);
+                    const double2 pt = sa[u][2], me = sa[u][3];
+                    const double mr = zm.y * wk;
+                    tp += mr * pt.x;
+                    flt += mr;
+                    tt += mr * pt.y;
+                    tr += me.x * wk;
+                }
+            }
+            __syncwarp();
+        }
+        if (!act) continue;
+        double pw, rw;
+        if (flt * scale < 1e-6) {
+            rw = W.rho_ref[i];
+            pw = 0.0;
+        } else {
+            pw = tp / flt;
+            S.temp[i] = tt / flt;
+            rw = rec.f1[i].w * tr / flt;
+        }
+        wall_store<double>(P, W, pres, i, pw, rw, patch_p);
+    }
+}
+
+template <bool OCC>
+__global__ void __launch_bounds__(64) k_neumann_tiled64(DevParams P, SphState<double> S, SphWork<double> W,
+                                                        double* pres, const int* __restrict__ gs,
+                                                        const int* __restrict__ ge, const int4* __restrict__ rows,
+                                                        int patch_p, const int* __restrict__ occ,
+                                                        const int* __restrict__ occ_n) {
+    grid_dep_wait();
+    __shared__ double2 sa[2][N64_CH][4];
+    __shared__ int sj[2][N64_CH];
+    __shared__ int srow[2][20];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if constexpr (OCC) {   // a sparse grid: the occupied cells, grid-stride
+        const int no = *occ_n;
+        for (int q = blockIdx.x * 2 + w; q < no; q += gridDim.x * 2) {
+            neumann_cell64(occ[q], P, S, W, pres, gs, ge, rows, patch_p, sa[w], sj[w], srow[w], lane);
+            __syncwarp();
+        }
+    } else {
+        const int c = blockIdx.x * 2 + w;
+        if (c < P.NI * P.NJ * P.NK) neumann_cell64(c, P, S, W, pres, gs, ge, rows, patch_p, sa[w], sj[w], srow[w], lane);
+    }
+}
+
 // ---------------------------------------------------------------------------
 // KERNEL_PPE3D_sph + KERNEL_PPE3D_calc_sph (functions_PPE2.cuh:542-698,
 // 868-878): one Jacobi sweep; p_new = (b + sum A_ij p_j) / sum A_ij for
