@@ -447,7 +447,9 @@ static int enqueue_krylov(SphdemHandle* H, EngineHost<R>* EH, SphState<R>& S, Sp
     CK(cudaMemsetAsync(K.sc + KS_DONE, 0, sizeof(double), st));
     {
         KTIME(KT_PPE_ASM);
-        k_kry_assemble<R><<<nblocks(n, TPB), TPB, 0, st>>>(P, S, W, K, H->p.warm_start == SPHDEM_WARM_EXTRAPOLATE);
+        const int ext = H->p.warm_start == SPHDEM_WARM_EXTRAPOLATE;
+        if (K.fraw) k_kry_assemble<R, true><<<nblocks(n, TPB), TPB, 0, st>>>(P, S, W, K, ext);
+        else k_kry_assemble<R, false><<<nblocks(n, TPB), TPB, 0, st>>>(P, S, W, K, ext);
         if (EH->has_mg) mg_setup<R>(EH, st);
     }
     if (phase || K.D) {

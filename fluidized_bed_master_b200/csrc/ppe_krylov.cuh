@@ -29,9 +29,9 @@
 // Krylov vectors, dot products and norms are FP64; coefficients are R.
 // Coefficient storage: entry k of row i = {j, a_ij} (8 B in the FP32
 // build), solved neighbours only, in slices of 32 rows: the entries of
-// rows 32s..32s+31 are one contiguous block, entry k of the slice's rows
-// adjacent (kent_at), so a warp's load of entry k is one 256-B line pair
-// and a warp's whole row block one contiguous stream.
+// rows 32s..32s+31 are one contiguous block, entries k and k + 1 of the
+// slice's rows adjacent (kent_at), so a warp's load of two entries is 512
+// contiguous bytes and a warp's whole row block one contiguous stream.
 // Dot products are reduced deterministically: every block writes a
 // partial sum; the kernel that needs the totals (or the last block of the
 // producing kernel) adds the partials in block order.
@@ -45,7 +45,8 @@
 namespace sphdem {
 
 constexpr int KRY_G = 1184;  // blocks of the vector kernels (8 per SM)
-constexpr int KRY_GS = 444;  // blocks of the CG product: the 3 per SM its registers allow, one wave
+constexpr int KRY_GS = 444;  // blocks of the CG product: 3 per SM, one wave (4 per SM at 64 registers:
+                             // column 49 -> 56 us an iteration, bench bed 80 -> 76)
 constexpr int KRY_T = 256;
 constexpr int KRY_NPART = 10;
 
@@ -81,10 +82,50 @@ struct KEnt<double> {
     }
 };
 
-// slot of entry k of row i (cap entries per row)
+// slot of entry k of row i (cap entries per row, a multiple of 8): pairs of
+// entries of a row side by side, the 32 rows of a slice next to each other, so
+// a warp reads two entries of its rows in one 16-byte load per lane.  A row is
+// padded with zero coefficients to a multiple of 8 entries (kent_pad).
 __device__ __forceinline__ size_t kent_at(int i, int k, int cap) {
-    return ((size_t)(i >> 5) * cap + k) * 32 + (i & 31);
+    return ((size_t)(i >> 5) * cap + (k & ~1)) * 32 + (i & 31) * 2 + (k & 1);
 }
+template <typename R>
+__device__ __forceinline__ void kent_pad(typename KEnt<R>::T* e, int i, int k, int cap) {
+    for (; k & 7; k++) e[kent_at(i, k, cap)] = KEnt<R>::make(i, (R)0);
+}
+// two entries, past L1 (they stream once per product; L1 keeps the vector)
+struct KPair {
+    int j0, j1;
+    double a0, a1;
+};
+__device__ __forceinline__ int4 kent_ld16(const void* p) {
+    int4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.b32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "l"(p));
+    return v;
+}
+template <typename R>
+struct KRaw;   // a pair as loaded
+template <>
+struct KRaw<float> {
+    int4 v;
+    __device__ __forceinline__ void load(const int2* e) { v = kent_ld16(e); }
+    __device__ __forceinline__ KPair get() const {
+        return KPair{v.x, v.z, (double)__int_as_float(v.y), (double)__int_as_float(v.w)};
+    }
+};
+template <>
+struct KRaw<double> {
+    int4 v, w;
+    __device__ __forceinline__ void load(const int4* e) {
+        v = kent_ld16(e);
+        w = kent_ld16(e + 1);
+    }
+    __device__ __forceinline__ KPair get() const {
+        return KPair{v.x, w.x, __hiloint2double(v.w, v.z), __hiloint2double(w.w, w.z)};
+    }
+};
 
 template <typename R>
 struct KryWork {
@@ -156,7 +197,8 @@ __device__ __forceinline__ bool kry_solve_row(const DevParams& P, int it, int pt
 // Same neighbour terms and source as k_ppe.  Initial iterate: the previous
 // pressure, plus its last change when extrapolate is set (the learned
 // warm start overwrites it later).
-template <typename R>
+// FEAT: the learned warm start's features are formed too.
+template <typename R, bool FEAT>
 __global__ void __launch_bounds__(128) k_kry_assemble(DevParams P, SphState<R> S, SphWork<R> W, KryWork<R> K,
                                                       int extrapolate) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -173,7 +215,7 @@ __global__ void __launch_bounds__(128) k_kry_assemble(DevParams P, SphState<R> S
         K.d[i] = 1.0;
         K.b[i] = 0.0;
         K.x[i] = 0.0;
-        if (K.fraw) {
+        if (FEAT) {
             float* f = K.fraw + (size_t)i * MLP_FEAT;
 #pragma unroll
             for (int q = 0; q < MLP_FEAT; q++) f[q] = 0.f;
@@ -237,23 +279,26 @@ __global__ void __launch_bounds__(128) k_kry_assemble(DevParams P, SphState<R> S
                 } else {
                     bfix += (double)a * (double)uj.w;
                 }
-                double pj = (double)uj.w;
-                apsum += (double)a * pj;
-                pmean += pj;
-                pmin = fmin(pmin, pj);
-                pmax = fmax(pmax, pj);
-                np++;
+                if (FEAT) {
+                    double pj = (double)uj.w;
+                    apsum += (double)a * pj;
+                    pmean += pj;
+                    pmin = fmin(pmin, pj);
+                    pmax = fmax(pmax, pj);
+                    np++;
+                }
             }
         });
     R bdiv = (R)P.rho_gas * (bx + by + bz) / (R)P.sdt;
     R bpor = (R)P.rho_gas * ((R)2 * S.dDEMpor[i] - W.dDEMpor_prev[i]) / (R)P.sdt;
     R bsrc = (R)P.rho_gas * (bx + by + bz + (R)2 * S.dDEMpor[i] - W.dDEMpor_prev[i]) / (R)P.sdt;
+    kent_pad<R>(ent, i, k, K.cap);
     K.kcnt[i] = k + 1;
     K.wm[i] = (double)fi.x;
     K.d[i] = dsum;
     K.b[i] = (double)bsrc + bfix;
     K.x[i] = (double)upi.w + (extrapolate ? (double)S.dpres[i] : 0.0);
-    if (K.fraw) {
+    if (FEAT) {
         // features of the learned warm start: the previous pressure, the
         // reference's one-sweep update (b_i + sum_j a_ij p_j)/d_i and its
         // increment, neighbour pressure statistics, the terms of the
@@ -285,43 +330,46 @@ __global__ void __launch_bounds__(128) k_kry_assemble(DevParams P, SphState<R> S
     }
 }
 
-// y_i = d_i x_i - sum_k a_ik x_j(k) over the stored entries of row i, in
-// list order.  Software pipelined: the entries of the next group of B load
-// while the current group's gathers are in flight (B = 8 measured best:
-// 57 us per PCG iteration on the bench bed against 72 us unpipelined).
-template <typename R, int B = 8>
+// y_i = d_i x_i - sum_k a_ik x_j(k) over the stored entries of row i.  Groups
+// of 8 entries (rows are padded to whole groups, so nothing is predicated):
+// the next group's entries load while the current one's gathers are in
+// flight; even and odd entries have their own sums.  With a test per entry
+// and 8-byte loads a product ran 31 instructions per entry.
+template <typename R>
 __device__ __forceinline__ double kry_row(const KryWork<R>& K, int n, int i, int cnt, const double* __restrict__ xin) {
-    using E = KEnt<R>;
-    using T = typename E::T;
-    const T* __restrict__ ent = K.e + kent_at(i, 0, K.cap);   // entry k at ent[32 k]
+    using T = typename KEnt<R>::T;
+    const T* __restrict__ ent = K.e + kent_at(i, 0, K.cap);   // pair q at ent[64 q]
     (void)n;
-    T cur[B], nxt[B];
+    double s0 = 0, s1 = 0;
+    if (cnt > 0) {
+        KRaw<R> cur[4];
 #pragma unroll
-    for (int q = 0; q < B; q++)
-        if (q < cnt) cur[q] = __ldg(ent + (size_t)q * 32);
-    double acc = 0;
-    for (int k = 0; k < cnt; k += B) {
+        for (int q = 0; q < 4; q++) cur[q].load(ent + q * 64);
+        for (int k = 0; k < cnt; k += 8) {
+            KRaw<R> nxt[4];
+            ent += 256;
+            if (k + 8 < cnt) {
 #pragma unroll
-        for (int q = 0; q < B; q++)
-            if (k + B + q < cnt) nxt[q] = __ldg(ent + (size_t)(k + B + q) * 32);
-        double xv[B], av[B];
-#pragma unroll
-        for (int q = 0; q < B; q++) {
-            xv[q] = 0.0;
-            av[q] = 0.0;
-            if (k + q < cnt) {
-                int j;
-                E::get(cur[q], j, av[q]);
-                xv[q] = __ldg(xin + j);
+                for (int q = 0; q < 4; q++) nxt[q].load(ent + q * 64);
             }
+            double x0[4], x1[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const KPair e = cur[q].get();
+                x0[q] = __ldg(xin + e.j0);
+                x1[q] = __ldg(xin + e.j1);
+            }
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const KPair e = cur[q].get();
+                s0 += e.a0 * x0[q];
+                s1 += e.a1 * x1[q];
+            }
+#pragma unroll
+            for (int q = 0; q < 4; q++) cur[q] = nxt[q];
         }
-#pragma unroll
-        for (int q = 0; q < B; q++)
-            if (k + q < cnt) acc += av[q] * xv[q];
-#pragma unroll
-        for (int q = 0; q < B; q++) cur[q] = nxt[q];
     }
-    return K.d[i] * xin[i] - acc;
+    return K.d[i] * xin[i] - (s0 + s1);
 }
 
 // y = A x over the stored coefficients; optional fused dots
@@ -815,10 +863,11 @@ __global__ void __launch_bounds__(PROJ_T) k_proj_spmv(int n, KryWork<R> K, int f
             const int ne = cnt - 1;
             int k = 0;
             for (; k + 2 <= ne; k += 2) {
-                int j0, j1;
-                double a0, a1;
-                E::get(__ldg(er + (size_t)k * 32), j0, a0);
-                E::get(__ldg(er + (size_t)(k + 1) * 32), j1, a1);
+                KRaw<R> e;
+                e.load(er + (size_t)k * 32);
+                const KPair pr = e.get();
+                const int j0 = pr.j0, j1 = pr.j1;
+                const double a0 = pr.a0, a1 = pr.a1;
                 float4 p0 = __ldg(D4 + (size_t)j0 * 3), p1 = G > 1 ? __ldg(D4 + (size_t)j0 * 3 + 1) : z4,
                        p2 = G > 2 ? __ldg(D4 + (size_t)j0 * 3 + 2) : z4;
                 float4 q0 = __ldg(D4 + (size_t)j1 * 3), q1 = G > 1 ? __ldg(D4 + (size_t)j1 * 3 + 1) : z4,

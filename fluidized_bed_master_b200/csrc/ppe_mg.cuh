@@ -87,10 +87,12 @@ template <typename R>
 __global__ void __launch_bounds__(128) k_mg_assemble0(KryWork<R> K, MgWork M) {
     const MgLevel L0 = M.L[0];
     const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    // a lane's 27 sums in a shared column of its own (indexed by the entry)
+    __shared__ double s_acc[4][27 * 32];
+    double* acc = s_acc[threadIdx.x >> 5];
     if (c >= L0.n) return;
-    double acc[27];
 #pragma unroll
-    for (int q = 0; q < 27; q++) acc[q] = 0.0;
+    for (int q = 0; q < 27; q++) acc[q * 32 + lane] = 0.0;
     const int a0 = M.gs[c];
     if (a0 >= 0) {
         const int e0 = M.ge[c];
@@ -100,24 +102,41 @@ __global__ void __launch_bounds__(128) k_mg_assemble0(KryWork<R> K, MgWork M) {
             const int cnt = K.kcnt[i];
             if (!cnt) continue;
             const double w = K.wm[i];
-            acc[13] += w * K.d[i];
-            for (int k = 0; k < cnt - 1; k++) {
-                int j;
-                double a;
-                KEnt<R>::get(K.e[kent_at(i, k, K.cap)], j, a);
-                const long long pj = M.cxyz[j];
-                if (pj < 0) continue;
+            acc[13 * 32 + lane] += w * K.d[i];
+            auto add = [&](long long pj, double a) {
+                if (pj < 0) return;
                 const int dx = (int)(pj & 0x1FFFFF) - cx, dy = (int)((pj >> 21) & 0x1FFFFF) - cy,
                           dz = (int)(pj >> 42) - cz;
-                if (dx < -1 || dx > 1 || dy < -1 || dy > 1 || dz < -1 || dz > 1) continue;
-                acc[(dz + 1) * 9 + (dy + 1) * 3 + (dx + 1)] -= w * a;
+                if (dx < -1 || dx > 1 || dy < -1 || dy > 1 || dz < -1 || dz > 1) return;
+                acc[((dz + 1) * 9 + (dy + 1) * 3 + (dx + 1)) * 32 + lane] -= w * a;
+            };
+            // 8 entries at a time (the padding adds zeros to the row's own
+            // cell), their cells in flight together
+            const typename KEnt<R>::T* ent = K.e + kent_at(i, 0, K.cap);
+            for (int k = 0; k < cnt - 1; k += 8) {
+                KRaw<R> e[4];
+                long long c0[4], c1[4];
+#pragma unroll
+                for (int q = 0; q < 4; q++) e[q].load(ent + (size_t)k * 32 + q * 64);
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const KPair r = e[q].get();
+                    c0[q] = __ldg(M.cxyz + r.j0);
+                    c1[q] = __ldg(M.cxyz + r.j1);
+                }
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const KPair r = e[q].get();
+                    add(c0[q], r.a0);
+                    add(c1[q], r.a1);
+                }
             }
         }
     }
     double mine = 0.0;   // lane q keeps entry q
 #pragma unroll
     for (int q = 0; q < 27; q++) {
-        const double v = warp_sum(acc[q]);
+        const double v = warp_sum(acc[q * 32 + lane]);
         if (lane == q) mine = v;
     }
     if (lane < 27) L0.A[(size_t)c * 32 + lane] = mine;
