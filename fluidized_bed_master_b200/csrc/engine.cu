@@ -204,6 +204,10 @@ void alloc_work(Alloc& A, SphWork<R>& W, DemWork<double>& DW, int ns, int nd, in
     DW.ncs = A.get<int>(nd);
     DW.nbd = A.get<int>((size_t)nd * DEM_DEM_CAP);
     DW.ncd = A.get<int>(nd);
+    DW.ra = A.get<Dbl4>(nd);
+    DW.rb = A.get<Dbl4>(nd);
+    DW.rc = A.get<Dbl4>(nd);
+    DW.rd = A.get<double2>(nd);
     DW.dcs = A.get<double>((size_t)nd * 14);
     DW.dcf = A.get<int>(nd);
 }
@@ -304,7 +308,7 @@ int nnps_dem(SphdemHandle* H, EngineHost<R>* EH, int src, int dst, int64_t* nl, 
     }
     {
         KTIME_ON(KT_GATHER_D, st);
-        CK((launch_pdl(k_cells_gather_dem<double>, nblocks(n, TPB), TPB, 0, st, P, D, E.D[dst], DW.val_out)));
+        CK((launch_pdl(k_cells_gather_dem<double>, nblocks(n, TPB), TPB, 0, st, P, D, E.D[dst], DW.val_out, DW)));
         CK((launch_pdl(k_gather_history, nblocks(n * SPHDEM_NSLOT, TPB), TPB, 0, st, n, DW.val_out, D.hid, D.hds, E.D[dst].hid,
                                                                          E.D[dst].hds)));
     }
@@ -782,7 +786,7 @@ int enqueue_step(SphdemHandle* H, EngineHost<R>* EH, int flags, int64_t* nl) {
             *nl += 1;
         }
         CK(wait(1, st));
-        { KTIME(KT_PASSA); CK((launch_pdl(kt3 ? k_passA<R> : k_passA_any<R>, bs, TPB, 0, st, P, S, W, D, DW.rows))); }
+        { KTIME(KT_PASSA); CK((launch_pdl(kt3 ? k_passA<R> : k_passA_any<R>, bs, TPB, 0, st, P, S, W, D, DW, DW.rows))); }
         *nl += 1;
         {
             KTIME(KT_PASSB);

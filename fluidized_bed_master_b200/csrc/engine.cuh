@@ -89,6 +89,10 @@ struct DemWork {
     int4* rows;
     int *nbs, *ncs;              // SPH neighbours of each sphere (k_dem_prep): nbs[i*DEM_SPH_CAP+k], exact count
     int *nbd, *ncd;              // spheres within the search range (k_dem_near): nbd[i*DEM_DEM_CAP+k], exact count
+    // packed per sphere for the SPH passes: {x, y, z, radius}, {ux, uy, uz, m}
+    // (k_cells_gather_dem), {drag, fluid heat}, {flt_sd2, flt_s} (k_dem_finish)
+    Dbl4 *ra, *rb, *rc;
+    double2* rd;
     R* dcs;                      // 14*n pair sums of k_dem_coupling for k_dem_finish (DcSums, plane-major)
     int* dcf;                    // n: bit0 coupled, bit1 fluid seen, bit2 air seen; -1 not reached
 };

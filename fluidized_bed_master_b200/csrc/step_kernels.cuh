@@ -213,17 +213,23 @@ __global__ void k_refresh_sph(DevParams P, SphGatherSrc<R> g, SphState<R> S, Sph
 }
 
 template <typename R>
-__global__ void k_cells_gather_dem(DevParams P, DemState<R> src, DemState<R> dst, const int* __restrict__ perm) {
+__global__ void k_cells_gather_dem(DevParams P, DemState<R> src, DemState<R> dst, const int* __restrict__ perm,
+                                   DemWork<R> DW) {
     grid_dep_wait();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     int n = P.nd;
     if (i >= n) return;
     int p = perm[i];
-    dst.x[i] = src.x[p]; dst.y[i] = src.y[p]; dst.z[i] = src.z[p];
-    dst.h[i] = src.h[p]; dst.rad[i] = src.rad[p];
-    dst.ux[i] = src.ux[p]; dst.uy[i] = src.uy[p]; dst.uz[i] = src.uz[p];
+    const R x = src.x[p], y = src.y[p], z = src.z[p], rad = src.rad[p], m = src.m[p];
+    const R ux = src.ux[p], uy = src.uy[p], uz = src.uz[p];
+    dst.x[i] = x; dst.y[i] = y; dst.z[i] = z;
+    dst.h[i] = src.h[p]; dst.rad[i] = rad;
+    dst.ux[i] = ux; dst.uy[i] = uy; dst.uz[i] = uz;
+    // what the SPH passes read of a sphere
+    DW.ra[i] = Dbl4{x, y, z, rad};
+    DW.rb[i] = Dbl4{ux, uy, uz, m};
     dst.wx[i] = src.wx[p]; dst.wy[i] = src.wy[p]; dst.wz[i] = src.wz[p];
-    dst.m[i] = src.m[p]; dst.rho[i] = src.rho[p]; dst.ri[i] = src.ri[p];
+    dst.m[i] = m; dst.rho[i] = src.rho[p]; dst.ri[i] = src.ri[p];
     dst.temp[i] = src.temp[p]; dst.temp1[i] = src.temp1[p]; dst.temp2[i] = src.temp2[p]; dst.temp3[i] = src.temp3[p];
     dst.Fdx_df[i] = src.Fdx_df[p]; dst.Fdy_df[i] = src.Fdy_df[p]; dst.Fdz_df[i] = src.Fdz_df[p];
     dst.Q_sd[i] = src.Q_sd[p];
@@ -746,6 +752,65 @@ __global__ void __launch_bounds__(DL_WARPS * 32) k_build_dlist(DevParams P, cons
     }
 }
 
+// A walk over the SPH -> DEM list of particle i, two entries at a time: the
+// list entries and the spheres' records (load(j)) of both are in flight before
+// either is summed; one dependent chain per entry made this most of pass A on
+// beds whose spheres are small against the kernel.  Sums in list order.
+template <typename T, typename L, typename C>
+__device__ __forceinline__ void dem_walk(const int* __restrict__ nbrd, int cd, int n, int i, L load, C comp) {
+    int j0 = 0, j1 = 0;
+    if (cd > 0) j0 = nbrd[i];
+    if (cd > 1) j1 = nbrd[(size_t)n + i];
+    int k = 0;
+    for (; k + 2 <= cd; k += 2) {
+        const T r0 = load(j0), r1 = load(j1);
+        const int a = j0, b = j1;
+        if (k + 2 < cd) j0 = nbrd[(size_t)(k + 2) * n + i];
+        if (k + 3 < cd) j1 = nbrd[(size_t)(k + 3) * n + i];
+        comp(a, r0);
+        comp(b, r1);
+    }
+    if (k < cd) comp(j0, load(j0));
+}
+struct DemAB {
+    Dbl4 a, b;
+};
+// KERNEL_clc_prep3D_coupling_sph (functions_PREP2.cuh:3190-3364): the sums of
+// particle i over its spheres
+template <typename R, typename K>
+__device__ __forceinline__ void sph_dem_porosity(const DevParams& P, const SphWork<R>& W, const DemState<double>& D,
+                                                 const DemWork<double>& DW, const int4* __restrict__ drows, int i,
+                                                 double xi, double yi, double zi, double hi, const K& Kn, R& por,
+                                                 R& dfx, R& dfy, R& dfz) {
+    const double Rr = P.kappa * hi;
+    const float r2l = r2_lo(Rr), r2h = r2_hi(Rr);
+    const int n = P.ns;
+    auto load = [&](int j) { return DemAB{ldr(DW.ra + j), ldr(DW.rb + j)}; };
+    auto dem = [&](int, const DemAB& q) {
+        PairT<R> g = pair_test<R>(xi, yi, zi, q.a.x, q.a.y, q.a.z, Rr, 1e-20, r2l, r2h);
+        if (!g.in) return;
+        R r = g.r + (R)1e-20, ir = rcp(r);
+        R w = kw(Kn, r);
+        R dw = kdw(Kn, r);
+        R rj = (R)q.a.w;
+        R v = dem_measure(P, rj);
+        por += w * v;
+        dfx += dw * g.dx * ir * (R)q.b.x * v;
+        dfy += dw * g.dy * ir * (R)q.b.y * v;
+        dfz += dw * g.dz * ir * (R)q.b.z * v;
+    };
+    const int cd = W.ncntd[i];
+    if (cd <= P.nbd_cap) {
+        dem_walk<DemAB>(W.nbrd, cd, n, i, load, dem);
+    } else {
+        int ic, jc, kc;
+        cell_ijk(P, xi, yi, zi, ic, jc, kc);
+        for_stencil_j(P, ic, jc, kc, drows, make_cull(xi, yi, zi, Rr), [&](int j) {
+            if (D.ptype[j] > 1000) dem(j, load(j));
+        });
+    }
+}
+
 // ---------------------------------------------------------------------------
 // pass A: KERNEL_clc_mass_init_sph (functions_MASS.cuh:24-43),
 // KERNEL_clc_correction_KGC_3D_sph (functions_PREP2.cuh:452-568),
@@ -760,7 +825,7 @@ __global__ void __launch_bounds__(DL_WARPS * 32) k_build_dlist(DevParams P, cons
 // (spills), 86 at 7, 92 at 6.
 template <typename R>
 __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 7 : 1) k_passA(DevParams P, SphState<R> S, SphWork<R> W, DemState<double> D,
-                                               const int4* __restrict__ drows) {
+                                               DemWork<double> DW, const int4* __restrict__ drows) {
     grid_dep_wait();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     int n = P.ns;
@@ -847,35 +912,10 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 7 : 1) k_passA(DevParams
         W.Cm[(size_t)4 * n + i] = C.yz;
         W.Cm[(size_t)5 * n + i] = C.zz;
     }
-    // SPH-DEM porosity over the SPH -> DEM list (DEM arrays are small and
-    // L2-resident: plain loads)
-    double Rr = P.kappa * hi;
     R por = 0, dfx = 0, dfy = 0, dfz = 0;
     if (P.nd > 0) {
         const Knl<R, 3> Kd = knl_make<R, 3>(P, th);
-        float r2l = r2_lo(Rr), r2h = r2_hi(Rr);
-        auto dem = [&](int j) {
-            if (D.ptype[j] <= 1000) return;
-            PairT<R> g = pair_test<R>(xi, yi, zi, D.x[j], D.y[j], D.z[j], Rr, 1e-20, r2l, r2h);
-            if (!g.in) return;
-            R r = g.r + (R)1e-20, ir = rcp(r);
-            R w = kw(Kd, r);
-            R dw = kdw(Kd, r);
-            R rj = (R)D.rad[j];
-            R v = dem_measure(P, rj);
-            por += w * v;
-            dfx += dw * g.dx * ir * (R)D.ux[j] * v;
-            dfy += dw * g.dy * ir * (R)D.uy[j] * v;
-            dfz += dw * g.dz * ir * (R)D.uz[j] * v;
-        };
-        const int cd = W.ncntd[i];
-        if (cd <= P.nbd_cap) {
-            for (int k = 0; k < cd; k++) dem(W.nbrd[(size_t)k * n + i]);
-        } else {
-            int ic, jc, kc;
-            cell_ijk(P, xi, yi, zi, ic, jc, kc);
-            for_stencil_j(P, ic, jc, kc, drows, make_cull(xi, yi, zi, Rr), dem);
-        }
+        sph_dem_porosity(P, W, D, DW, drows, i, xi, yi, zi, hi, Kd, por, dfx, dfy, dfz);
     }
     R isf = rcp(sflt + (R)1e-20);
     R pori = (R)1 - por * isf;
@@ -1931,6 +1971,9 @@ __global__ void __launch_bounds__(128) k_dem_finish(DevParams P, DemState<double
     a.has_f = (f >> 1) & 1;
     a.has_a = (f >> 2) & 1;
     dem_coupling_finish(P, D, DW, i, (f & 1) != 0, a);
+    // what the reaction force reads of a sphere
+    DW.rc[i] = Dbl4{D.Fdx_df[i], D.Fdy_df[i], D.Fdz_df[i], D.Q_sd[i]};
+    DW.rd[i] = make_double2(DW.flt_sd2[i], DW.flt_s[i]);
 }
 
 // ---------------------------------------------------------------------------
@@ -1959,28 +2002,35 @@ __global__ void __launch_bounds__(128) k_sph_coupling(DevParams P, SphState<R> S
         R tx = 0, ty = 0, tz = 0, tt = 0;
         if (P.nd > 0 && (pt == 1 || pt == 3)) {
             float r2l = r2_lo(Rr), r2h = r2_hi(Rr);
-            auto dem = [&](int j) {
-                if (D.ptype[j] <= 1000) return;
-                PairT<R> g = pair_test<R>(xi, yi, zi, D.x[j], D.y[j], D.z[j], Rr, 0.0, r2l, r2h);
+            struct Rec {
+                Dbl4 a, c;
+                double2 f;
+                double m;
+            };
+            auto load = [&](int j) { return Rec{ldr(DW.ra + j), ldr(DW.rc + j), ldr(DW.rd + j), ldr(&DW.rb[j].w)}; };
+            auto dem = [&](int, const Rec& q) {
+                PairT<R> g = pair_test<R>(xi, yi, zi, q.a.x, q.a.y, q.a.z, Rr, 0.0, r2l, r2h);
                 if (!g.in) return;
-                R ffj = (R)DW.flt_sd2[j] + (R)DW.flt_s[j];
+                R ffj = (R)q.f.x + (R)q.f.y;
                 if (!(ffj > (R)0)) return;
                 R w = kw(K, g.r);
-                if (P.dim == 2) w *= (R)0.75 / (R)D.rad[j];   // per unit depth (depth 4 r / 3)
+                if (P.dim == 2) w *= (R)0.75 / (R)q.a.w;   // per unit depth (depth 4 r / 3)
                 R c = w / (ffj + (R)1.0e-20);
-                R mr = (R)D.m[j] / rhoi;
-                tx += -mr * (R)D.Fdx_df[j] * c;
-                ty += -mr * (R)D.Fdy_df[j] * c;
-                tz += -mr * (R)D.Fdz_df[j] * c;
-                tt += -(R)D.Q_sd[j] / (rhoi * cpi) * c;
+                R mr = (R)q.m / rhoi;
+                tx += -mr * (R)q.c.x * c;
+                ty += -mr * (R)q.c.y * c;
+                tz += -mr * (R)q.c.z * c;
+                tt += -(R)q.c.w / (rhoi * cpi) * c;
             };
             const int cd = W.ncntd[i];
             if (cd <= P.nbd_cap) {
-                for (int k = 0; k < cd; k++) dem(W.nbrd[(size_t)k * n + i]);
+                dem_walk<Rec>(W.nbrd, cd, n, i, load, dem);
             } else {
                 int ic, jc, kc;
                 cell_ijk(P, xi, yi, zi, ic, jc, kc);
-                for_stencil_j(P, ic, jc, kc, drows, make_cull(xi, yi, zi, Rr), dem);
+                for_stencil_j(P, ic, jc, kc, drows, make_cull(xi, yi, zi, Rr), [&](int j) {
+                    if (D.ptype[j] > 1000) dem(j, load(j));
+                });
             }
         }
         ftx += tx;
@@ -2919,7 +2969,7 @@ __device__ __forceinline__ void cm_store(R* Cm, int n, int i, const R* C) {
 }
 template <typename R>
 __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 8 : 1) k_passA_any(DevParams P, SphState<R> S, SphWork<R> W, DemState<double> D,
-                                               const int4* __restrict__ drows) {
+                                               DemWork<double> DW, const int4* __restrict__ drows) {
     grid_dep_wait();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     int n = P.ns;
@@ -3003,34 +3053,9 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 8 : 1) k_passA_any(DevPa
         }
         cm_store(W.Cm, n, i, C);
     }
-    // SPH-DEM porosity over the SPH -> DEM list (DEM arrays are small and
-    // L2-resident: plain loads)
-    double Rr = P.kappa * hi;
     R por = 0, dfx = 0, dfy = 0, dfz = 0;
     if (P.nd > 0) {
-        float r2l = r2_lo(Rr), r2h = r2_hi(Rr);
-        auto dem = [&](int j) {
-            if (D.ptype[j] <= 1000) return;
-            PairT<R> g = pair_test<R>(xi, yi, zi, D.x[j], D.y[j], D.z[j], Rr, 1e-20, r2l, r2h);
-            if (!g.in) return;
-            R r = g.r + (R)1e-20, ir = rcp(r);
-            R w = kw(K, r);
-            R dw = kdw(K, r);
-            R rj = (R)D.rad[j];
-            R v = dem_measure(P, rj);
-            por += w * v;
-            dfx += dw * g.dx * ir * (R)D.ux[j] * v;
-            dfy += dw * g.dy * ir * (R)D.uy[j] * v;
-            dfz += dw * g.dz * ir * (R)D.uz[j] * v;
-        };
-        const int cd = W.ncntd[i];
-        if (cd <= P.nbd_cap) {
-            for (int k = 0; k < cd; k++) dem(W.nbrd[(size_t)k * n + i]);
-        } else {
-            int ic, jc, kc;
-            cell_ijk(P, xi, yi, zi, ic, jc, kc);
-            for_stencil_j(P, ic, jc, kc, drows, make_cull(xi, yi, zi, Rr), dem);
-        }
+        sph_dem_porosity(P, W, D, DW, drows, i, xi, yi, zi, hi, K, por, dfx, dfy, dfz);
     }
     R isf = rcp(sflt + (R)1e-20);
     R pori = (R)1 - por * isf;
