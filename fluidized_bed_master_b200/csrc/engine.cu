@@ -734,7 +734,7 @@ int enqueue_step(SphdemHandle* H, EngineHost<R>* EH, int flags, int64_t* nl) {
     // Wendland C2 (the configurations' kernel) has its own forms of the
     // neighbour passes; the other kernels run the general ones, whose sums
     // keep the reference's form pair by pair
-    const bool kt3 = P.kernel_type == 3;
+    const bool kt3 = P.kernel_type == 3, kt5 = P.kernel_type == 5;
     const bool fork = H->concurrent && ns > 0 && nd > 0 && H->dem_stream;
     cudaStream_t sd = fork ? H->dem_stream : st;
     // event k recorded on stream a / waited for on stream b (fork only)
@@ -786,7 +786,7 @@ int enqueue_step(SphdemHandle* H, EngineHost<R>* EH, int flags, int64_t* nl) {
             *nl += 1;
         }
         CK(wait(1, st));
-        { KTIME(KT_PASSA); CK((launch_pdl(kt3 ? k_passA<R> : k_passA_any<R>, bs, TPB, 0, st, P, S, W, D, DW, DW.rows))); }
+        { KTIME(KT_PASSA); CK((launch_pdl(kt3 ? k_passA<R> : kt5 ? k_passA_any<R, 5> : k_passA_any<R, -1>, bs, TPB, 0, st, P, S, W, D, DW, DW.rows))); }
         *nl += 1;
         {
             KTIME(KT_PASSB);
@@ -794,9 +794,9 @@ int enqueue_step(SphdemHandle* H, EngineHost<R>* EH, int flags, int64_t* nl) {
                 CK((launch_pdl(kt3 ? k_sps<R, 3> : k_sps<R, -1>, bs, TPB, 0, st, P, S, W)));
                 *nl += 1;
             }
-            auto kb = !kt3 ? k_passB_any<R, false> : P.con ? k_passB<R, true> : k_passB<R, false>;
-            if (P.iface | P.fb | P.sps | P.ipf) kb = k_passB_any<R, true>;
-            else if (P.fva) kb = k_passB_any<R, false>;
+            auto kb = kt5 ? k_passB_any<R, false, 5> : !kt3 ? k_passB_any<R, false, -1> : P.con ? k_passB<R, true> : k_passB<R, false>;
+            if (P.iface | P.fb | P.sps | P.ipf) kb = k_passB_any<R, true, -1>;
+            else if (P.fva) kb = k_passB_any<R, false, -1>;
             CK((launch_pdl(kb, bs, TPB, 0, st, P, S, W, E.flags)));
         }
         *nl += 1;
@@ -817,7 +817,7 @@ int enqueue_step(SphdemHandle* H, EngineHost<R>* EH, int flags, int64_t* nl) {
     }
     if (ns > 0) {
         KTIME(KT_SPHCOUPLING);
-        CK((launch_pdl(kt3 ? k_sph_coupling<R, 3> : k_sph_coupling<R, -1>, bs, TPB, 0, st, P, S, W, D, DW, DW.rows, (flags & F_TIME0) ? 1 : 0)));
+        CK((launch_pdl(kt3 ? k_sph_coupling<R, 3> : kt5 ? k_sph_coupling<R, 5> : k_sph_coupling<R, -1>, bs, TPB, 0, st, P, S, W, D, DW, DW.rows, (flags & F_TIME0) ? 1 : 0)));
         *nl += 1;
     }
     CK(rec(4, st));   // the SPH coupling has read the DEM set
@@ -834,23 +834,23 @@ int enqueue_step(SphdemHandle* H, EngineHost<R>* EH, int flags, int64_t* nl) {
         }
         {
             KTIME(KT_PPE);
-            if (H->p.ppe_mode == SPHDEM_PPE_REFERENCE) CK((launch_pdl(kt3 ? k_ppe<R> : k_ppe_any<R>, bs, TPB, 0, st, P, S, W)));
+            if (H->p.ppe_mode == SPHDEM_PPE_REFERENCE) CK((launch_pdl(kt3 ? k_ppe<R> : kt5 ? k_ppe_any<R, 5> : k_ppe_any<R, -1>, bs, TPB, 0, st, P, S, W)));
             else if ((r = enqueue_krylov<R>(H, EH, S, W))) return r;
         }
         {
             KTIME(KT_NEUMANN);
             CK(launch_neumann<R>(E, S, W.p_new, 0, st));
         }
-        { KTIME(KT_PASSC); CK((launch_pdl(kt3 ? k_passC<R> : k_passC_any<R>, bs, TPB, 0, st, P, S, W))); }
+        { KTIME(KT_PASSC); CK((launch_pdl(kt3 ? k_passC<R> : kt5 ? k_passC_any<R, 5> : k_passC_any<R, -1>, bs, TPB, 0, st, P, S, W))); }
         *nl += 3;
         if (P.open_bc > 0) {
             KTIME(KT_OPENBC);
-            CK((launch_pdl(kt3 ? k_open_bc<R, 3> : k_open_bc<R, -1>, bbw, TPB, 0, st, P, S, W, W.rows)));
+            CK((launch_pdl(kt3 ? k_open_bc<R, 3> : kt5 ? k_open_bc<R, 5> : k_open_bc<R, -1>, bbw, TPB, 0, st, P, S, W, W.rows)));
             *nl += 1;
         }
         if (P.xsph) {
             KTIME(KT_XSPH);
-            CK((launch_pdl(kt3 ? k_xsph<R> : k_xsph_any<R>, bs, TPB, 0, st, P, S, W)));
+            CK((launch_pdl(kt3 ? k_xsph<R> : kt5 ? k_xsph_any<R, 5> : k_xsph_any<R, -1>, bs, TPB, 0, st, P, S, W)));
             *nl += 1;
         }
     }

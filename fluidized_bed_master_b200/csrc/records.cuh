@@ -316,10 +316,11 @@ __device__ __forceinline__ double fdiv(double a, double b) { return a / b; }
 // ---- smoothing kernel with per-particle constants -----------------------
 // W and dW/dr of functions_KNL.cuh:2-144 with 1/h precomputed.
 // KT is the kernel type when the kernel instantiation fixes it (3: Wendland
-// C2, the loops then carry no type test), -1 when it is read from kt.
+// C2, 5: Wendland C6; the loops then carry no type test), -1 when it is read
+// from kt.
 template <typename R, int KT = -1>
 struct Knl {
-    static_assert(KT == -1 || KT == 3, "kernel types fixed at compile time: Wendland C2");
+    static_assert(KT == -1 || KT == 3 || KT == 5, "kernel types fixed at compile time: Wendland C2 and C6");
     int kt;
     R tA, ih, th;   // normalisation, 1/h, h
 };
@@ -346,39 +347,39 @@ __device__ __noinline__ R knl_dw_call(int kt, R tA, R tH, R rr) {
 }
 template <typename R, int KT>
 __device__ __forceinline__ R kw(const Knl<R, KT>& k, R rr) {
-    if (KT == 3 || k.kt == 3) {
+    if (KT == 3 || (KT == -1 && k.kt == 3)) {
         R q = rr * k.ih * (R)0.5;
         if (!(q < (R)1)) return (R)0;
         R a = (R)1 - q, a2 = a * a;
         return k.tA * a2 * a2 * ((R)1 + (R)4 * q);
     }
-    if constexpr (KT == -1) {
-        if (k.kt == 5) {
+    if constexpr (KT != 3) {
+        if (KT == 5 || k.kt == 5) {
             R q = rr * k.ih * (R)0.5;
             if (!(q < (R)1)) return (R)0;
             R a = (R)1 - q, a2 = a * a, a4 = a2 * a2;
             return k.tA * a4 * a4 * ((R)1 + (R)8 * q + (R)25 * q * q + (R)32 * q * q * q);
         }
-        return knl_w_call<R>(k.kt, k.tA, k.th, rr);
+        if constexpr (KT == -1) return knl_w_call<R>(k.kt, k.tA, k.th, rr);
     }
     return (R)0;
 }
 template <typename R, int KT>
 __device__ __forceinline__ R kdw(const Knl<R, KT>& k, R rr) {
-    if (KT == 3 || k.kt == 3) {
+    if (KT == 3 || (KT == -1 && k.kt == 3)) {
         R q = rr * k.ih * (R)0.5;
         if (!(q < (R)1)) return (R)0;
         R a = (R)1 - q;
         return ((R)0.5 * k.ih) * k.tA * ((R)-20 * q * a * a * a);
     }
-    if constexpr (KT == -1) {
-        if (k.kt == 5) {
+    if constexpr (KT != 3) {
+        if (KT == 5 || k.kt == 5) {
             R q = rr * k.ih * (R)0.5;
             if (!(q < (R)1)) return (R)0;
             R a = (R)1 - q, a2 = a * a, a4 = a2 * a2;
             return ((R)0.5 * k.ih) * k.tA * ((R)-22 * q * a4 * a2 * a * ((R)16 * q * q + (R)7 * q + (R)1));
         }
-        return knl_dw_call<R>(k.kt, k.tA, k.th, rr);
+        if constexpr (KT == -1) return knl_dw_call<R>(k.kt, k.tA, k.th, rr);
     }
     return (R)0;
 }
@@ -603,31 +604,28 @@ __device__ __forceinline__ void nb_sum(int cnt, const int* __restrict__ nb, int 
     if (k < cnt) batch(e0, cnt - k);
 }
 
-// the same list, one entry after another in batches of B (passes that keep
-// per-pair control flow)
+// the same list in batches of 4 for the passes that keep per-pair control
+// flow; entries requested one batch ahead
 template <int B, typename T, typename L, typename C>
 __device__ __forceinline__ void nb_walk(int cnt, const int* __restrict__ nb, int n, int i, L load, C comp) {
-    static_assert(B == 2 || B == 4, "list walks load 2 or 4 entries at a time");
+    static_assert(B == 4, "list walks load 4 entries at a time");
+    if (cnt <= 0) return;
     int k = 0;
-    for (; k + B <= cnt; k += B) {
-        int j[B];
-        T r[B];
-        if constexpr (B == 4) {
-            const int4 v = __ldg(reinterpret_cast<const int4*>(nb + nb_at(k, n, i)));
-            j[0] = v.x; j[1] = v.y; j[2] = v.z; j[3] = v.w;
-        } else {
-            const int2 v = __ldg(reinterpret_cast<const int2*>(nb + nb_at(k, n, i)));
-            j[0] = v.x; j[1] = v.y;
-        }
+    int4 v = nb_ld4(nb + nb_at(0, n, i));
+    for (; k + 4 <= cnt; k += 4) {
+        const int j[4] = {v.x, v.y, v.z, v.w};
+        if (k + 4 < cnt) v = nb_ld4(nb + nb_at(k + 4, n, i));
+        T r[4];
 #pragma unroll
-        for (int u = 0; u < B; u++) r[u] = load(j[u]);
+        for (int u = 0; u < 4; u++) r[u] = load(j[u]);
 #pragma unroll
-        for (int u = 0; u < B; u++) comp(j[u], r[u]);
+        for (int u = 0; u < 4; u++) comp(j[u], r[u]);
     }
     for (; k < cnt; k++) {
-        int j = __ldg(nb + nb_at(k, n, i));
-        T r = load(j);
-        comp(j, r);
+        const T r = load(v.x);
+        comp(v.x, r);
+        v.x = v.y;
+        v.y = v.z;
     }
 }
 

@@ -2269,6 +2269,31 @@ __device__ __forceinline__ void neumann_cell(int c, DevParams P, SphState<float>
                     }
                 }
                 scale = K.tA;
+            } else if (act && !slow_chunk && K.kt == 5) {
+                // Wendland C6 in line, no branches between the candidates
+                Knl<float, 5> K5{K.kt, K.tA, K.ih, K.th};
+#pragma unroll 4
+                for (int u = 0; u < ns; u++) {
+                    const float4 cj = saw[u];
+                    const float dx = fx - cj.x, dy = fy - cj.y, dz = fz - cj.z;
+                    const float r2 = dx * dx + dy * dy + dz * dz;
+                    bool in = r2 < lo2;
+                    if (!in && r2 <= hi2) {
+                        const int j = __float_as_int(cj.w);
+                        in = __dadd_rn(pair_dist(xi, yi, zi, S.x[j], S.y[j], S.z[j]), 1e-20) < R2;
+                    }
+                    float r, rinv;
+                    rdist(r2, r, rinv);
+                    const float wk = kw(K5, r);
+                    const float4 bj = sbw[u];
+                    if (in) {
+                        const float mr = bj.x * wk;
+                        tp += mr * bj.y;
+                        flt += mr;
+                        tt += mr * bj.z;
+                        tr += bj.w * wk;
+                    }
+                }
             } else if (act && !slow_chunk) {
                 // as above, any kernel
 #pragma unroll 2
@@ -2807,6 +2832,7 @@ __global__ void __launch_bounds__(128) k_dem_update(DevParams P, DemState<R> D, 
 // around their mirror point.  Only non-buffer fluid is read, so the update
 // is done in place.  One warp per buffer particle (W.buf_idx).
 // ---------------------------------------------------------------------------
+constexpr int OB_Q = 8;   // queued hits per lane
 template <typename R, int KT>
 __global__ void __launch_bounds__(128) k_open_bc(DevParams P, SphState<R> S, SphWork<R> W, const int4* __restrict__ rows) {
     grid_dep_wait();
@@ -2832,27 +2858,50 @@ __global__ void __launch_bounds__(128) k_open_bc(DevParams P, SphState<R> S, Sph
     R trho = 0, tp = 0, tux = 0, tuy = 0, tuz = 0, tt = 0, flt = 0;
     const Cull cu = make_cull(xi, yi, zg, Rr);
     // the candidate's type and the prefilter from its packed record (one
-    // load); the FP64 predicate only inside the band
-    for_rows_warp(P, ic, jc, kc, rows, cu, sm, lane, [&](int j) {
-        const PosRec<R> qj = ldr(W.rec.pos + j);
-        if (tag_ptype(qj.w) != 1 || tag_btype(qj.w) != 0) return;
-        Disp<R> d;
-        R r2;
-        if (!test_pair(P, qp, qj, xi, yi, zg, S.x, S.y, S.z, j, Rr, 1e-20, bd, d, r2)) return;
-        R r, rinv;
-        rdist(r2, r, rinv);
-        R wk = kw(K, r);
-        R hj = (R)S.h[j];
-        R volj = sph_volume(P, hj, hd);
-        R vw = volj * wk;
-        trho += W.rho_new[j] / W.DEMpor[j] * wk * volj;
-        tp += vw * W.p_new[j];
-        tuz += vw * S.uz[j];
-        tux += vw * S.ux[j];
-        tuy += vw * S.uy[j];
-        tt += vw * S.temp[j];
-        flt += vw;
+    // load); the FP64 predicate only inside the band.  A lane queues its hits
+    // and the warp sums them when a queue is full and at the end, all lanes
+    // together: summed where they were found, a few lanes at a time ran the
+    // seven sums in nearly every round.  Each lane's sums keep their order.
+    __shared__ int s_q[4][OB_Q][32];
+    int(*qu)[32] = s_q[threadIdx.x >> 5];
+    int nq = 0;
+    auto flush = [&]() {
+        const int m = __reduce_max_sync(0xffffffffu, nq);
+        for (int k = 0; k < m; k++) {
+            if (k >= nq) continue;
+            const int j = qu[k][lane];
+            const PosRec<R> qj = ldr(W.rec.pos + j);
+            const Disp<R> d = disp_pt(P, qp, qj, xi, yi, zg, S.x, S.y, S.z, j);
+            const R r2 = d.dx * d.dx + d.dy * d.dy + d.dz * d.dz;
+            R r, rinv;
+            rdist(r2, r, rinv);
+            R wk = kw(K, r);
+            R hj = (R)S.h[j];
+            R volj = sph_volume(P, hj, hd);
+            R vw = volj * wk;
+            trho += W.rho_new[j] / W.DEMpor[j] * wk * volj;
+            tp += vw * W.p_new[j];
+            tuz += vw * S.uz[j];
+            tux += vw * S.ux[j];
+            tuy += vw * S.uy[j];
+            tt += vw * S.temp[j];
+            flt += vw;
+        }
+        nq = 0;
+    };
+    for_rows_warp_all(P, ic, jc, kc, rows, cu, sm, lane, [&](int j) {
+        bool in = false;
+        if (j >= 0) {
+            const PosRec<R> qj = ldr(W.rec.pos + j);
+            Disp<R> d;
+            R r2;
+            in = tag_ptype(qj.w) == 1 && tag_btype(qj.w) == 0 &&
+                 test_pair(P, qp, qj, xi, yi, zg, S.x, S.y, S.z, j, Rr, 1e-20, bd, d, r2);
+        }
+        if (in) qu[nq++][lane] = j;
+        if (__any_sync(0xffffffffu, nq == OB_Q)) flush();
     });
+    flush();
     trho = warp_sum(trho); tp = warp_sum(tp); tux = warp_sum(tux); tuy = warp_sum(tuy);
     tuz = warp_sum(tuz); tt = warp_sum(tt); flt = warp_sum(flt);
     if (lane != 0 || P.open_bc != 1) return;
@@ -2967,7 +3016,7 @@ __device__ __forceinline__ void cm_store(R* Cm, int n, int i, const R* C) {
     Cm[(size_t)4 * n + i] = C[5];
     Cm[(size_t)5 * n + i] = C[8];
 }
-template <typename R>
+template <typename R, int KT>
 __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 8 : 1) k_passA_any(DevParams P, SphState<R> S, SphWork<R> W, DemState<double> D,
                                                DemWork<double> DW, const int4* __restrict__ drows) {
     grid_dep_wait();
@@ -2987,7 +3036,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 8 : 1) k_passA_any(DevPa
     W.dDEMpor_prev[i] = dprev;
     double xi = S.x[i], yi = S.y[i], zi = S.z[i], hi = S.h[i];
     R th = (R)hi;
-    Knl<R> K = knl_make<R>(P, th);
+    Knl<R, KT> K = knl_make<R, KT>(P, th);
     PosRec<R> qi = ldr(rec.pos + i);
     int cnt = min(W.ncnt[i], P.nb_cap);
     R txx = 0, tyy = 0, tzz = 0, txy = 0, tyz = 0, tzx = 0, sflt = 0;
@@ -3081,7 +3130,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 8 : 1) k_passA_any(DevPa
     rec.f1[i] = mk4<R>(mn, rn, S.temp[i], pori);
 }
 
-template <typename R, bool FORCES>
+template <typename R, bool FORCES, int KT>
 __global__ void __launch_bounds__(128) k_passB_any(DevParams P, SphState<R> S, SphWork<R> W, const DevFlags* F) {
     grid_dep_wait();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -3098,7 +3147,7 @@ __global__ void __launch_bounds__(128) k_passB_any(DevParams P, SphState<R> S, S
     bool adv = !(P.open_bc > 0 && bt > 0) && pt < 1000 && pt > 0;
     if (!filt && !adv) return;
     R th = (R)S.h[i];
-    Knl<R> K = knl_make<R>(P, th);
+    Knl<R, KT> K = knl_make<R, KT>(P, th);
     PosRec<R> qi = ldr(rec.pos + i);
     V4<R> upi = rec.up[i];
     V4<R> fi = rec.f1[i];
@@ -3229,7 +3278,7 @@ __global__ void __launch_bounds__(128) k_passB_any(DevParams P, SphState<R> S, S
     if ((P.con != 0)) W.dtemp[i] = Rc / (R)P.cp_sph * (R)(pt != -1) - et;
 }
 
-template <typename R>
+template <typename R, int KT>
 __global__ void __launch_bounds__(128) k_ppe_any(DevParams P, SphState<R> S, SphWork<R> W) {
     grid_dep_wait();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -3244,7 +3293,7 @@ __global__ void __launch_bounds__(128) k_ppe_any(DevParams P, SphState<R> S, Sph
         return;
     }
     R th = (R)S.h[i];
-    Knl<R> K = knl_make<R>(P, th);
+    Knl<R, KT> K = knl_make<R, KT>(P, th);
     PosRec<R> qi = ldr(rec.pos + i);
     V4<R> fi = rec.f1[i];
     R uxi = upi.x, uyi = upi.y, uzi = upi.z, rhoi = fi.y, pori = fi.w;
@@ -3289,7 +3338,7 @@ __global__ void __launch_bounds__(128) k_ppe_any(DevParams P, SphState<R> S, Sph
     W.p_new[i] = (b + AP) / A;
 }
 
-template <typename R>
+template <typename R, int KT>
 __global__ void __launch_bounds__(128) k_passC_any(DevParams P, SphState<R> S, SphWork<R> W) {
     grid_dep_wait();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -3306,7 +3355,7 @@ __global__ void __launch_bounds__(128) k_passC_any(DevParams P, SphState<R> S, S
     bool pf = !(P.open_bc > 0 && bt > 0) && pt < 1000 && pt > 0;
     if (pf && (P.fp != 0)) {
         R th = (R)S.h[i];
-        Knl<R> K = knl_make<R>(P, th);
+        Knl<R, KT> K = knl_make<R, KT>(P, th);
         PosRec<R> qi = ldr(rec.pos + i);
         R pi = W.p_new[i], rhoi = W.rho_new[i], pori = rec.f1[i].w;
         R cpi = -pori * rcp(rhoi);
@@ -3372,7 +3421,7 @@ __global__ void __launch_bounds__(128) k_passC_any(DevParams P, SphState<R> S, S
     rec.ut[i] = mk4<R>(uxc, uyc, uzc, tn);
 }
 
-template <typename R>
+template <typename R, int KT>
 __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 6 : 1) k_xsph_any(DevParams P, SphState<R> S, SphWork<R> W) {
     grid_dep_wait();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -3387,7 +3436,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 6 : 1) k_xsph_any(DevPar
         return;
     }
     R th = (R)S.h[i];
-    Knl<R> K = knl_make<R>(P, th);
+    Knl<R, KT> K = knl_make<R, KT>(P, th);
     PosRec<R> qi = ldr(rec.pos + i);
     R c = (R)P.c_xsph;
     int cnt = min(W.ncnt[i], P.nb_cap);
