@@ -1025,13 +1025,13 @@ __global__ void __launch_bounds__(128) k_dem_prep(DevParams P, SphState<R> S, Sp
         DW.ncs[i] = cs;
         for_stencil_j(P, ic, jc, kc, drows, cu, dem_por);
     } else {
-    for_rows_warp_all(P, ic, jc, kc, srows, cu, sm, lane, [&](int j) {
+    auto pos = [&](int j) { return ldr(rec.pos + j); };
+    for_rows_warp_pre<PosRec<R>>(P, ic, jc, kc, srows, cu, sm, lane, pos, [&](int j, const PosRec<R>& qj) {
         bool in = false, in20 = false;
         int ptj = 0;
         Disp<R> d;
         R r2 = 0;
         if (j >= 0) {
-            const PosRec<R> qj = ldr(rec.pos + j);
             ptj = tag_ptype(qj.w);
             if (ptj <= 1000) test_pair2(P, qp, qj, xi, yi, zi, S.x, S.y, S.z, j, Rr, bd, d, r2, in, in20);
         }
@@ -1095,10 +1095,10 @@ __global__ void __launch_bounds__(128) k_dem_prep_c2(DevParams P, SphState<R> S,
     // the sphere's SPH neighbours (p_type <= 1000, the add = 0 form of the
     // predicate, which k_dem_coupling_c2 uses), in visit order
     int cs = 0;
-    for_rows_warp_all(P, ic, jc, kc, srows, cu, sm, lane, [&](int j) {
+    auto pos = [&](int j) { return ldr(rec.pos + j); };
+    for_rows_warp_pre<PosRec<R>>(P, ic, jc, kc, srows, cu, sm, lane, pos, [&](int j, const PosRec<R>& qj) {
         bool in = false;
         if (j >= 0) {
-            const PosRec<R> qj = ldr(rec.pos + j);
             Disp<R> d;
             R r2;
             in = tag_ptype(qj.w) <= 1000 && test_pair(P, qp, qj, xi, yi, zi, S.x, S.y, S.z, j, Rr, 0.0, bd, d, r2);
@@ -1370,10 +1370,16 @@ __global__ void __launch_bounds__(128) k_dem_near(DevParams P, DemState<double> 
     cell_ijk(P, xi, yi, zi, ic, jc, kc);
     const unsigned lt = (1u << lane) - 1u;
     int c = 0;
-    for_rows_warp_all(P, ic, jc, kc, drows, make_cull(xi, yi, zi, R), s_rows[threadIdx.x >> 5], lane, [&](int j) {
+    struct Cand {
+        Dbl4 a;
+        int pt;
+    };
+    auto load = [&](int j) { return Cand{ldr(DW.ra + j), __ldg(D.ptype + j)}; };
+    for_rows_warp_pre<Cand>(P, ic, jc, kc, drows, make_cull(xi, yi, zi, R), s_rows[threadIdx.x >> 5], lane, load,
+                            [&](int j, const Cand& q) {
         bool in = false;
-        if (j >= 0 && __ldg(D.ptype + j) > 1000) {
-            const double xj = __ldg(D.x + j), yj = __ldg(D.y + j), zj = __ldg(D.z + j);
+        if (j >= 0 && q.pt > 1000) {
+            const double xj = q.a.x, yj = q.a.y, zj = q.a.z;
             const double dx = xi - xj, dy = yi - yj, dz = zi - zj, d2 = dx * dx + dy * dy + dz * dz;
             in = d2 < lo;
             if (!in && !(d2 > hi)) in = pair_dist(xi, yi, zi, xj, yj, zj) < R;
@@ -2889,10 +2895,10 @@ __global__ void __launch_bounds__(128) k_open_bc(DevParams P, SphState<R> S, Sph
         }
         nq = 0;
     };
-    for_rows_warp_all(P, ic, jc, kc, rows, cu, sm, lane, [&](int j) {
+    auto pos = [&](int j) { return ldr(W.rec.pos + j); };
+    for_rows_warp_pre<PosRec<R>>(P, ic, jc, kc, rows, cu, sm, lane, pos, [&](int j, const PosRec<R>& qj) {
         bool in = false;
         if (j >= 0) {
-            const PosRec<R> qj = ldr(W.rec.pos + j);
             Disp<R> d;
             R r2;
             in = tag_ptype(qj.w) == 1 && tag_btype(qj.w) == 0 &&
