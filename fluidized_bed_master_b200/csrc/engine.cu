@@ -543,11 +543,15 @@ inline cudaError_t launch_neumann_tiled(Engine<float>& E, const SphState<float>&
     const DevParams& P = E.P;
     SphWork<float>& W = E.sw;
     if (cell_sort_sparse(E.cs_s, P.ns))
-        return launch_pdl(k_neumann_tiled<true>, (occ_warps(P) + NT_WARPS - 1) / NT_WARPS, NT_WARPS * 32, 0, st, P,
-                          S, W, pres, (const int*)W.g_str, (const int*)W.g_end, (const int4*)W.rows, patch_up,
+        return launch_pdl(P.kernel_type == 5 ? k_neumann_tiled<true, 5> : k_neumann_tiled<true, -1>, (occ_warps(P) + NT_WARPS - 1) / NT_WARPS, NT_WARPS * 32, 0, st, P,
+                          S, W, pres, (const int*)W.g_str, (const int*)W.g_end, (const int4*)W.rows, patch_up, 1,
                           (const int*)E.cs_s.occ, (const int*)E.cs_s.occ_n);
-    return launch_pdl(k_neumann_tiled<false>, (P.NI * P.NJ * P.NK + NT_WARPS - 1) / NT_WARPS, NT_WARPS * 32, 0, st,
-                      P, S, W, pres, (const int*)W.g_str, (const int*)W.g_end, (const int4*)W.rows, patch_up,
+    // Fewer than 64 warps per SM with a warp per cell: two per cell, so that a
+    // cell of more than 32 particles is not one warp's serial work (spouted bed
+    // 174 -> 122 us; with more cells the second warp only exits).
+    const int ncell = P.NI * P.NJ * P.NK, parts = ncell < 148 * 64 ? 2 : 1;
+    return launch_pdl(P.kernel_type == 5 ? k_neumann_tiled<false, 5> : k_neumann_tiled<false, -1>, (ncell * parts + NT_WARPS - 1) / NT_WARPS, NT_WARPS * 32, 0, st,
+                      P, S, W, pres, (const int*)W.g_str, (const int*)W.g_end, (const int4*)W.rows, patch_up, parts,
                       (const int*)nullptr, (const int*)nullptr);
 }
 

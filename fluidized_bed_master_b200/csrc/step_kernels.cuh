@@ -2168,13 +2168,17 @@ __global__ void __launch_bounds__(128) k_neumann(DevParams P, SphState<R> S, Sph
 // order per wall, so the FP32 results differ from it by rounding only.
 constexpr int NT_WARPS = 4, NT_CH = 128;
 // one cell of k_neumann_tiled (saw, sbw, srw: the warp's shared staging)
+template <int KT>   // 5: Wendland C6; -1: the others
 __device__ __forceinline__ void neumann_cell(int c, DevParams P, SphState<float> S, SphWork<float> W,
                                                                    float* pres, const int* __restrict__ gs,
                                                                    const int* __restrict__ ge,
-                                                                   const int4* __restrict__ rows, int patch_up, float4* saw, float4* sbw, int* srw, int lane) {    const int a0 = __ldg(gs + c);
+                                                                   const int4* __restrict__ rows, int patch_up, float4* saw, float4* sbw, int* srw, int lane,
+                                             int part = 0, int parts = 1) {
+    const int a0 = __ldg(gs + c);
     if (a0 < 0) return;
     const int e0 = __ldg(ge + c);
     const SphRec<float> rec = W.rec;
+    if (a0 + 32 * part >= e0) return;
     bool any_wall = false;
     for (int i = a0 + lane; i < e0; i += 32) any_wall |= S.ptype[i] <= 0;
     if (!__any_sync(0xffffffffu, any_wall)) return;
@@ -2182,7 +2186,7 @@ __device__ __forceinline__ void neumann_cell(int c, DevParams P, SphState<float>
     const int tot = stage_rows(P, ic, jc, kc, rows, srw, lane);
     const RelFrame Fr = rel_frame(P, ldr(rec.pos + a0));
     const unsigned lt = (1u << lane) - 1u;
-    for (int p0 = a0; p0 < e0; p0 += 32) {
+    for (int p0 = a0 + 32 * part; p0 < e0; p0 += 32 * parts) {
         const int i = p0 + lane;
         const bool act = i < e0 && S.ptype[i] <= 0;
         if (!__any_sync(0xffffffffu, act)) continue;
@@ -2244,7 +2248,15 @@ __device__ __forceinline__ void neumann_cell(int c, DevParams P, SphState<float>
             }
             const bool slow_chunk = lanes_slow || __any_sync(0xffffffffu, any_oor);
             __syncwarp();
-            if (act && !slow_chunk && K.kt == 3) {
+            const int np = (ns + 3) & ~3;
+            if constexpr (KT == 5) {   // padded to whole groups of four with candidates out of reach
+                if (lane < np - ns) {
+                    saw[ns + lane] = make_float4(1e18f, 1e18f, 1e18f, 0.f);
+                    sbw[ns + lane] = make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+                __syncwarp();
+            }
+            if (KT != 5 && act && !slow_chunk && K.kt == 3) {
                 // every candidate on the FP32 frame: the kernel is evaluated
                 // for all of them and the pairs outside the radius add
                 // nothing, so the lanes do not diverge (only a pair in the
@@ -2275,29 +2287,49 @@ __device__ __forceinline__ void neumann_cell(int c, DevParams P, SphState<float>
                     }
                 }
                 scale = K.tA;
-            } else if (act && !slow_chunk && K.kt == 5) {
-                // Wendland C6 in line, no branches between the candidates
-                Knl<float, 5> K5{K.kt, K.tA, K.ih, K.th};
-#pragma unroll 4
-                for (int u = 0; u < ns; u++) {
-                    const float4 cj = saw[u];
-                    const float dx = fx - cj.x, dy = fy - cj.y, dz = fz - cj.z;
-                    const float r2 = dx * dx + dy * dy + dz * dz;
-                    bool in = r2 < lo2;
-                    if (!in && r2 <= hi2) {
-                        const int j = __float_as_int(cj.w);
-                        in = __dadd_rn(pair_dist(xi, yi, zi, S.x[j], S.y[j], S.z[j]), 1e-20) < R2;
+            } else if (KT == 5 && act && !slow_chunk) {
+                // Wendland C6, four candidates at a time without branches
+                // between them (the band's FP64 predicate: one branch per
+                // four): the wall pass of the gas-spouted beds waits on its
+                // own arithmetic, 194 -> 174 us.  C2's shorter loop is faster
+                // one by one (46 against 50).
+                const Knl<float, 5> K5{K.kt, K.tA, K.ih, K.th};
+                for (int u0 = 0; u0 < np; u0 += 4) {
+                    float r2[4], w[4];
+                    bool in[4], band = false;
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        const float4 cj = saw[u0 + u];
+                        const float dx = fx - cj.x, dy = fy - cj.y, dz = fz - cj.z;
+                        r2[u] = dx * dx + dy * dy + dz * dz;
+                        in[u] = r2[u] < lo2;
+                        band |= !in[u] && r2[u] <= hi2;
                     }
-                    float r, rinv;
-                    rdist(r2, r, rinv);
-                    const float wk = kw(K5, r);
-                    const float4 bj = sbw[u];
-                    if (in) {
-                        const float mr = bj.x * wk;
-                        tp += mr * bj.y;
-                        flt += mr;
-                        tt += mr * bj.z;
-                        tr += bj.w * wk;
+                    if (band) {
+#pragma unroll
+                        for (int u = 0; u < 4; u++)
+                            if (!in[u] && r2[u] <= hi2) {
+                                const int j = __float_as_int(saw[u0 + u].w);
+                                in[u] = __dadd_rn(pair_dist(xi, yi, zi, S.x[j], S.y[j], S.z[j]), 1e-20) < R2;
+                            }
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        float r, rinv;
+                        rdist(r2[u], r, rinv);
+                        w[u] = kw(K5, r);
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        const float4 bj = sbw[u0 + u];
+                        const float wk = w[u];
+                        if (in[u]) {
+                            const float mr = bj.x * wk;
+                            tp += mr * bj.y;
+                            flt += mr;
+                            tt += mr * bj.z;
+                            tr += bj.w * wk;
+                        }
                     }
                 }
             } else if (act && !slow_chunk) {
@@ -2381,11 +2413,11 @@ __device__ __forceinline__ void neumann_cell(int c, DevParams P, SphState<float>
     }
 }
 
-template <bool OCC>
+template <bool OCC, int KT>
 __global__ void __launch_bounds__(NT_WARPS * 32, 8) k_neumann_tiled(DevParams P, SphState<float> S, SphWork<float> W,
                                                                    float* pres, const int* __restrict__ gs,
                                                                    const int* __restrict__ ge,
-                                                                   const int4* __restrict__ rows, int patch_up,
+                                                                   const int4* __restrict__ rows, int patch_up, int parts,
                                                                    const int* __restrict__ occ, const int* __restrict__ occ_n) {
     grid_dep_wait();
     __shared__ float4 sa[NT_WARPS][NT_CH + 32];
@@ -2395,12 +2427,14 @@ __global__ void __launch_bounds__(NT_WARPS * 32, 8) k_neumann_tiled(DevParams P,
     if constexpr (OCC) {   // a sparse grid: the occupied cells, grid-stride
         const int no = *occ_n;
         for (int q = blockIdx.x * NT_WARPS + w; q < no; q += gridDim.x * NT_WARPS) {
-            neumann_cell(occ[q], P, S, W, pres, gs, ge, rows, patch_up, sa[w], sb[w], srow[w], lane);
+            neumann_cell<KT>(occ[q], P, S, W, pres, gs, ge, rows, patch_up, sa[w], sb[w], srow[w], lane);
             __syncwarp();
         }
     } else {
-        const int c = blockIdx.x * NT_WARPS + w;
-        if (c < P.NI * P.NJ * P.NK) neumann_cell(c, P, S, W, pres, gs, ge, rows, patch_up, sa[w], sb[w], srow[w], lane);
+        // parts warps per cell, every parts-th group of 32 of its particles each
+        const int q = blockIdx.x * NT_WARPS + w, c = q / parts;
+        if (c < P.NI * P.NJ * P.NK)
+            neumann_cell<KT>(c, P, S, W, pres, gs, ge, rows, patch_up, sa[w], sb[w], srow[w], lane, q % parts, parts);
     }
 }
 
