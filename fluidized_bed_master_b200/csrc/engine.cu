@@ -29,6 +29,7 @@ using namespace sphdem;
     } while (0)
 
 static const int TPB = 128;
+static const int SMALL_SET = 148 * 4 * 32;   // small_set_lanes
 
 // kernel slots for per-kernel timing
 enum {
@@ -533,6 +534,11 @@ static int enqueue_krylov(SphdemHandle* H, EngineHost<R>* EH, SphState<R>& S, Sp
 // configuration, so a given bed always runs one form.
 inline bool dem_thread_per_sphere(const DevParams& P) { return P.dim == 2 && P.nd >= 65536; }
 
+// Lanes per particle of the general passes and the reaction force: a set whose
+// particles fill at most one warp per scheduler (148 x 4) runs 8 lanes each,
+// which keep the bits of one thread's walk.
+inline bool small_set_lanes(const DevParams& P) { return P.ns <= SMALL_SET && P.kernel_type != 3; }
+
 // warps of a grid-stride pass over the occupied cells of a sparse grid: at
 // most one per SPH particle, at most 128 per SM
 inline int occ_warps(const DevParams& P) { return std::max(1, std::min(P.ns, 148 * 128)); }
@@ -749,7 +755,8 @@ int enqueue_step(SphdemHandle* H, EngineHost<R>* EH, int flags, int64_t* nl) {
     if ((r = nnps_dem<R>(H, EH, dox, dn, nl, sd))) return r;
     SphState<R>& S = E.S[sn];
     DemState<double>& D = E.D[dn];
-    int bs = nblocks(ns, TPB), bd = nblocks(nd, TPB);
+    const bool sl = small_set_lanes(P);
+    int bs = nblocks(ns, TPB), bl = sl ? nblocks(ns * 8, TPB) : bs, bd = nblocks(nd, TPB);
     int bdw = nblocks(nd * 32, TPB), bbw = nblocks(P.nbuf * 32, TPB);
     if (!keep) {
         if ((r = nnps_sph<R>(H, EH, so, sn, nl))) return r;
@@ -790,7 +797,7 @@ int enqueue_step(SphdemHandle* H, EngineHost<R>* EH, int flags, int64_t* nl) {
             *nl += 1;
         }
         CK(wait(1, st));
-        { KTIME(KT_PASSA); CK((launch_pdl(kt3 ? k_passA<R> : kt5 ? k_passA_any<R, 5> : k_passA_any<R, -1>, bs, TPB, 0, st, P, S, W, D, DW, DW.rows))); }
+        { KTIME(KT_PASSA); CK((launch_pdl(kt3 ? k_passA<R> : sl ? (kt5 ? k_passA_any<R, 5, 8> : k_passA_any<R, -1, 8>) : kt5 ? k_passA_any<R, 5, 1> : k_passA_any<R, -1, 1>, bl, TPB, 0, st, P, S, W, D, DW, DW.rows))); }
         *nl += 1;
         {
             KTIME(KT_PASSB);
@@ -798,10 +805,12 @@ int enqueue_step(SphdemHandle* H, EngineHost<R>* EH, int flags, int64_t* nl) {
                 CK((launch_pdl(kt3 ? k_sps<R, 3> : k_sps<R, -1>, bs, TPB, 0, st, P, S, W)));
                 *nl += 1;
             }
-            auto kb = kt5 ? k_passB_any<R, false, 5> : !kt3 ? k_passB_any<R, false, -1> : P.con ? k_passB<R, true> : k_passB<R, false>;
-            if (P.iface | P.fb | P.sps | P.ipf) kb = k_passB_any<R, true, -1>;
-            else if (P.fva) kb = k_passB_any<R, false, -1>;
-            CK((launch_pdl(kb, bs, TPB, 0, st, P, S, W, E.flags)));
+            auto kb = !kt3 && sl ? (kt5 ? k_passB_any<R, false, 5, 8> : k_passB_any<R, false, -1, 8>)
+                      : kt5 ? k_passB_any<R, false, 5, 1> : !kt3 ? k_passB_any<R, false, -1, 1> : P.con ? k_passB<R, true> : k_passB<R, false>;
+            int bb = bl;
+            if (P.iface | P.fb | P.sps | P.ipf) kb = k_passB_any<R, true, -1, 1>, bb = bs;
+            else if (P.fva) kb = k_passB_any<R, false, -1, 1>, bb = bs;
+            CK((launch_pdl(kb, bb, TPB, 0, st, P, S, W, E.flags)));
         }
         *nl += 1;
     }
@@ -821,7 +830,7 @@ int enqueue_step(SphdemHandle* H, EngineHost<R>* EH, int flags, int64_t* nl) {
     }
     if (ns > 0) {
         KTIME(KT_SPHCOUPLING);
-        CK((launch_pdl(kt3 ? k_sph_coupling<R, 3> : kt5 ? k_sph_coupling<R, 5> : k_sph_coupling<R, -1>, bs, TPB, 0, st, P, S, W, D, DW, DW.rows, (flags & F_TIME0) ? 1 : 0)));
+        CK((launch_pdl(kt3 ? k_sph_coupling<R, 3, 1> : sl ? (kt5 ? k_sph_coupling<R, 5, 8> : k_sph_coupling<R, -1, 8>) : kt5 ? k_sph_coupling<R, 5, 1> : k_sph_coupling<R, -1, 1>, bl, TPB, 0, st, P, S, W, D, DW, DW.rows, (flags & F_TIME0) ? 1 : 0)));
         *nl += 1;
     }
     CK(rec(4, st));   // the SPH coupling has read the DEM set
@@ -838,14 +847,14 @@ int enqueue_step(SphdemHandle* H, EngineHost<R>* EH, int flags, int64_t* nl) {
         }
         {
             KTIME(KT_PPE);
-            if (H->p.ppe_mode == SPHDEM_PPE_REFERENCE) CK((launch_pdl(kt3 ? k_ppe<R> : kt5 ? k_ppe_any<R, 5> : k_ppe_any<R, -1>, bs, TPB, 0, st, P, S, W)));
+            if (H->p.ppe_mode == SPHDEM_PPE_REFERENCE) CK((launch_pdl(kt3 ? k_ppe<R> : sl ? (kt5 ? k_ppe_any<R, 5, 8> : k_ppe_any<R, -1, 8>) : kt5 ? k_ppe_any<R, 5, 1> : k_ppe_any<R, -1, 1>, bl, TPB, 0, st, P, S, W)));
             else if ((r = enqueue_krylov<R>(H, EH, S, W))) return r;
         }
         {
             KTIME(KT_NEUMANN);
             CK(launch_neumann<R>(E, S, W.p_new, 0, st));
         }
-        { KTIME(KT_PASSC); CK((launch_pdl(kt3 ? k_passC<R> : kt5 ? k_passC_any<R, 5> : k_passC_any<R, -1>, bs, TPB, 0, st, P, S, W))); }
+        { KTIME(KT_PASSC); CK((launch_pdl(kt3 ? k_passC<R> : sl ? (kt5 ? k_passC_any<R, 5, 8> : k_passC_any<R, -1, 8>) : kt5 ? k_passC_any<R, 5, 1> : k_passC_any<R, -1, 1>, bl, TPB, 0, st, P, S, W))); }
         *nl += 3;
         if (P.open_bc > 0) {
             KTIME(KT_OPENBC);
@@ -854,7 +863,7 @@ int enqueue_step(SphdemHandle* H, EngineHost<R>* EH, int flags, int64_t* nl) {
         }
         if (P.xsph) {
             KTIME(KT_XSPH);
-            CK((launch_pdl(kt3 ? k_xsph<R> : kt5 ? k_xsph_any<R, 5> : k_xsph_any<R, -1>, bs, TPB, 0, st, P, S, W)));
+            CK((launch_pdl(kt3 ? k_xsph<R> : sl ? (kt5 ? k_xsph_any<R, 5, 8> : k_xsph_any<R, -1, 8>) : kt5 ? k_xsph_any<R, 5, 1> : k_xsph_any<R, -1, 1>, bl, TPB, 0, st, P, S, W)));
             *nl += 1;
         }
     }

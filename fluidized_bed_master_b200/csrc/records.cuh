@@ -629,4 +629,53 @@ __device__ __forceinline__ void nb_walk(int cnt, const int* __restrict__ nb, int
     }
 }
 
+// ---- several lanes per particle, sums in list order -------------------------
+// A set of a few thousand particles leaves a scheduler less than a warp, and a
+// pass then lasts one thread's walk.  L lanes share a particle: each forms the
+// terms of one entry (the operands of the sums' FMAs), then all add them in
+// list order, so every lane holds the bits that one thread's walk gives.
+template <int L>
+struct LaneGroup {
+    int i, lane;
+    unsigned mask, base;
+    __device__ __forceinline__ LaneGroup() {
+        const int t = blockIdx.x * blockDim.x + threadIdx.x;
+        i = t / L;
+        lane = t % L;
+        base = (threadIdx.x & 31) & ~(L - 1);
+        mask = (L == 32 ? 0xffffffffu : (1u << L) - 1u) << base;
+    }
+};
+template <int L, typename T>
+__device__ __forceinline__ T shfl_terms(unsigned mask, const T& t, int l) {
+    static_assert(sizeof(T) % 4 == 0, "terms are 32- or 64-bit values");
+    constexpr int N = sizeof(T) / 4;
+    T o;
+    const int* a = reinterpret_cast<const int*>(&t);
+    int* b = reinterpret_cast<int*>(&o);
+#pragma unroll
+    for (int q = 0; q < N; q++) b[q] = __shfl_sync(mask, a[q], l, L);
+    return o;
+}
+// entry(k): list entry k; load(j): its record; terms(j, r, t): false when the
+// pair adds nothing; add(t)
+template <int L, typename Rec, typename T, typename E, typename LD, typename TM, typename AD>
+__device__ __forceinline__ void ordered_walk(const LaneGroup<L>& g, int cnt, E entry, LD load, TM terms, AD add) {
+    int j = g.lane < cnt ? entry(g.lane) : 0;
+    for (int k0 = 0; k0 < cnt; k0 += L) {
+        const int k = k0 + g.lane, jc = j;
+        T t{};
+        bool ok = false;
+        if (k < cnt) {
+            const Rec r = load(jc);
+            if (k + L < cnt) j = entry(k + L);
+            ok = terms(jc, r, t);
+        }
+        const unsigned m = (__ballot_sync(g.mask, ok) & g.mask) >> g.base;
+#pragma unroll
+        for (int l = 0; l < L; l++)
+            if ((m >> l) & 1u) add(shfl_terms<L, T>(g.mask, t, l));
+    }
+}
+
 }  // namespace sphdem

@@ -777,36 +777,50 @@ struct DemAB {
 };
 // KERNEL_clc_prep3D_coupling_sph (functions_PREP2.cuh:3190-3364): the sums of
 // particle i over its spheres
-template <typename R, typename K>
+template <typename R, int L, typename K>
 __device__ __forceinline__ void sph_dem_porosity(const DevParams& P, const SphWork<R>& W, const DemState<double>& D,
-                                                 const DemWork<double>& DW, const int4* __restrict__ drows, int i,
-                                                 double xi, double yi, double zi, double hi, const K& Kn, R& por,
-                                                 R& dfx, R& dfy, R& dfz) {
+                                                 const DemWork<double>& DW, const int4* __restrict__ drows,
+                                                 const LaneGroup<L>& g, double xi, double yi, double zi, double hi,
+                                                 const K& Kn, R& por, R& dfx, R& dfy, R& dfz) {
     const double Rr = P.kappa * hi;
     const float r2l = r2_lo(Rr), r2h = r2_hi(Rr);
-    const int n = P.ns;
+    const int n = P.ns, i = g.i;
+    struct T {
+        R w, v, ax, ay, az;
+    };
     auto load = [&](int j) { return DemAB{ldr(DW.ra + j), ldr(DW.rb + j)}; };
-    auto dem = [&](int, const DemAB& q) {
+    auto terms = [&](int, const DemAB& q, T& t) {
         PairT<R> g = pair_test<R>(xi, yi, zi, q.a.x, q.a.y, q.a.z, Rr, 1e-20, r2l, r2h);
-        if (!g.in) return;
+        if (!g.in) return false;
         R r = g.r + (R)1e-20, ir = rcp(r);
-        R w = kw(Kn, r);
+        t.w = kw(Kn, r);
         R dw = kdw(Kn, r);
         R rj = (R)q.a.w;
-        R v = dem_measure(P, rj);
-        por += w * v;
-        dfx += dw * g.dx * ir * (R)q.b.x * v;
-        dfy += dw * g.dy * ir * (R)q.b.y * v;
-        dfz += dw * g.dz * ir * (R)q.b.z * v;
+        t.v = dem_measure(P, rj);
+        t.ax = dw * g.dx * ir * (R)q.b.x;
+        t.ay = dw * g.dy * ir * (R)q.b.y;
+        t.az = dw * g.dz * ir * (R)q.b.z;
+        return true;
+    };
+    auto add = [&](const T& t) {
+        por += t.w * t.v;
+        dfx += t.ax * t.v;
+        dfy += t.ay * t.v;
+        dfz += t.az * t.v;
+    };
+    auto one = [&](int j, const DemAB& q) {
+        T t;
+        if (terms(j, q, t)) add(t);
     };
     const int cd = W.ncntd[i];
     if (cd <= P.nbd_cap) {
-        dem_walk<DemAB>(W.nbrd, cd, n, i, load, dem);
+        if constexpr (L == 1) dem_walk<DemAB>(W.nbrd, cd, n, i, load, one);
+        else ordered_walk<L, DemAB, T>(g, cd, [&](int k) { return W.nbrd[(size_t)k * n + i]; }, load, terms, add);
     } else {
         int ic, jc, kc;
         cell_ijk(P, xi, yi, zi, ic, jc, kc);
         for_stencil_j(P, ic, jc, kc, drows, make_cull(xi, yi, zi, Rr), [&](int j) {
-            if (D.ptype[j] > 1000) dem(j, load(j));
+            if (D.ptype[j] > 1000) one(j, load(j));
         });
     }
 }
@@ -915,7 +929,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 7 : 1) k_passA(DevParams
     R por = 0, dfx = 0, dfy = 0, dfz = 0;
     if (P.nd > 0) {
         const Knl<R, 3> Kd = knl_make<R, 3>(P, th);
-        sph_dem_porosity(P, W, D, DW, drows, i, xi, yi, zi, hi, Kd, por, dfx, dfy, dfz);
+        sph_dem_porosity<R, 1>(P, W, D, DW, drows, LaneGroup<1>(), xi, yi, zi, hi, Kd, por, dfx, dfy, dfz);
     }
     R isf = rcp(sflt + (R)1e-20);
     R pori = (R)1 - por * isf;
@@ -1986,11 +2000,13 @@ __global__ void __launch_bounds__(128) k_dem_finish(DevParams P, DemState<double
 // KERNEL_SPH_coupling3D_sph (functions_SPH_DEM_COUPLING2.cuh:1815-2019) +
 // KERNEL_clc_projection_sph (functions_TIME_ISPH2.cuh:104-204).
 // ---------------------------------------------------------------------------
-template <typename R, int KT>
-__global__ void __launch_bounds__(128) k_sph_coupling(DevParams P, SphState<R> S, SphWork<R> W, DemState<double> D,
+// L lanes per particle (small sets, small_set_lanes in engine.cu)
+template <typename R, int KT, int L>
+__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 6 : 1) k_sph_coupling(DevParams P, SphState<R> S, SphWork<R> W, DemState<double> D,
                                                       DemWork<double> DW, const int4* __restrict__ drows, int time_zero) {
     grid_dep_wait();
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const LaneGroup<L> grp;
+    const int i = grp.i;
     int n = P.ns;
     if (i >= n) return;
     int it = S.itype[i], pt = S.ptype[i];
@@ -2014,31 +2030,47 @@ __global__ void __launch_bounds__(128) k_sph_coupling(DevParams P, SphState<R> S
                 double m;
             };
             auto load = [&](int j) { return Rec{ldr(DW.ra + j), ldr(DW.rc + j), ldr(DW.rd + j), ldr(&DW.rb[j].w)}; };
-            auto dem = [&](int, const Rec& q) {
+            struct T {
+                R c, ax, ay, az, at;
+            };
+            auto terms = [&](int, const Rec& q, T& t) {
                 PairT<R> g = pair_test<R>(xi, yi, zi, q.a.x, q.a.y, q.a.z, Rr, 0.0, r2l, r2h);
-                if (!g.in) return;
+                if (!g.in) return false;
                 R ffj = (R)q.f.x + (R)q.f.y;
-                if (!(ffj > (R)0)) return;
+                if (!(ffj > (R)0)) return false;
                 R w = kw(K, g.r);
                 if (P.dim == 2) w *= (R)0.75 / (R)q.a.w;   // per unit depth (depth 4 r / 3)
-                R c = w / (ffj + (R)1.0e-20);
+                t.c = w / (ffj + (R)1.0e-20);
                 R mr = (R)q.m / rhoi;
-                tx += -mr * (R)q.c.x * c;
-                ty += -mr * (R)q.c.y * c;
-                tz += -mr * (R)q.c.z * c;
-                tt += -(R)q.c.w / (rhoi * cpi) * c;
+                t.ax = -mr * (R)q.c.x;
+                t.ay = -mr * (R)q.c.y;
+                t.az = -mr * (R)q.c.z;
+                t.at = -(R)q.c.w / (rhoi * cpi);
+                return true;
+            };
+            auto add = [&](const T& t) {
+                tx += t.ax * t.c;
+                ty += t.ay * t.c;
+                tz += t.az * t.c;
+                tt += t.at * t.c;
+            };
+            auto one = [&](int j, const Rec& q) {
+                T t;
+                if (terms(j, q, t)) add(t);
             };
             const int cd = W.ncntd[i];
             if (cd <= P.nbd_cap) {
-                dem_walk<Rec>(W.nbrd, cd, n, i, load, dem);
+                if constexpr (L == 1) dem_walk<Rec>(W.nbrd, cd, n, i, load, one);
+                else ordered_walk<L, Rec, T>(grp, cd, [&](int k) { return W.nbrd[(size_t)k * n + i]; }, load, terms, add);
             } else {
                 int ic, jc, kc;
                 cell_ijk(P, xi, yi, zi, ic, jc, kc);
                 for_stencil_j(P, ic, jc, kc, drows, make_cull(xi, yi, zi, Rr), [&](int j) {
-                    if (D.ptype[j] > 1000) dem(j, load(j));
+                    if (D.ptype[j] > 1000) one(j, load(j));
                 });
             }
         }
+        if (grp.lane) return;
         ftx += tx;
         fty += ty;
         ftz += tz;
@@ -2048,6 +2080,7 @@ __global__ void __launch_bounds__(128) k_sph_coupling(DevParams P, SphState<R> S
         W.ftot[i] = sqrt(ftx * ftx + fty * fty + ftz * ftz);
         if (P.con) W.dtemp[i] += tt;
     }
+    if (grp.lane) return;
     // predictor (SPH), KERNEL_clc_projection_sph; eps u* also goes to the
     // {eps u*, p} record the PPE reads
     R uxi = S.ux[i], uyi = S.uy[i], uzi = S.uz[i];
@@ -3056,11 +3089,12 @@ __device__ __forceinline__ void cm_store(R* Cm, int n, int i, const R* C) {
     Cm[(size_t)4 * n + i] = C[5];
     Cm[(size_t)5 * n + i] = C[8];
 }
-template <typename R, int KT>
+template <typename R, int KT, int L>
 __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 8 : 1) k_passA_any(DevParams P, SphState<R> S, SphWork<R> W, DemState<double> D,
                                                DemWork<double> DW, const int4* __restrict__ drows) {
     grid_dep_wait();
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const LaneGroup<L> grp;
+    const int i = grp.i;
     int n = P.ns;
     if (i >= n) return;
     const SphRec<R> rec = W.rec;
@@ -3073,7 +3107,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 8 : 1) k_passA_any(DevPa
         return;
     }
     R dprev = S.dDEMpor[i];
-    W.dDEMpor_prev[i] = dprev;
+    if (grp.lane == 0) W.dDEMpor_prev[i] = dprev;
     double xi = S.x[i], yi = S.y[i], zi = S.z[i], hi = S.h[i];
     R th = (R)hi;
     Knl<R, KT> K = knl_make<R, KT>(P, th);
@@ -3082,33 +3116,60 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 8 : 1) k_passA_any(DevPa
     R txx = 0, tyy = 0, tzz = 0, txy = 0, tyz = 0, tzx = 0, sflt = 0;
     const int* __restrict__ nb = W.nbr;
     const bool kgc = (P.kgc == 1);
-    nb_walk<4, NbQ2<R>>(
-        cnt, nb, n, i,
-        [&](int j) {
-            NbQ2<R> t;
-            t.q = ldr(rec.pos + j);
-            t.a = ldr(rec.mr0 + j);
-            return t;
-        },
-        [&](int j, const NbQ2<R>& t) {
-            int ptj = tag_ptype(t.q.w);
-            if (ptj > 1000) return;
-            Disp<R> g = disp(P, qi, t.q, S.x, S.y, S.z, i, j);
-            R r2 = g.dx * g.dx + g.dy * g.dy + g.dz * g.dz, r, rinv;
-            rdist(r2, r, rinv);
-            R irj = rcp(t.a.y);
-            if (ptj == 1) sflt += t.a.x * irj * kw(K, r);
-            if (kgc && r2 > (R)0) {
-                R dw = kdw(K, r);
-                R c = -t.a.x * dw * irj * rinv;
-                txx += c * g.dx * g.dx;
-                txy += c * g.dy * g.dx;
-                tyy += c * g.dy * g.dy;
-                tzx += c * g.dx * g.dz;
-                tyz += c * g.dy * g.dz;
-                tzz += c * g.dz * g.dz;
-            }
+    struct T {
+        R p, w, cx, cy, cz, dx, dy, dz;
+        int f;
+    };
+    auto load = [&](int j) {
+                NbQ2<R> t;
+                t.q = ldr(rec.pos + j);
+                t.a = ldr(rec.mr0 + j);
+                return t;
+            };
+    auto terms = [&](int j, const NbQ2<R>& t, T& o) {
+        int ptj = tag_ptype(t.q.w);
+        if (ptj > 1000) return false;
+        Disp<R> g = disp(P, qi, t.q, S.x, S.y, S.z, i, j);
+        R r2 = g.dx * g.dx + g.dy * g.dy + g.dz * g.dz, r, rinv;
+        rdist(r2, r, rinv);
+        R irj = rcp(t.a.y);
+        o.f = 0;
+        if (ptj == 1) {
+            o.f |= 1;
+            o.p = t.a.x * irj;
+            o.w = kw(K, r);
+        }
+        if (kgc && r2 > (R)0) {
+            R dw = kdw(K, r);
+            R c = -t.a.x * dw * irj * rinv;
+            o.f |= 2;
+            o.cx = c * g.dx;
+            o.cy = c * g.dy;
+            o.cz = c * g.dz;
+            o.dx = g.dx;
+            o.dy = g.dy;
+            o.dz = g.dz;
+        }
+        return true;
+    };
+    auto add = [&](const T& o) {
+        if (o.f & 1) sflt += o.p * o.w;
+        if (o.f & 2) {
+            txx += o.cx * o.dx;
+            txy += o.cy * o.dx;
+            tyy += o.cy * o.dy;
+            tzx += o.cx * o.dz;
+            tyz += o.cy * o.dz;
+            tzz += o.cz * o.dz;
+        }
+    };
+    if constexpr (L == 1)
+        nb_walk<4, NbQ2<R>>(cnt, nb, n, i, load, [&](int j, const NbQ2<R>& t) {
+            T o;
+            if (terms(j, t, o)) add(o);
         });
+    else
+        ordered_walk<L, NbQ2<R>, T>(grp, cnt, [&](int k) { return __ldg(nb + nb_at(k, n, i)); }, load, terms, add);
     if (kgc && P.dim == 2) {
         // a bed in a plane y = const: the x-z block of the moment matrix
         const R det = txx * tzz - tzx * tzx;
@@ -3144,8 +3205,9 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 8 : 1) k_passA_any(DevPa
     }
     R por = 0, dfx = 0, dfy = 0, dfz = 0;
     if (P.nd > 0) {
-        sph_dem_porosity(P, W, D, DW, drows, i, xi, yi, zi, hi, K, por, dfx, dfy, dfz);
+        sph_dem_porosity<R, L>(P, W, D, DW, drows, grp, xi, yi, zi, hi, K, por, dfx, dfy, dfz);
     }
+    if (grp.lane) return;
     R isf = rcp(sflt + (R)1e-20);
     R pori = (R)1 - por * isf;
     W.DEMpor[i] = pori;
@@ -3170,19 +3232,22 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 8 : 1) k_passA_any(DevPa
     rec.f1[i] = mk4<R>(mn, rn, S.temp[i], pori);
 }
 
-template <typename R, bool FORCES, int KT>
+template <typename R, bool FORCES, int KT, int L>
 __global__ void __launch_bounds__(128) k_passB_any(DevParams P, SphState<R> S, SphWork<R> W, const DevFlags* F) {
     grid_dep_wait();
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const LaneGroup<L> grp;
+    const int i = grp.i;
     int n = P.ns;
     if (i >= n) return;
     const SphRec<R> rec = W.rec;
     // Shepard filter every freq_filt*decouple_stride steps (functions_PREP2.cuh:2120)
     const int filt = (F->step_count % P.filt_period) == 0;
     int it = S.itype[i], pt = S.ptype[i], bt = S.btype[i];
-    W.ftx[i] = 0; W.fty[i] = 0; W.ftz[i] = 0; W.ftot[i] = 0;
-    W.pgfx[i] = 0; W.pgfy[i] = 0; W.pgfz[i] = 0;
-    W.dtemp[i] = 0;
+    if (grp.lane == 0) {
+        W.ftx[i] = 0; W.fty[i] = 0; W.ftz[i] = 0; W.ftot[i] = 0;
+        W.pgfx[i] = 0; W.pgfy[i] = 0; W.pgfz[i] = 0;
+        W.dtemp[i] = 0;
+    }
     if (it > 2 || pt > 1000) return;
     bool adv = !(P.open_bc > 0 && bt > 0) && pt < 1000 && pt > 0;
     if (!filt && !adv) return;
@@ -3208,6 +3273,93 @@ __global__ void __launch_bounds__(128) k_passB_any(DevParams P, SphState<R> S, S
     int cnt = min(W.ncnt[i], P.nb_cap);
     R flt = 0, tx = 0, ty = 0, tz = 0, px = 0, py = 0, pz = 0, Rc = 0, ex = 0, ey = 0, ez = 0, et = 0;
     const int* __restrict__ nb = W.nbr;
+    if constexpr (L > 1) {
+        static_assert(!FORCES, "several lanes: the default forces");
+        struct T {
+            R p, w, s, gx, gy, gz, cv, dux, duy, duz, pij, ex, ey, ez, mr, et, rc, rr;
+            int f;   // 1 filter, 2 forces, 4 artificial viscosity
+        };
+        auto load = [&](int j) {
+            NbQ44<R> t;
+            t.q = ldr(rec.pos + j);
+            t.a = ldr(rec.f1 + j);
+            t.b = ldr(rec.up + j);
+            return t;
+        };
+        auto terms = [&](int j, const NbQ44<R>& t, T& o) {
+            const V4<R>& fj = t.a;
+            const V4<R>& uj = t.b;
+            Disp<R> g = disp(P, qi, t.q, S.x, S.y, S.z, i, j);
+            R r2 = g.dx * g.dx + g.dy * g.dy + g.dz * g.dz, r, rinv;
+            rdist(r2, r, rinv);
+            R mj = fj.x, irj = rcp(fj.y);
+            o.f = 0;
+            if (filt) {
+                o.f |= 1;
+                o.p = mj * irj;
+                o.w = kw(K, r);
+            }
+            if (!adv || tag_ptype(t.q.w) >= 1000) return o.f != 0;
+            o.f |= 2;
+            R dw = kdw(K, r);
+            R gx = dw * g.dx * rinv, gy = dw * g.dy * rinv, gz = dw * g.dz * rinv;
+            cm_apply(Cm, kgc, gx, gy, gz);
+            R tj = fj.z;
+            o.gx = gx;
+            o.gy = gy;
+            o.gz = gz;
+            o.s = cp_i * mj * (pi + uj.w) * irj;
+            o.cv = (g.dx * gx + g.dy * gy + g.dz * gz) * cv_i * mj * irj * rinv * rinv;
+            o.dux = uxi - uj.x;
+            o.duy = uyi - uj.y;
+            o.duz = uzi - uj.z;
+            if (P.fva != 0) {
+                R uij = (uxi - uj.x) * g.dx + (uyi - uj.y) * g.dy + (uzi - uj.z) * g.dz;
+                if (uij < (R)0) {
+                    R hij = (th + th) * (R)0.5;
+                    R phi = hij * uij / (r * r + (R)0.01 * hij * hij);
+                    o.pij = mi * phi * ((R)-0.1 * (R)P.soundspeed + (R)0.02 * phi) / (rhoi + fj.y) * (R)0.5;
+                    o.f |= 4;
+                }
+            }
+            o.mr = mj * irj * ((R)1 - eli);
+            R ug = uxi * gx + uyi * gy + uzi * gz;
+            o.ex = (uj.x - uxi) * ug;
+            o.ey = (uj.y - uyi) * ug;
+            o.ez = (uj.z - uzi) * ug;
+            o.et = (tj - tempi) * ug;
+            o.rc = ch_i * mj * (tempi - tj) * dw * irj;
+            o.rr = rcp(r + (R)1e-10);
+            return true;
+        };
+        auto add = [&](const T& o) {
+            if (o.f & 1) flt += o.p * o.w;
+            if (!(o.f & 2)) return;
+            if (P.fp != 0) {
+                px += o.s * o.gx;
+                py += o.s * o.gy;
+                pz += o.s * o.gz;
+            }
+            if (P.fv != 0) {
+                tx += o.cv * o.dux;
+                ty += o.cv * o.duy;
+                tz += o.cv * o.duz;
+            }
+            if (o.f & 4) {
+                tx += -o.pij * o.gx;
+                ty += -o.pij * o.gy;
+                tz += -o.pij * o.gz;
+            }
+            if (eli < (R)1) {
+                ex += o.ex * o.mr;
+                ey += o.ey * o.mr;
+                ez += o.ez * o.mr;
+                if (P.con != 0) et += o.et * o.mr;
+            }
+            if (P.con != 0) Rc += o.rc * o.rr;
+        };
+        ordered_walk<L, NbQ44<R>, T>(grp, cnt, [&](int k) { return __ldg(nb + nb_at(k, n, i)); }, load, terms, add);
+    } else {
     nb_walk<4, NbQ44<R>>(
         cnt, nb, n, i,
         [&](int j) {
@@ -3305,6 +3457,8 @@ __global__ void __launch_bounds__(128) k_passB_any(DevParams P, SphState<R> S, S
             }
             if ((P.con != 0)) Rc += ch_i * mj * (tempi - tj) * dw * irj * rcp(r + (R)1e-10);
         });
+    }
+    if (grp.lane) return;
     if (filt) S.flt_s[i] = flt;
     if (!adv) return;
     if (P.fg) tz += -(R)P.g_sph;
@@ -3318,10 +3472,11 @@ __global__ void __launch_bounds__(128) k_passB_any(DevParams P, SphState<R> S, S
     if ((P.con != 0)) W.dtemp[i] = Rc / (R)P.cp_sph * (R)(pt != -1) - et;
 }
 
-template <typename R, int KT>
+template <typename R, int KT, int L>
 __global__ void __launch_bounds__(128) k_ppe_any(DevParams P, SphState<R> S, SphWork<R> W) {
     grid_dep_wait();
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const LaneGroup<L> grp;
+    const int i = grp.i;
     int n = P.ns;
     if (i >= n) return;
     const SphRec<R> rec = W.rec;
@@ -3344,49 +3499,70 @@ __global__ void __launch_bounds__(128) k_ppe_any(DevParams P, SphState<R> S, Sph
     int cnt = min(W.ncnt[i], P.nb_cap);
     R bx = 0, by = 0, bz = 0, A = 0, AP = 0;
     const int* __restrict__ nb = W.nbr;
-    nb_walk<4, NbQ44<R>>(
-        cnt, nb, n, i,
-        [&](int j) {
-            NbQ44<R> t;
-            t.q = ldr(rec.pos + j);
-            t.a = ldr(rec.f1 + j);
-            t.b = ldr(rec.up + j);
-            return t;
-        },
-        [&](int j, const NbQ44<R>& t) {
-            int tj = t.q.w;
-            if (tag_ptype(tj) >= 1000 || tag_itype(tj) == 4) return;
-            const V4<R>& fj = t.a;
-            const V4<R>& uj = t.b;
-            Disp<R> g = disp(P, qi, t.q, S.x, S.y, S.z, i, j);
-            R r2 = g.dx * g.dx + g.dy * g.dy + g.dz * g.dz, r, rinv;
-            rdist(r2, r, rinv);
-            R mj = fj.x, rhoj = fj.y, porj = fj.w, irj = rcp(rhoj);
-            R dw = kdw(K, r);
-            R gx = dw * g.dx * rinv, gy = dw * g.dy * rinv, gz = dw * g.dz * rinv;
-            cm_apply(Cm, kgc, gx, gy, gz);
-            R mr = mj * irj;
-            bx += mr * (pux - porj * uj.x) * gx;
-            by += mr * (puy - porj * uj.y) * gy;
-            bz += mr * (puz - porj * uj.z) * gz;
-            R c = -(g.dx * gx + g.dy * gy + g.dz * gz) * rinv * rinv;
-            R a = mj * ((prhoi + porj * rhoj) * irj * irhoi) * c;
-            A += a;
-            AP += a * uj.w;
+    struct T {
+        R vx, vy, vz, gx, gy, gz, a, c, p;
+    };
+    auto load = [&](int j) {
+                NbQ44<R> t;
+                t.q = ldr(rec.pos + j);
+                t.a = ldr(rec.f1 + j);
+                t.b = ldr(rec.up + j);
+                return t;
+            };
+    auto terms = [&](int j, const NbQ44<R>& t, T& o) {
+        int tj = t.q.w;
+        if (tag_ptype(tj) >= 1000 || tag_itype(tj) == 4) return false;
+        const V4<R>& fj = t.a;
+        const V4<R>& uj = t.b;
+        Disp<R> g = disp(P, qi, t.q, S.x, S.y, S.z, i, j);
+        R r2 = g.dx * g.dx + g.dy * g.dy + g.dz * g.dz, r, rinv;
+        rdist(r2, r, rinv);
+        R mj = fj.x, rhoj = fj.y, porj = fj.w, irj = rcp(rhoj);
+        R dw = kdw(K, r);
+        R gx = dw * g.dx * rinv, gy = dw * g.dy * rinv, gz = dw * g.dz * rinv;
+        cm_apply(Cm, kgc, gx, gy, gz);
+        R mr = mj * irj;
+        o.vx = mr * (pux - porj * uj.x);
+        o.vy = mr * (puy - porj * uj.y);
+        o.vz = mr * (puz - porj * uj.z);
+        o.gx = gx;
+        o.gy = gy;
+        o.gz = gz;
+        o.c = -(g.dx * gx + g.dy * gy + g.dz * gz) * rinv * rinv;
+        o.a = mj * ((prhoi + porj * rhoj) * irj * irhoi);
+        o.p = uj.w;
+        return true;
+    };
+    auto add = [&](const T& o) {
+        bx += o.vx * o.gx;
+        by += o.vy * o.gy;
+        bz += o.vz * o.gz;
+        const R a = o.a * o.c;
+        A += a;
+        AP += a * o.p;
+    };
+    if constexpr (L == 1)
+        nb_walk<4, NbQ44<R>>(cnt, nb, n, i, load, [&](int j, const NbQ44<R>& t) {
+            T o;
+            if (terms(j, t, o)) add(o);
         });
+    else
+        ordered_walk<L, NbQ44<R>, T>(grp, cnt, [&](int k) { return __ldg(nb + nb_at(k, n, i)); }, load, terms, add);
+    if (grp.lane) return;
     R b = (R)P.rho_gas * (bx + by + bz + (R)2 * S.dDEMpor[i] - W.dDEMpor_prev[i]) / (R)P.sdt;
     W.p_new[i] = (b + AP) / A;
 }
 
-template <typename R, int KT>
+template <typename R, int KT, int L>
 __global__ void __launch_bounds__(128) k_passC_any(DevParams P, SphState<R> S, SphWork<R> W) {
     grid_dep_wait();
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const LaneGroup<L> grp;
+    const int i = grp.i;
     int n = P.ns;
     if (i >= n) return;
     const SphRec<R> rec = W.rec;
     int it = S.itype[i], pt = S.ptype[i], bt = S.btype[i];
-    W.fpx[i] = 0; W.fpy[i] = 0; W.fpz[i] = 0;
+    if (grp.lane == 0) W.fpx[i] = 0, W.fpy[i] = 0, W.fpz[i] = 0;
     if (it > 2) {
         rec.ut[i] = mk4<R>(S.ux[i], S.uy[i], S.uz[i], S.temp[i]);
         return;
@@ -3404,30 +3580,44 @@ __global__ void __launch_bounds__(128) k_passC_any(DevParams P, SphState<R> S, S
         int cnt = min(W.ncnt[i], P.nb_cap);
         const int* __restrict__ nb = W.nbr;
         const R* __restrict__ pn = W.p_new;
-        nb_walk<4, NbQ2S<R>>(
-            cnt, nb, n, i,
-            [&](int j) {
-                NbQ2S<R> t;
-                t.q = ldr(rec.pos + j);
-                t.a = ldr(reinterpret_cast<const V2<R>*>(rec.f1 + j));
-                t.s = __ldg(pn + j);
-                return t;
-            },
-            [&](int j, const NbQ2S<R>& t) {
-                if (tag_ptype(t.q.w) >= 1000) return;
-                Disp<R> g = disp(P, qi, t.q, S.x, S.y, S.z, i, j);
-                R r2 = g.dx * g.dx + g.dy * g.dy + g.dz * g.dz, r, rinv;
-                rdist(r2, r, rinv);
-                R dw = kdw(K, r);
-                R gx = dw * g.dx * rinv, gy = dw * g.dy * rinv, gz = dw * g.dz * rinv;
-                cm_apply(Cm, kgc, gx, gy, gz);
-                R Cp = cpi * t.a.x * (pi + t.s) * rcp(t.a.y);
-                fx += Cp * gx;
-                fy += Cp * gy;
-                fz += Cp * gz;
+        struct T {
+            R c, gx, gy, gz;
+        };
+        auto load = [&](int j) {
+                        NbQ2S<R> t;
+                        t.q = ldr(rec.pos + j);
+                        t.a = ldr(reinterpret_cast<const V2<R>*>(rec.f1 + j));
+                        t.s = __ldg(pn + j);
+                        return t;
+                    };
+        auto terms = [&](int j, const NbQ2S<R>& t, T& o) {
+            if (tag_ptype(t.q.w) >= 1000) return false;
+            Disp<R> g = disp(P, qi, t.q, S.x, S.y, S.z, i, j);
+            R r2 = g.dx * g.dx + g.dy * g.dy + g.dz * g.dz, r, rinv;
+            rdist(r2, r, rinv);
+            R dw = kdw(K, r);
+            o.gx = dw * g.dx * rinv;
+            o.gy = dw * g.dy * rinv;
+            o.gz = dw * g.dz * rinv;
+            cm_apply(Cm, kgc, o.gx, o.gy, o.gz);
+            o.c = cpi * t.a.x * (pi + t.s) * rcp(t.a.y);
+            return true;
+        };
+        auto add = [&](const T& o) {
+            fx += o.c * o.gx;
+            fy += o.c * o.gy;
+            fz += o.c * o.gz;
+        };
+        if constexpr (L == 1)
+            nb_walk<4, NbQ2S<R>>(cnt, nb, n, i, load, [&](int j, const NbQ2S<R>& t) {
+                T o;
+                if (terms(j, t, o)) add(o);
             });
-        W.fpx[i] = fx; W.fpy[i] = fy; W.fpz[i] = fz;
+        else
+            ordered_walk<L, NbQ2S<R>, T>(grp, cnt, [&](int k) { return __ldg(nb + nb_at(k, n, i)); }, load, terms, add);
+        if (grp.lane == 0) W.fpx[i] = fx, W.fpy[i] = fy, W.fpz[i] = fz;
     }
+    if (grp.lane) return;
     if (pt == 9) {
         rec.ut[i] = mk4<R>(S.ux[i], S.uy[i], S.uz[i], S.temp[i]);
         return;
@@ -3461,10 +3651,11 @@ __global__ void __launch_bounds__(128) k_passC_any(DevParams P, SphState<R> S, S
     rec.ut[i] = mk4<R>(uxc, uyc, uzc, tn);
 }
 
-template <typename R, int KT>
+template <typename R, int KT, int L>
 __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 6 : 1) k_xsph_any(DevParams P, SphState<R> S, SphWork<R> W) {
     grid_dep_wait();
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const LaneGroup<L> grp;
+    const int i = grp.i;
     int n = P.ns;
     if (i >= n) return;
     const SphRec<R> rec = W.rec;
@@ -3482,30 +3673,48 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 6 : 1) k_xsph_any(DevPar
     int cnt = min(W.ncnt[i], P.nb_cap);
     R tx = 0, ty = 0, tz = 0, tt = 0, flt = 0;
     const int* __restrict__ nb = W.nbr;
-    nb_walk<4, NbQ24<R>>(
-        cnt, nb, n, i,
-        [&](int j) {
-            NbQ24<R> t;
-            t.q = ldr(rec.pos + j);
-            t.a = ldr(reinterpret_cast<const V2<R>*>(rec.f1 + j));
-            t.b = ldr(rec.ut + j);
-            return t;
-        },
-        [&](int j, const NbQ24<R>& t) {
-            int ptj = tag_ptype(t.q.w);
-            if (ptj != 1 && ptj != 3) return;
-            Disp<R> g = disp(P, qi, t.q, S.x, S.y, S.z, i, j);
-            R r2 = g.dx * g.dx + g.dy * g.dy + g.dz * g.dz, r, rinv;
-            rdist(r2, r, rinv);
-            R w = kw(K, r);
-            R m = t.a.x * rcp(t.a.y) * w;
-            R cm = c * m;
-            tx += cm * (t.b.x - uxi);
-            ty += cm * (t.b.y - uyi);
-            tz += cm * (t.b.z - uzi);
-            tt += (R)0.01 * cm * (t.b.w - ti);
-            flt += m;
+    struct T {
+        R p, w, ux, uy, uz, t;
+    };
+    auto load = [&](int j) {
+                NbQ24<R> t;
+                t.q = ldr(rec.pos + j);
+                t.a = ldr(reinterpret_cast<const V2<R>*>(rec.f1 + j));
+                t.b = ldr(rec.ut + j);
+                return t;
+            };
+    auto terms = [&](int j, const NbQ24<R>& t, T& o) {
+        int ptj = tag_ptype(t.q.w);
+        if (ptj != 1 && ptj != 3) return false;
+        Disp<R> g = disp(P, qi, t.q, S.x, S.y, S.z, i, j);
+        R r2 = g.dx * g.dx + g.dy * g.dy + g.dz * g.dz, r, rinv;
+        rdist(r2, r, rinv);
+        R w = kw(K, r);
+        o.p = t.a.x * rcp(t.a.y);
+        o.w = w;
+        o.ux = t.b.x - uxi;
+        o.uy = t.b.y - uyi;
+        o.uz = t.b.z - uzi;
+        o.t = t.b.w - ti;
+        return true;
+    };
+    auto add = [&](const T& o) {
+        R m = o.p * o.w;
+        R cm = c * m;
+        tx += cm * o.ux;
+        ty += cm * o.uy;
+        tz += cm * o.uz;
+        tt += (R)0.01 * cm * o.t;
+        flt += m;
+    };
+    if constexpr (L == 1)
+        nb_walk<4, NbQ24<R>>(cnt, nb, n, i, load, [&](int j, const NbQ24<R>& t) {
+            T o;
+            if (terms(j, t, o)) add(o);
         });
+    else
+        ordered_walk<L, NbQ24<R>, T>(grp, cnt, [&](int k) { return __ldg(nb + nb_at(k, n, i)); }, load, terms, add);
+    if (grp.lane) return;
     R on = (R)(pt > 0);
     R iflt = rcp(flt);
     W.u_tmpx[i] = (uxi + tx * iflt) * on;
