@@ -146,27 +146,30 @@ __global__ void k_cells_gather_sph(DevParams P, SphState<R> src, SphGatherSrc<R>
     int n = P.ns;
     if (i >= n) return;
     int p = perm[i];
-    double x = src.x[p], y = src.y[p], z = src.z[p];
+    // all loads before the first store (see k_cells_gather_dem)
+    double x = src.x[p], y = src.y[p], z = src.z[p], h = src.h[p];
+    R ux = gsrc.ux[p], uy = gsrc.uy[p], uz = gsrc.uz[p], m = gsrc.m[p], rho = gsrc.rho[p], pr = gsrc.pres[p];
+    const R temp = gsrc.temp[p], dd = src.dDEMpor[p], fs = src.flt_s[p], dp = src.dpres[p];
+    int pt = src.ptype[p], bt = src.btype[p], it = src.itype[p];
+    const int id = src.pid[p];
     dst.x[i] = x;
     dst.y[i] = y;
     dst.z[i] = z;
-    dst.h[i] = src.h[p];
-    R ux = gsrc.ux[p], uy = gsrc.uy[p], uz = gsrc.uz[p], m = gsrc.m[p], rho = gsrc.rho[p], pr = gsrc.pres[p];
+    dst.h[i] = h;
     dst.ux[i] = ux;
     dst.uy[i] = uy;
     dst.uz[i] = uz;
     dst.m[i] = m;
     dst.rho[i] = rho;
     dst.pres[i] = pr;
-    dst.temp[i] = gsrc.temp[p];
-    dst.dDEMpor[i] = src.dDEMpor[p];
-    dst.flt_s[i] = src.flt_s[p];
-    dst.dpres[i] = src.dpres[p];
-    int pt = src.ptype[p], bt = src.btype[p], it = src.itype[p];
+    dst.temp[i] = temp;
+    dst.dDEMpor[i] = dd;
+    dst.flt_s[i] = fs;
+    dst.dpres[i] = dp;
     dst.ptype[i] = pt;
     dst.btype[i] = bt;
     dst.itype[i] = it;
-    dst.pid[i] = src.pid[p];
+    dst.pid[i] = id;
     const PosRec<R> q = make_pos<R>(P, x, y, z, pt, bt, it);
     store_pos(rec.pos, i, q);
     rec.mr0[i] = mk2<R>(m, rho);
@@ -220,21 +223,25 @@ __global__ void k_cells_gather_dem(DevParams P, DemState<R> src, DemState<R> dst
     int n = P.nd;
     if (i >= n) return;
     int p = perm[i];
-    const R x = src.x[p], y = src.y[p], z = src.z[p], rad = src.rad[p], m = src.m[p];
-    const R ux = src.ux[p], uy = src.uy[p], uz = src.uz[p];
-    dst.x[i] = x; dst.y[i] = y; dst.z[i] = z;
-    dst.h[i] = src.h[p]; dst.rad[i] = rad;
+    // all loads before the first store: the sets may alias for all the compiler
+    // knows, so a load waited behind each store, 26 latencies in a row.  20,000
+    // spheres with their contact history: 27 -> 17 us
+    const R x = src.x[p], y = src.y[p], z = src.z[p], h = src.h[p], rad = src.rad[p];
+    const R ux = src.ux[p], uy = src.uy[p], uz = src.uz[p], wx = src.wx[p], wy = src.wy[p], wz = src.wz[p];
+    const R m = src.m[p], rho = src.rho[p], ri = src.ri[p];
+    const R t0 = src.temp[p], t1 = src.temp1[p], t2 = src.temp2[p], t3 = src.temp3[p];
+    const R fx = src.Fdx_df[p], fy = src.Fdy_df[p], fz = src.Fdz_df[p], qs = src.Q_sd[p];
+    const int pt = src.ptype[p], bt = src.btype[p], it = src.itype[p], id = src.pid[p], di = src.dem_idx[p];
+    dst.x[i] = x; dst.y[i] = y; dst.z[i] = z; dst.h[i] = h; dst.rad[i] = rad;
     dst.ux[i] = ux; dst.uy[i] = uy; dst.uz[i] = uz;
+    dst.wx[i] = wx; dst.wy[i] = wy; dst.wz[i] = wz;
+    dst.m[i] = m; dst.rho[i] = rho; dst.ri[i] = ri;
+    dst.temp[i] = t0; dst.temp1[i] = t1; dst.temp2[i] = t2; dst.temp3[i] = t3;
+    dst.Fdx_df[i] = fx; dst.Fdy_df[i] = fy; dst.Fdz_df[i] = fz; dst.Q_sd[i] = qs;
+    dst.ptype[i] = pt; dst.btype[i] = bt; dst.itype[i] = it; dst.pid[i] = id; dst.dem_idx[i] = di;
     // what the SPH passes read of a sphere
     DW.ra[i] = Dbl4{x, y, z, rad};
     DW.rb[i] = Dbl4{ux, uy, uz, m};
-    dst.wx[i] = src.wx[p]; dst.wy[i] = src.wy[p]; dst.wz[i] = src.wz[p];
-    dst.m[i] = m; dst.rho[i] = src.rho[p]; dst.ri[i] = src.ri[p];
-    dst.temp[i] = src.temp[p]; dst.temp1[i] = src.temp1[p]; dst.temp2[i] = src.temp2[p]; dst.temp3[i] = src.temp3[p];
-    dst.Fdx_df[i] = src.Fdx_df[p]; dst.Fdy_df[i] = src.Fdy_df[p]; dst.Fdz_df[i] = src.Fdz_df[p];
-    dst.Q_sd[i] = src.Q_sd[p];
-    dst.ptype[i] = src.ptype[p]; dst.btype[i] = src.btype[p]; dst.itype[i] = src.itype[p];
-    dst.pid[i] = src.pid[p]; dst.dem_idx[i] = src.dem_idx[p];
 }
 
 // SPH neighbour list: the candidate set and predicate of every SPH gather
