@@ -288,7 +288,8 @@ int nnps_sph(SphdemHandle* H, EngineHost<R>* EH, int src, int dst, int64_t* nl) 
 }
 
 template <typename R>
-int nnps_dem(SphdemHandle* H, EngineHost<R>* EH, int src, int dst, int64_t* nl, cudaStream_t st) {
+int nnps_dem(SphdemHandle* H, EngineHost<R>* EH, int src, int dst, int64_t* nl, cudaStream_t st,
+             cudaEvent_t sorted = nullptr) {
     Engine<R>& E = EH->E;
     DevParams& P = E.P;
     DemWork<double>& DW = E.dw;
@@ -310,13 +311,16 @@ int nnps_dem(SphdemHandle* H, EngineHost<R>* EH, int src, int dst, int64_t* nl, 
     {
         KTIME_ON(KT_GATHER_D, st);
         CK((launch_pdl(k_cells_gather_dem<double>, nblocks(n, TPB), TPB, 0, st, P, D, E.D[dst], DW.val_out, DW)));
-        CK((launch_pdl(k_gather_history, nblocks(n * SPHDEM_NSLOT, TPB), TPB, 0, st, n, DW.val_out, D.hid, D.hds, E.D[dst].hid,
-                                                                         E.D[dst].hds)));
     }
     {
         KTIME_ON(KT_ROWS_D, st);
         CK((launch_pdl(k_rows, nblocks(P.NI * P.NJ * P.NK, TPB), TPB, 0, st, P, DW.g_str, DW.g_end, DW.rows)));
     }
+    // the sorted set and its rows are complete (the SPH -> DEM list may start
+    // on the other stream); the history follows for the contact
+    if (sorted) CK(cudaEventRecord(sorted, st));
+    CK((launch_pdl(k_gather_history, nblocks(n * SPHDEM_NSLOT, TPB), TPB, 0, st, n, DW.val_out, D.hid, D.hds,
+                   E.D[dst].hid, E.D[dst].hds)));
     *nl += 8;
     CK(cudaGetLastError());
     return SPHDEM_OK;
@@ -708,12 +712,16 @@ int tune_dlist(SphdemHandle* H, EngineHost<R>* EH, const SphState<R>& S, const D
 // The DEM kernels that read no SPH pass run on a second stream, forked from
 // and joined to the step stream by events (in the step graph: parallel
 // branches):
-//   step stream: SPH NNPS -> list (or, after a call's first step, the
-//                hand-over in place) -> [SPH->DEM list built] pass A -> pass B
+//   step stream: SPH NNPS -> list -> [SPH->DEM list built] pass A -> pass B
 //                -> [DEM prep done] DEM coupling -> SPH coupling -> walls, PPE,
 //                pass C, open boundary, XSPH -> [DEM update done] tick
 //   DEM stream:  DEM NNPS -> [SPH gathered] SPH->DEM list -> contact -> DEM prep
 //                ... [SPH coupling done] DEM corrector + walls
+// After a call's first step the step stream has no NNPS and no list build:
+//   step stream: hand-over in place -> [DEM set sorted] SPH->DEM list -> pass A ...
+//   DEM stream:  DEM NNPS -> history gather -> [SPH gathered] contact -> DEM prep ...
+// so the list build runs beside the contact instead of before it, and the DEM
+// prep ends earlier (bench bed 0.672 -> 0.653 ms per step).
 // The SPH -> DEM list reads both sorted sets; the DEM contact reads only
 // the DEM set; the DEM prep reads the gathered SPH records and the DEM set;
 // the DEM corrector writes the DEM set after the SPH coupling has read it,
@@ -752,7 +760,9 @@ int enqueue_step(SphdemHandle* H, EngineHost<R>* EH, int flags, int64_t* nl) {
     auto wait = [&](int k, cudaStream_t b) { return fork ? cudaStreamWaitEvent(b, H->fork_ev[k], 0) : cudaSuccess; };
     CK(rec(0, st));
     CK(wait(0, sd));
-    if ((r = nnps_dem<R>(H, EH, dox, dn, nl, sd))) return r;
+    // the step stream is idle until the SPH -> DEM list is there (see above)
+    const bool list_here = fork && keep;
+    if ((r = nnps_dem<R>(H, EH, dox, dn, nl, sd, list_here ? H->fork_ev[1] : nullptr))) return r;
     SphState<R>& S = E.S[sn];
     DemState<double>& D = E.D[dn];
     const bool sl = small_set_lanes(P);
@@ -767,12 +777,13 @@ int enqueue_step(SphdemHandle* H, EngineHost<R>* EH, int flags, int64_t* nl) {
     }
     CK(rec(2, st));   // SPH set gathered
     CK(wait(2, sd));
+    if (list_here) CK(wait(1, st));   // DEM set sorted
     if (ns > 0 && nd > 0) {
-        KTIME_ON(KT_DLIST, sd);
-        CK(launch_dlist<R>(EH, S, D, sd));
+        KTIME_ON(KT_DLIST, list_here ? st : sd);
+        CK(launch_dlist<R>(EH, S, D, list_here ? st : sd));
         *nl += 1;
     }
-    CK(rec(1, sd));   // SPH -> DEM list built
+    if (!list_here) CK(rec(1, sd));   // SPH -> DEM list built
     if (nd > 0) {
         {
             KTIME_ON(KT_DEMCONTACT, sd);
@@ -796,7 +807,7 @@ int enqueue_step(SphdemHandle* H, EngineHost<R>* EH, int flags, int64_t* nl) {
             CK(launch_list<R>(EH, S, EH->list_mode, st));
             *nl += 1;
         }
-        CK(wait(1, st));
+        if (!list_here) CK(wait(1, st));
         { KTIME(KT_PASSA); CK((launch_pdl(kt3 ? k_passA<R> : sl ? (kt5 ? k_passA_any<R, 5, 8> : k_passA_any<R, -1, 8>) : kt5 ? k_passA_any<R, 5, 1> : k_passA_any<R, -1, 1>, bl, TPB, 0, st, P, S, W, D, DW, DW.rows))); }
         *nl += 1;
         {
@@ -815,7 +826,7 @@ int enqueue_step(SphdemHandle* H, EngineHost<R>* EH, int flags, int64_t* nl) {
         *nl += 1;
     }
     CK(rec(3, sd));   // DEM contact and prep done
-    CK(wait(1, st));  // (without SPH particles the list wait above was skipped)
+    if (!list_here) CK(wait(1, st));  // (without SPH particles the list wait above was skipped)
     CK(wait(3, st));
     if (nd > 0) {
         {
