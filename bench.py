@@ -229,6 +229,14 @@ def profiled_traffic(kernel):
     return None
 
 
+def one_step_calls(eng, n):
+    """n steps in calls of one step, the calls that are timed: the engine
+    captures a step graph per place in a call and buffer parity, and steps
+    inside a longer call are not a call's first step."""
+    for _ in range(n):
+        eng.step(1)
+
+
 def load_peaks():
     path = os.path.join(ROOT, "MEASURED_PEAKS.json")
     try:
@@ -601,7 +609,7 @@ def run_column(args, world, rank, local, pg):
     n = eng.ns
     stream = torch.cuda.ExternalStream(eng.stream_ptr())
     flush = torch.empty(256 * 1024 * 1024 // 4, dtype=torch.float32, device="cuda")
-    eng.step(args.warmup)
+    one_step_calls(eng, args.warmup)
     torch.cuda.synchronize()
     vis = os.environ.get("CUDA_VISIBLE_DEVICES", "").split(",")[0]
     sampler = ClockSampler(int(vis) if vis.isdigit() else local)
@@ -656,7 +664,7 @@ def run_column(args, world, rank, local, pg):
         q2.ppe_precond = PRECOND_TWO_LEVEL
         e2 = Engine(q2, sph, {})
         s2 = torch.cuda.ExternalStream(e2.stream_ptr())
-        e2.step(args.warmup)
+        one_step_calls(e2, args.warmup)
         it2, t2 = [], 0.0
         for _ in range(args.steps):
             t2 += _timed_steps(e2, s2, flush, 1)
@@ -743,7 +751,7 @@ def run_dam2d_batch(args, world, rank, local, pg):
     n = eng.ns
     stream = torch.cuda.ExternalStream(eng.stream_ptr())
     flush = torch.empty(256 * 1024 * 1024 // 4, dtype=torch.float32, device="cuda")
-    eng.step(args.warmup)
+    one_step_calls(eng, args.warmup)
     torch.cuda.synchronize()
     vis = os.environ.get("CUDA_VISIBLE_DEVICES", "").split(",")[0]
     sampler = ClockSampler(int(vis) if vis.isdigit() else local)
@@ -794,7 +802,7 @@ def run_dam2d_batch(args, world, rank, local, pg):
         for bd in beds:
             e = Engine(q1, bd, {})
             st = torch.cuda.ExternalStream(e.stream_ptr())
-            e.step(3)
+            one_step_calls(e, 3)
             seq_ms += _timed_steps(e, st, flush, ks) / ks
             e.close()
     line = {
@@ -866,12 +874,12 @@ def run_bed2d_batch(args, world, rank, local, pg):
     n = eng.ns + eng.nd
     stream = torch.cuda.ExternalStream(eng.stream_ptr())
     flush = torch.empty(256 * 1024 * 1024 // 4, dtype=torch.float32, device="cuda")
-    eng.step(args.warmup)
+    one_step_calls(eng, args.warmup)
     torch.cuda.synchronize()
     # per-kernel breakdown (in-graph events, every kernel) before the timed
     # region, which runs without events
     eng.set_timing(True)
-    eng.step(2)
+    one_step_calls(eng, 2)
     eng.collect_timing()
     b0 = eng.timing()
     for _ in range(PROFILE_STEPS // 2):
@@ -883,7 +891,7 @@ def run_bed2d_batch(args, world, rank, local, pg):
     kms = {k: round(v, 4) for k, v in sorted(kms.items(), key=lambda kv: -kv[1]) if v > 0}
     # the same with the DEM branch on the step stream: each kernel alone
     eng.set_concurrency(False)
-    eng.step(2)
+    one_step_calls(eng, 2)
     eng.collect_timing()
     b1 = eng.timing()
     for _ in range(PROFILE_STEPS // 2):
@@ -895,7 +903,7 @@ def run_bed2d_batch(args, world, rank, local, pg):
     kser = {k: round(v, 4) for k, v in sorted(kser.items(), key=lambda kv: -kv[1]) if v > 0}
     eng.set_concurrency(True)
     eng.set_timing(False)
-    eng.step(2)
+    one_step_calls(eng, 2)
     torch.cuda.synchronize()
     vis = os.environ.get("CUDA_VISIBLE_DEVICES", "").split(",")[0]
     sampler = ClockSampler(int(vis) if vis.isdigit() else local)
@@ -949,7 +957,7 @@ def run_bed2d_batch(args, world, rank, local, pg):
         for sb, db, rb in parts:
             e = Engine(q, sb, db, beds=rb)
             st = torch.cuda.ExternalStream(e.stream_ptr())
-            e.step(3)
+            one_step_calls(e, 3)
             seq_ms += _timed_steps(e, st, flush, ks) / ks
             e.close()
     line = {
@@ -1028,10 +1036,10 @@ def run_dam2d(args, world, rank, local, pg):
     n = eng.ns
     stream = torch.cuda.ExternalStream(eng.stream_ptr())
     flush = torch.empty(256 * 1024 * 1024 // 4, dtype=torch.float32, device="cuda")
-    eng.step(args.warmup)
+    one_step_calls(eng, args.warmup)
     torch.cuda.synchronize()
     eng.set_timing(True)
-    eng.step(2)
+    one_step_calls(eng, 2)
     eng.collect_timing()
     counts, _ = eng.neighbors(cap=1)
     avg_nb = float(counts.mean())
@@ -1139,7 +1147,7 @@ def run_engine(args, world, rank, local, pg):
     stream = torch.cuda.ExternalStream(eng.stream_ptr())
     flush = torch.empty(256 * 1024 * 1024 // 4, dtype=torch.float32, device="cuda")
 
-    eng.step(args.warmup)
+    one_step_calls(eng, args.warmup)
     torch.cuda.synchronize()
     # Per-kernel breakdown: every kernel timed by in-graph events over
     # PROFILE_STEPS steps before the timed region (each timed kernel adds two
@@ -1147,7 +1155,7 @@ def run_engine(args, world, rank, local, pg):
     # The timed region then times only the dominant kernel, live, for the
     # roofline.
     eng.set_timing(True)
-    eng.step(2)          # capture both graph parities with timing events
+    one_step_calls(eng, 2)          # capture both graph parities with timing events
     eng.collect_timing()
     b0 = eng.timing()
     for _ in range(PROFILE_STEPS):
@@ -1159,7 +1167,7 @@ def run_engine(args, world, rank, local, pg):
     per_kernel = {k: (v[0] - b0.get(k, (0, 0))[0], v[1] - b0.get(k, (0, 0))[1]) for k, v in t_prof.items()}
     dom_name = max(per_kernel.items(), key=lambda kv: kv[1][0])[0]
     eng.set_timing_only(dom_name)
-    eng.step(2)          # recapture with the dominant kernel's events only
+    one_step_calls(eng, 2)          # recapture with the dominant kernel's events only
     eng.collect_timing()
     counts, _ = eng.neighbors(cap=1)
     avg_nb = float(counts.mean()) if eng.ns else 0.0
@@ -1225,7 +1233,7 @@ def run_engine(args, world, rank, local, pg):
     serial = None
     if eng.ns and eng.nd:
         eng.set_concurrency(False)
-        eng.step(2)
+        one_step_calls(eng, 2)
         eng.collect_timing()
         b2 = eng.timing()
         ks = max(3, min(args.steps, 10))
@@ -1348,7 +1356,7 @@ def precision_keys(args, seed):
     q.precision = 1
     e64 = Engine(q, sph, dem)
     stream = torch.cuda.ExternalStream(e64.stream_ptr())
-    e64.step(args.warmup)
+    one_step_calls(e64, args.warmup)
     torch.cuda.synchronize()
     total = 0.0
     for _ in range(args.steps):
