@@ -1516,6 +1516,8 @@ __global__ void __launch_bounds__(128, 4) k_dem_contact(DevParams P, DemState<do
         oid[s] = D.hid[s * n + i];
         if (free_slot < 0 && oid[s] < 1) free_slot = s;
     }
+    // every lane of the group holds the start-of-step ids before one releases a slot
+    if constexpr (G > 1) __syncwarp(gm);
     Q tx = 0, ty = 0, tz = 0, tqx = 0, tqy = 0, tqz = 0, dtr = 0, dtc = 0;
     const double kdt = P.dt;
     // this lane's last new contact (visit order t) and its spring
