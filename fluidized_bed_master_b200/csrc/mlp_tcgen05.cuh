@@ -218,11 +218,13 @@ __device__ __forceinline__ void load_vectors(float* v, const MlpDev& net) {
     }
 }
 
-// a row's features as loaded (zero past n), and its place in the X tile
+// a row's features as loaded (zero past n), and its place in the X tile.  Rows
+// are unsigned: the row of the next tile lies up to a grid of tiles past n, which
+// may itself be close to 2^31.
 struct XRow {
     uint4 a, b;
 };
-__device__ __forceinline__ XRow ld_x_row(const __nv_bfloat16* feat, int n, int row) {
+__device__ __forceinline__ XRow ld_x_row(const __nv_bfloat16* feat, unsigned n, unsigned row) {
     XRow x{make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
     if (row < n) {
         const uint4* src = reinterpret_cast<const uint4*>(feat + (size_t)row * MLP_IN);
@@ -305,7 +307,7 @@ __global__ void __launch_bounds__(128, MLP_INFER_CTAS) k_mlp_infer(int n, const 
     const int ntiles = (n + MLP_TILE - 1) / MLP_TILE;
     XRow x = ld_x_row(feat, n, blockIdx.x * MLP_TILE + tid);
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const int row = tile * MLP_TILE + tid;
+        const unsigned row = tile * MLP_TILE + tid;
         st_x_row(sm, tid, x);
         MLP_SYNC_ISSUE(tc_mma(tm + TM_D1, smem_desc(sm + SM_X, 128, 256), smem_desc(sm + SM_W1, 128, 256), id64, 0));
         x = ld_x_row(feat, n, row + gridDim.x * MLP_TILE);   // the next tile's, while this one is worked on
@@ -326,7 +328,7 @@ __global__ void __launch_bounds__(128, MLP_INFER_CTAS) k_mlp_infer(int n, const 
         tc_ld64(tm + lane_off + TM_D2, v);
 #pragma unroll
         for (int q = 0; q < MLP_H; q++) y += fmaxf(v[q] + vec[MLP_H + q], 0.f) * vec[2 * MLP_H + q];
-        if (row < n) out[row] = fail ? 0.f : y;
+        if (row < (unsigned)n) out[row] = fail ? 0.f : y;
         tc_fence_before();
         __syncthreads();
         if (fail) break;
@@ -395,11 +397,12 @@ __global__ void __launch_bounds__(128, MLP_GRAD_CTAS) k_mlp_grad(int n, const __
     const int stall = 0;
     int first = 1;
     const int ntiles = (n + MLP_TILE - 1) / MLP_TILE;
-    int row = blockIdx.x * MLP_TILE + tid;
-    XRow x = ld_x_row(feat, n, row);
-    float wn = row < n ? __ldg(weight + row) : 0.f, tn = row < n ? __ldg(target + row) : 0.f;
+    const unsigned nu = n;
+    unsigned row = blockIdx.x * MLP_TILE + tid;
+    XRow x = ld_x_row(feat, nu, row);
+    float wn = row < nu ? __ldg(weight + row) : 0.f, tn = row < nu ? __ldg(target + row) : 0.f;
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const bool valid = row < n;
+        const bool valid = row < nu;
         const float wi = wn, ti = tn;
         st_x_row(sm, tid, x);
         {
@@ -416,9 +419,9 @@ __global__ void __launch_bounds__(128, MLP_GRAD_CTAS) k_mlp_grad(int n, const __
         MLP_SYNC_ISSUE(tc_mma(tm + TM_D1, smem_desc(sm + SM_X, 128, 256), smem_desc(sm + SM_W1, 128, 256), id64, 0));
         // the next tile's row, while this one is worked on
         row += gridDim.x * MLP_TILE;
-        x = ld_x_row(feat, n, row);
-        wn = row < n ? __ldg(weight + row) : 0.f;
-        tn = row < n ? __ldg(target + row) : 0.f;
+        x = ld_x_row(feat, nu, row);
+        wn = row < nu ? __ldg(weight + row) : 0.f;
+        tn = row < nu ? __ldg(target + row) : 0.f;
         uint32_t m1lo = 0, m1hi = 0;   // ReLU masks of layer 1 (bit c: z1_c > 0)
         float v[MLP_H];
         tc_ld64(tm + lane_off + TM_D1, v);
