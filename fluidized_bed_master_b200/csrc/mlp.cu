@@ -46,8 +46,10 @@ int mlp_alloc(MlpNet& m) {
     if (cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, SM_TRAIN_END + SM_ALIGN) !=
             cudaSuccess ||
         cudaFuncSetAttribute(k_mlp_infer, cudaFuncAttributeMaxDynamicSharedMemorySize, SM_INFER_END + SM_ALIGN) !=
-            cudaSuccess)
+            cudaSuccess) {
+        mlp_free(m);
         return SPHDEM_E_CUDA;
+    }
     return SPHDEM_OK;
 }
 
