@@ -1,6 +1,7 @@
 // mlp.cu -- host side of the learned PPE warm start network
 // (mlp_tcgen05.cuh): device buffers, launches, and the C-ABI entry points
 // that run the network on caller-owned device arrays.
+#include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <algorithm>
@@ -161,25 +162,83 @@ using namespace sphdem;
 // device time of the last forward / gradient kernel of this host thread
 static thread_local double g_last_fwd_ms = 0.0, g_last_grad_ms = 0.0;
 
+// Contexts by id.  An id belongs to one context of the program: after a device
+// reset the primary context comes back at the same address with another id.
+// 0: not known.  The driver's entries come through the runtime (no link to
+// libcuda).
+struct DriverCtx {
+    CUresult (*current)(CUcontext*) = nullptr;
+    CUresult (*id_of)(CUcontext, unsigned long long*) = nullptr;
+    CUresult (*state)(CUdevice, unsigned*, int*) = nullptr;
+    CUresult (*retain)(CUcontext*, CUdevice) = nullptr;
+    CUresult (*release)(CUdevice) = nullptr;
+    bool ok;
+    template <typename F>
+    static bool entry(const char* name, F& f) {
+        cudaDriverEntryPointQueryResult q;
+        return cudaGetDriverEntryPoint(name, (void**)&f, cudaEnableDefault, &q) == cudaSuccess && f &&
+               q == cudaDriverEntryPointSuccess;
+    }
+    DriverCtx()
+        : ok(entry("cuCtxGetCurrent", current) && entry("cuCtxGetId", id_of) &&
+             entry("cuDevicePrimaryCtxGetState", state) && entry("cuDevicePrimaryCtxRetain", retain) &&
+             entry("cuDevicePrimaryCtxRelease", release)) {}
+    static const DriverCtx& get() {
+        static const DriverCtx d;
+        return d;
+    }
+};
+// of the context that this thread's calls run in
+static unsigned long long current_ctx() {
+    const DriverCtx& d = DriverCtx::get();
+    CUcontext c = nullptr;
+    unsigned long long id = 0;
+    if (!d.ok || d.current(&c) != CUDA_SUCCESS || !c || d.id_of(c, &id) != CUDA_SUCCESS) return 0;
+    return id;
+}
+// of a device's primary context; 0 while it has none
+static unsigned long long primary_ctx(int dev) {
+    const DriverCtx& d = DriverCtx::get();
+    unsigned flags = 0;
+    int active = 0;
+    CUcontext c = nullptr;
+    unsigned long long id = 0;
+    if (!d.ok || d.state(dev, &flags, &active) != CUDA_SUCCESS || !active || d.retain(&c, dev) != CUDA_SUCCESS)
+        return 0;
+    if (d.id_of(c, &id) != CUDA_SUCCESS) id = 0;
+    d.release(dev);
+    return id;
+}
+
 // Workspace of the two entries below: the network's device buffers, the event
 // pair and a page-locked error word, one set per host thread.  Allocating and
 // freeing it in each call cost 2.4 ms of a 4.2 ms forward + gradient pass.
 // A call returns only when its stream has finished, so the next call of the
-// thread may use the set on any stream; another device, a failed call or the
-// thread's end frees it.
+// thread may use the set on any stream; another context (a device reset makes
+// one), a failed call or the thread's end gives it up.  What a context held
+// ends with it and is not freed again.
 struct MlpScratch {
     MlpNet net;
-    int device = -1;   // -1: nothing allocated
+    bool held = false;
+    int device = 0;
+    unsigned long long ctx = 0;   // 0: not known, the set is then not kept between calls
     int* err = nullptr;
     cudaEvent_t a = nullptr, b = nullptr;
-    int use() {   // ready on the current device
+    int use() {   // ready in the current context
         int dev = 0;
         if (cudaGetDevice(&dev) != cudaSuccess) return SPHDEM_E_CUDA;
-        if (device == dev) return SPHDEM_OK;
+        unsigned long long id = current_ctx();
+        if (!id) {   // the thread's first call, or the first after a reset
+            if (cudaFree(nullptr) != cudaSuccess) return SPHDEM_E_CUDA;
+            id = current_ctx();
+        }
+        if (held && id && id == ctx) return SPHDEM_OK;
         drop();
         int r = mlp_alloc(net);
         if (r) return r;
+        held = true;
         device = dev;
+        ctx = id;
         // its clearing runs on the legacy stream, the calls on the caller's
         if (cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess ||
             cudaHostAlloc((void**)&err, sizeof(int), cudaHostAllocDefault) != cudaSuccess ||
@@ -190,14 +249,17 @@ struct MlpScratch {
         return SPHDEM_OK;
     }
     void drop() {
-        if (device < 0) return;
-        mlp_free(net);
-        if (err) cudaFreeHost(err);
-        if (a) cudaEventDestroy(a);
-        if (b) cudaEventDestroy(b);
+        if (!held) return;
+        // (without ids a set never outlives its call, so its context is the current one)
+        if (!ctx || ctx == current_ctx() || ctx == primary_ctx(device)) {
+            mlp_free(net);
+            if (err) cudaFreeHost(err);
+            if (a) cudaEventDestroy(a);
+            if (b) cudaEventDestroy(b);
+        }
         err = nullptr;
         a = b = nullptr;
-        device = -1;
+        held = false;
     }
     ~MlpScratch() { drop(); }
 };
@@ -218,7 +280,7 @@ static int mlp_call(const float* params, cudaStream_t st, double& ms, F work) {
     if (!r && *w.err) r = SPHDEM_E_TIMEOUT;
     float t = 0.f;
     if (!r && cudaEventElapsedTime(&t, w.a, w.b) == cudaSuccess) ms = (double)t;
-    if (r) w.drop();
+    if (r || !w.ctx) w.drop();
     return r;
 }
 

@@ -66,3 +66,44 @@ def test_failed_kernel_attribute_leaves_nothing(L):
 
     _in_thread(L, run)
     assert L.fake_live(0) == 0 and L.fake_errors() == 0
+
+
+def test_device_reset_ends_the_workspace(L):
+    """The next call on the thread builds a new set, a thread's end after a reset frees nothing; neither uses what
+    ended with the context."""
+    def run():
+        assert _forward(L) == OK
+        n = L.fake_live(0)
+        assert _forward(L) == OK and L.fake_live(0) == n > 0
+        L.fake_reset()
+        assert L.fake_live(0) == 0
+        assert _forward(L) == OK and L.fake_live(0) == n and L.fake_errors() == 0
+        L.fake_reset()
+
+    _in_thread(L, run)
+    assert L.fake_live(0) == 0 and L.fake_errors() == 0
+
+
+def test_other_device_and_threads(L):
+    def run():
+        L.fake_device(0)
+        assert _forward(L) == OK
+        n = L.fake_live(0)
+        L.fake_device(1)
+        assert _forward(L) == OK and (L.fake_live(0), L.fake_live(1)) == (0, n)
+
+        def inner():
+            L.fake_device(0)
+            assert _forward(L) == OK and (L.fake_live(0), L.fake_live(1)) == (n, n)
+
+        t = threading.Thread(target=inner)
+        t.start()
+        t.join()
+        for _ in range(500):
+            if not L.fake_live(0):
+                break
+            time.sleep(0.01)
+        assert (L.fake_live(0), L.fake_live(1)) == (0, n)
+
+    _in_thread(L, run)
+    assert L.fake_live(0) == L.fake_live(1) == 0 and L.fake_errors() == 0
