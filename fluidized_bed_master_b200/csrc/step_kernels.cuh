@@ -2271,6 +2271,7 @@ __device__ __forceinline__ void neumann_cell(int c, DevParams P, SphState<float>
         if (!__any_sync(0xffffffffu, act)) continue;
         double xi = 0, yi = 0, zi = 0, R2 = 0;
         float lo2 = 0, hi2 = 0, fx = 0, fy = 0, fz = 0;
+        float scale = 1.f;   // the sums times scale are the normalised sums
         Knl<float> K{};
         bool slow = false;
         if (act) {
@@ -2282,6 +2283,10 @@ __device__ __forceinline__ void neumann_cell(int c, DevParams P, SphState<float>
             K = knl_make<float>(P, (float)hi);
             K.ih = rcp(th2);
             K.th = th2;
+            if (KT != 5 && K.kt == 3) {   // every chunk's sums leave out tA
+                scale = K.tA;
+                K.tA = 1.f;
+            }
             R2 = 2.0 * (P.kappa * hi);
             const double b = rel_band(P, Fr, R2), r2 = R2 * R2;
             lo2 = (float)(r2 * (1.0 - b));
@@ -2295,7 +2300,6 @@ __device__ __forceinline__ void neumann_cell(int c, DevParams P, SphState<float>
         }
         const bool lanes_slow = __any_sync(0xffffffffu, act && slow);
         float tp = 0.f, flt = 0.f, tt = 0.f, tr = 0.f;
-        float scale = 1.f;   // the sums times scale are the normalised sums
         int t = 0;   // next raw candidate
         while (t < tot) {
             // stage fluid candidates in order until the chunk is full
@@ -2365,7 +2369,6 @@ __device__ __forceinline__ void neumann_cell(int c, DevParams P, SphState<float>
                         tr += bj.w * wk;
                     }
                 }
-                scale = K.tA;
             } else if (KT == 5 && act && !slow_chunk) {
                 // Wendland C6, four candidates at a time without branches
                 // between them (the band's FP64 predicate: one branch per
