@@ -3106,7 +3106,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 6 : 1) k_xsph(DevParams 
         },
         [&](int, const NbP4<R>& t, const PairV<R>& g) {
             const R v = g.vs;
-            const bool in = v > (R)0;   // a wall's fields stay out of the sums
+            const bool in = v != (R)0;   // a wall's fields stay out of the sums
             const R r2 = g.dx * g.dx + g.dy * g.dy + g.dz * g.dz;
             const R r = r2 * rsq_floor(r2);
             const R m = v * c2_w(K, r);
