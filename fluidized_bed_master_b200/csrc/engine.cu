@@ -1877,7 +1877,7 @@ static int w_commit_t(SphdemHandle* H) {
     W.g_str = A.get<int>(P.num_cells + 1); W.g_end = A.get<int>(P.num_cells + 1);
     W.rows = A.get<int4>(NI * NJ * NK);
     W.ncnt = A.get<int>(ns);
-    W.rp = A.get<V4<R>>(ns);
+    W.rp = A.get<WPos<R>>(ns);
     W.rb = A.get<V4<R>>(ns);
     W.rc = sizeof(R) == 4 ? A.get<V2<R>>(ns) : nullptr;
     W.nbr = nullptr;

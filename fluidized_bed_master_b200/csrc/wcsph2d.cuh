@@ -71,6 +71,20 @@ __device__ __forceinline__ double2 w_cell_off(const WState<R>& S, int i) {
     return S.boff ? S.boff[S.bed[i]] : make_double2(0.0, 0.0);
 }
 
+// the position record of the neighbour loops (WWork::rp)
+template <typename R>
+struct WPosT;
+template <>
+struct WPosT<float> {
+    typedef double2 t;
+};
+template <>
+struct WPosT<double> {
+    typedef Dbl4 t;
+};
+template <typename R>
+using WPos = typename WPosT<R>::t;
+
 template <typename R>
 struct WWork {
     R *ftx, *fty, *ftot, *drho;  // last step's values (read by the predictor in the old order)
@@ -82,34 +96,32 @@ struct WWork {
     int *key_in, *key_out, *val_in, *val_out, *g_str, *g_end, *nbr, *ncnt;
     int4* rows;
     // neighbour records of the sorted, predicted state (k_w_gather):
-    //   FP32: rp {x_hi, x_lo, y_hi, y_lo} (x = x_hi + x_lo to 2^-48), rc {rho, +-h}
+    //   FP32: rp {x, y}, rc {rho, +-h}
     //   FP64: rp {x, y, rho, +-h}
     // rb {ux, uy, m / rho, p}; h negative for p_type <= 0
-    V4<R>*rp, *rb;
+    WPos<R>* rp;
+    V4<R>* rb;
     V2<R>* rc;
 };
 
-__device__ __forceinline__ float4 w_pos_rec(double x, double y, float, float) {
-    const float xh = (float)x, yh = (float)y;
-    return make_float4(xh, (float)(x - (double)xh), yh, (float)(y - (double)yh));
+__device__ __forceinline__ void w_pos_rec(double2* p, double x, double y, float, float) { *p = make_double2(x, y); }
+__device__ __forceinline__ void w_pos_rec(Dbl4* p, double x, double y, double rho, double h) {
+    *p = Dbl4{x, y, rho, h};
 }
-__device__ __forceinline__ Dbl4 w_pos_rec(double x, double y, double rho, double h) { return Dbl4{x, y, rho, h}; }
-// displacement x_i - x_j: FP32 differences of the high parts are exact for
-// neighbours, so it is rounded once, like (float)(x_i - x_j)
-__device__ __forceinline__ float2 w_disp(const float4& a, const float4& b) {
-    return make_float2((a.x - b.x) + (a.y - b.y), (a.z - b.z) + (a.w - b.w));
+// displacement x_i - x_j
+template <typename T>
+__device__ __forceinline__ double2 w_disp(const T& a, const T& b) { return make_double2(a.x - b.x, a.y - b.y); }
+// its length, rounded once to R.  FP32: the root of the rounded square, put
+// right by its residual in FP64
+__device__ __forceinline__ float w_len(const double2& d, float) {
+    const double r2 = d.x * d.x + d.y * d.y;
+    const float t = (float)r2, s = rsq_floor(t), r = t * s;
+    return fmaf((float)(r2 - (double)r * (double)r), 0.5f * s, r);
 }
-__device__ __forceinline__ double2 w_disp(const Dbl4& a, const Dbl4& b) { return make_double2(a.x - b.x, a.y - b.y); }
+__device__ __forceinline__ double w_len(const double2& d, double) { return sqrt(d.x * d.x + d.y * d.y); }
 // {rho, +-h} of slot j
-__device__ __forceinline__ float2 w_rho_h(const float4&, const float2* rc, int j) { return ldr(rc + j); }
+__device__ __forceinline__ float2 w_rho_h(const double2&, const float2* rc, int j) { return ldr(rc + j); }
 __device__ __forceinline__ double2 w_rho_h(const Dbl4& p, const double2*, int) { return make_double2(p.z, p.w); }
-// the width (relative to Rr^2) of the band around the list radius that the
-// exact predicate decides: r^2 of w_disp is within 4 roundings (2.4e-7 in
-// FP32) plus the records' 2^-48 of the coordinates (FP64: 4 x 1.1e-16)
-__device__ __forceinline__ double w_band(float, double x, double y, double Rr) {
-    return 1e-6 + 1.5e-14 * (fabs(x) + fabs(y) + Rr) / Rr;
-}
-__device__ __forceinline__ double w_band(double, double, double, double) { return 4e-15; }
 
 struct WParams {
     double alpha, beta, delta;   // artificial viscosity, delta-SPH
@@ -217,12 +229,12 @@ __global__ void __launch_bounds__(128) k_w_list(DevParams P, WState<R> S, WWork<
     if (key < P.NI * P.NJ) {
         const int jc = key / P.NI, ic = key - jc * P.NI;
         const double xi = S.x[i], yi = S.y[i], Rr = __dmul_rn(P.kappa, S.h[i]);
-        const double bd = w_band((R)0, xi, yi, Rr), R2 = Rr * Rr;
-        const R lo = (R)(R2 * (1.0 - bd)), hi = (R)(R2 * (1.0 + bd));
-        const V4<R> pi = ldr(W.rp + i);
-        auto test = [&](const V4<R>& pj, int j) {
-            const V2<R> d = w_disp(pi, pj);
-            const R r2 = d.x * d.x + d.y * d.y;
+        // r^2 is rounded by less than 1e-15 of itself
+        const double lo = Rr * Rr * (1.0 - 4e-15), hi = Rr * Rr * (1.0 + 4e-15);
+        const WPos<R> pi = ldr(W.rp + i);
+        auto test = [&](const WPos<R>& pj, int j) {
+            const double2 d = w_disp(pi, pj);
+            const double r2 = d.x * d.x + d.y * d.y;
             if (r2 < lo) return true;
             if (r2 > hi) return false;
             return __dadd_rn(w_dist(xi, yi, S.x[j], S.y[j]), 1e-20) < Rr;
@@ -232,7 +244,7 @@ __global__ void __launch_bounds__(128) k_w_list(DevParams P, WState<R> S, WWork<
             const int4 r = __ldg(W.rows + ic + P.NI * jy);
             if constexpr (L == 1) {
                 for (int j0 = r.x; j0 < r.w; j0 += 4) {
-                    V4<R> q[4];
+                    WPos<R> q[4];
 #pragma unroll
                     for (int u = 0; u < 4; u++) q[u] = ldr(W.rp + min(j0 + u, r.w - 1));
 #pragma unroll
@@ -474,7 +486,8 @@ __global__ void __launch_bounds__(128) k_w_pair(DevParams P, WParams Q, WState<R
     if (i >= n || S.itype[i] > 2) return;
     const bool force = S.itype[i] == 1, filt = F->filt_now != 0;
     const C2Sum<R> K = c2_sum<R>(P, (R)S.h[i]);
-    const V4<R> pi = ldr(W.rp + i), bi = ldr(W.rb + i);
+    const WPos<R> pi = ldr(W.rp + i);
+    const V4<R> bi = ldr(W.rb + i);
     const V2<R> ci = w_rho_h(pi, W.rc, i);
     const R hi = fabs(ci.y), rhoi = ci.x, mi = (R)S.m[i];
     const bool mov = ci.y > (R)0;   // p_type > 0
@@ -485,10 +498,10 @@ __global__ void __launch_bounds__(128) k_w_pair(DevParams P, WParams Q, WState<R
     const R mux = mov ? bi.x : (R)0, muy = mov ? bi.y : (R)0;
     const int cnt = min(W.ncnt[i], P.nb_cap);
     R dr = 0, tx = 0, ty = 0, px = 0, py = 0, flt = 0;
-    auto pair = [&](const V4<R>& pj, const V4<R>& bj, const V2<R>& cj) {
-        const V2<R> d = w_disp(pi, pj);
-        const R r2 = d.x * d.x + d.y * d.y;
-        const R r = sqrt(r2);
+    auto pair = [&](const WPos<R>& pj, const V4<R>& bj, const V2<R>& cj) {
+        const double2 dd = w_disp(pi, pj);
+        const R r = w_len(dd, (R)0);
+        const V2<R> d = mk2<R>((R)dd.x, (R)dd.y);
         if (filt) flt += bj.z * c2_w(K, r);
         const R G = c2_g(K, r), vg = bj.z * G;
         const bool mj = cj.y > (R)0;
@@ -504,7 +517,7 @@ __global__ void __launch_bounds__(128) k_w_pair(DevParams P, WParams Q, WState<R
             const R uij = dux * d.x + duy * d.y;
             if (uij < (R)0) {
                 const R hij = (hi + fabs(cj.y)) * (R)0.5;
-                const R phi = hij * uij / (r2 + (R)0.01 * hij * hij);
+                const R phi = hij * uij / (r * r + (R)0.01 * hij * hij);
                 const R q = -mi * phi * (al + be * phi) / (rhoi + cj.x) * (R)0.5 * G;
                 tx += q * d.x;
                 ty += q * d.y;
@@ -515,7 +528,8 @@ __global__ void __launch_bounds__(128) k_w_pair(DevParams P, WParams Q, WState<R
     int k = g.lane;
     for (; k + (U - 1) * L < cnt; k += U * L) {
         int j[U];
-        V4<R> pj[U], bj[U];
+        WPos<R> pj[U];
+        V4<R> bj[U];
         V2<R> cj[U];
 #pragma unroll
         for (int u = 0; u < U; u++) j[u] = __ldg(W.nbr + (size_t)(k + u * L) * n + i);
@@ -530,7 +544,7 @@ __global__ void __launch_bounds__(128) k_w_pair(DevParams P, WParams Q, WState<R
     }
     for (; k < cnt; k += L) {
         const int j = __ldg(W.nbr + (size_t)k * n + i);
-        const V4<R> pj = ldr(W.rp + j);
+        const WPos<R> pj = ldr(W.rp + j);
         pair(pj, ldr(W.rb + j), w_rho_h(pj, W.rc, j));
     }
     dr = g.sum(dr);
@@ -726,7 +740,7 @@ __global__ void k_w_gather(DevParams P, WParams Q, WState<R> src, WState<R> dst,
     dst.ptype[i] = pt; dst.btype[i] = bt; dst.itype[i] = it; dst.pid[i] = id;
     if (src.bed) dst.bed[i] = bed;
     const R hs = pt > 0 ? (R)h : -(R)h;
-    W.rp[i] = w_pos_rec(x, y, (R)rho, hs);
+    w_pos_rec(W.rp + i, x, y, (R)rho, hs);
     W.rb[i] = mk4<R>(ux, uy, (R)(m / rho), pres);
     if (W.rc) W.rc[i] = mk2<R>((R)rho, hs);
 }
