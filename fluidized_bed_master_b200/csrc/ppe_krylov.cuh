@@ -110,6 +110,7 @@ struct KRaw;   // a pair as loaded
 template <>
 struct KRaw<float> {
     int4 v;
+    __device__ __forceinline__ void none(int i) { v = make_int4(i, 0, i, 0); }   // zeros at the row itself
     __device__ __forceinline__ void load(const int2* e) { v = kent_ld16(e); }
     __device__ __forceinline__ KPair get() const {
         return KPair{v.x, v.z, (double)__int_as_float(v.y), (double)__int_as_float(v.w)};
@@ -118,6 +119,7 @@ struct KRaw<float> {
 template <>
 struct KRaw<double> {
     int4 v, w;
+    __device__ __forceinline__ void none(int i) { v = w = make_int4(i, 0, 0, 0); }
     __device__ __forceinline__ void load(const int4* e) {
         v = kent_ld16(e);
         w = kent_ld16(e + 1);
@@ -330,19 +332,72 @@ __global__ void __launch_bounds__(128) k_kry_assemble(DevParams P, SphState<R> S
     }
 }
 
-// y_i = d_i x_i - sum_k a_ik x_j(k) over the stored entries of row i.  Groups
-// of 8 entries (rows are padded to whole groups, so nothing is predicated):
-// the next group's entries load while the current one's gathers are in
+// y_i = d_i x_i - sum_k a_ik x_j(k) over the stored entries of row i, 8 at a
+// time: the next group's entries load while the current one's gathers are in
 // flight; even and odd entries have their own sums.  With a test per entry
 // and 8-byte loads a product ran 31 instructions per entry.
-template <typename R>
+//   EXACT: groups that every row of the warp fills load without a test (that
+//     loop is the warp's, so its rows stay together); from there on each pair
+//     is tested and nothing past the row is read.
+//   else: rows are read to the end of their last group, whose padding is zeros;
+//     no test at all and fewer registers.
+// Past the row lie 6 % of the bytes: a system that streams its entries
+// (rows_exact) takes EXACT; 2.83 million rows 339 -> 316 us an iteration of the
+// CG (325 with a test per entry), 655 -> 591 us of the BiCGStab.  At 300,000
+// rows only the FP32 CG gains from it (column 50.6 -> 49.2 us); the BiCGStab
+// loses by its registers (79 -> 83 us an iteration) and the FP64 CG is level.
+template <typename R, bool EXACT>
 __device__ __forceinline__ double kry_row(const KryWork<R>& K, int n, int i, int cnt, const double* __restrict__ xin) {
     using T = typename KEnt<R>::T;
     const T* __restrict__ ent = K.e + kent_at(i, 0, K.cap);   // pair q at ent[64 q]
     (void)n;
     double s0 = 0, s1 = 0;
-    if (cnt > 0) {
-        KRaw<R> cur[4];
+    KRaw<R> cur[4];
+    auto sum = [&]() {
+        double x0[4], x1[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const KPair e = cur[q].get();
+            x0[q] = __ldg(xin + e.j0);
+            x1[q] = __ldg(xin + e.j1);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const KPair e = cur[q].get();
+            s0 += e.a0 * x0[q];
+            s1 += e.a1 * x1[q];
+        }
+    };
+    if constexpr (EXACT) {
+        const int full = __reduce_min_sync(__activemask(), cnt >> 3);   // groups that every row fills
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            cur[q].none(i);
+            if (2 * q < cnt) cur[q].load(ent + q * 64);
+        }
+        int left = cnt;   // entries from the current group on
+        for (int g = 1; g < full; g++, left -= 8) {
+            KRaw<R> nxt[4];
+            ent += 256;
+#pragma unroll
+            for (int q = 0; q < 4; q++) nxt[q].load(ent + q * 64);
+            sum();
+#pragma unroll
+            for (int q = 0; q < 4; q++) cur[q] = nxt[q];
+        }
+        for (; left > 0; left -= 8) {
+            KRaw<R> nxt[4];
+            ent += 256;
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                nxt[q].none(i);
+                if (8 + 2 * q < left) nxt[q].load(ent + q * 64);
+            }
+            sum();
+#pragma unroll
+            for (int q = 0; q < 4; q++) cur[q] = nxt[q];
+        }
+    } else if (cnt > 0) {
 #pragma unroll
         for (int q = 0; q < 4; q++) cur[q].load(ent + q * 64);
         for (int k = 0; k < cnt; k += 8) {
@@ -352,19 +407,7 @@ __device__ __forceinline__ double kry_row(const KryWork<R>& K, int n, int i, int
 #pragma unroll
                 for (int q = 0; q < 4; q++) nxt[q].load(ent + q * 64);
             }
-            double x0[4], x1[4];
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const KPair e = cur[q].get();
-                x0[q] = __ldg(xin + e.j0);
-                x1[q] = __ldg(xin + e.j1);
-            }
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const KPair e = cur[q].get();
-                s0 += e.a0 * x0[q];
-                s1 += e.a1 * x1[q];
-            }
+            sum();
 #pragma unroll
             for (int q = 0; q < 4; q++) cur[q] = nxt[q];
         }
@@ -374,7 +417,7 @@ __device__ __forceinline__ double kry_row(const KryWork<R>& K, int n, int i, int
 
 // y = A x over the stored coefficients; optional fused dots
 // part[s0] += w0.y, part[s1] += w1.y (w1 == nullptr: y.y)
-template <typename R>
+template <typename R, bool EXACT>
 __global__ void __launch_bounds__(KRY_T) k_kry_spmv(int n, KryWork<R> K, const int* __restrict__ nb,
                                                     const double* __restrict__ xin, double* __restrict__ yout,
                                                     const double* __restrict__ w0, int s0, const double* w1, int s1,
@@ -385,7 +428,7 @@ __global__ void __launch_bounds__(KRY_T) k_kry_spmv(int n, KryWork<R> K, const i
     double d0 = 0, d1 = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         int cnt = K.kcnt[i];
-        double y = cnt ? kry_row<R>(K, n, i, cnt - 1, xin) : 0.0;
+        double y = cnt ? kry_row<R, EXACT>(K, n, i, cnt - 1, xin) : 0.0;
         yout[i] = y;
         d0 += w0[i] * y;
         if (two) d1 += (w1 ? w1[i] : y) * y;
@@ -560,7 +603,7 @@ __global__ void __launch_bounds__(KRY_T) k_cg_upd(int n, const double* __restric
 // the last block to finish adds the partials in block order and advances
 // the scalars: the residual, the stop decision (and the while node's
 // condition), alpha and beta of the next update
-template <typename R>
+template <typename R, bool EXACT>
 __global__ void __launch_bounds__(KRY_T) k_cg_spmv(int n, KryWork<R> K, const double* __restrict__ u,
                                                    double* __restrict__ w, const double* __restrict__ r,
                                                    const double* __restrict__ b, int first,
@@ -576,7 +619,7 @@ __global__ void __launch_bounds__(KRY_T) k_cg_spmv(int n, KryWork<R> K, const do
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         int cnt = K.kcnt[i];
         double ui = u[i];
-        double wi = cnt ? kry_row<R>(K, n, i, cnt - 1, u) : 0.0;
+        double wi = cnt ? kry_row<R, EXACT>(K, n, i, cnt - 1, u) : 0.0;
         w[i] = wi;
         double ri = r[i], mi = K.wm[i];
         g += mi * ri * ui;
