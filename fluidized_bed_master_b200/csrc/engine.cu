@@ -838,8 +838,10 @@ int enqueue_step(SphdemHandle* H, EngineHost<R>* EH, int flags, int64_t* nl) {
             auto kb = !kt3 && sl ? (kt5 ? k_passB_any<R, false, 5, 8> : k_passB_any<R, false, -1, 8>)
                       : kt5 ? k_passB_any<R, false, 5, 1> : !kt3 ? k_passB_any<R, false, -1, 1> : P.con ? k_passB<R, true> : k_passB<R, false>;
             int bb = bl;
-            if (P.iface | P.fb | P.sps | P.ipf) kb = k_passB_any<R, true, -1, 1>, bb = bs;
-            else if (P.fva) kb = k_passB_any<R, false, -1, 1>, bb = bs;
+            // the optional forces and the artificial viscosity read m_j and rho_j:
+            // the general pass, one thread per particle, the type fixed for C2
+            if (P.iface | P.fb | P.sps | P.ipf) kb = kt3 ? k_passB_any<R, true, 3, 1> : k_passB_any<R, true, -1, 1>, bb = bs;
+            else if (P.fva) kb = kt3 ? k_passB_any<R, false, 3, 1> : k_passB_any<R, false, -1, 1>, bb = bs;
             CK((launch_pdl(kb, bb, TPB, 0, st, P, S, W, E.flags)));
         }
         *nl += 1;
