@@ -1151,7 +1151,7 @@ __global__ void __launch_bounds__(128) k_dem_prep_c2(DevParams P, SphState<R> S,
     const Cull cu = make_cull(xi, yi, zi, Rr);
     const unsigned lt = (1u << lane) - 1u;
     // the sphere's SPH neighbours (p_type <= 1000, the add = 0 form of the
-    // predicate, which k_dem_coupling_c2 uses), in visit order
+    // predicate, which k_dem_coupling uses), in visit order
     int cs = 0;
     auto pos = [&](int j) { return ldr(rec.pos + j); };
     for_rows_warp_pre<PosRec<R>>(P, ic, jc, kc, srows, cu, sm, lane, pos, [&](int j, const PosRec<R>& qj) {
@@ -3323,10 +3323,10 @@ __global__ void __launch_bounds__(128) k_passB_any(DevParams P, SphState<R> S, S
     R flt = 0, tx = 0, ty = 0, tz = 0, px = 0, py = 0, pz = 0, Rc = 0, ex = 0, ey = 0, ez = 0, et = 0;
     const int* __restrict__ nb = W.nbr;
     if constexpr (L > 1) {
-        static_assert(!FORCES, "several lanes: the default forces");
+        static_assert(!FORCES, "several lanes: the default forces, without artificial viscosity");
         struct T {
-            R p, w, s, gx, gy, gz, cv, dux, duy, duz, pij, ex, ey, ez, mr, et, rc, rr;
-            int f;   // 1 filter, 2 forces, 4 artificial viscosity
+            R p, w, s, gx, gy, gz, cv, dux, duy, duz, ex, ey, ez, mr, et, rc, rr;
+            int f;   // 1 filter, 2 forces
         };
         auto load = [&](int j) {
             NbQ44<R> t;
@@ -3362,15 +3362,6 @@ __global__ void __launch_bounds__(128) k_passB_any(DevParams P, SphState<R> S, S
             o.dux = uxi - uj.x;
             o.duy = uyi - uj.y;
             o.duz = uzi - uj.z;
-            if (P.fva != 0) {
-                R uij = (uxi - uj.x) * g.dx + (uyi - uj.y) * g.dy + (uzi - uj.z) * g.dz;
-                if (uij < (R)0) {
-                    R hij = (th + th) * (R)0.5;
-                    R phi = hij * uij / (r * r + (R)0.01 * hij * hij);
-                    o.pij = mi * phi * ((R)-0.1 * (R)P.soundspeed + (R)0.02 * phi) / (rhoi + fj.y) * (R)0.5;
-                    o.f |= 4;
-                }
-            }
             o.mr = mj * irj * ((R)1 - eli);
             R ug = uxi * gx + uyi * gy + uzi * gz;
             o.ex = (uj.x - uxi) * ug;
@@ -3393,11 +3384,6 @@ __global__ void __launch_bounds__(128) k_passB_any(DevParams P, SphState<R> S, S
                 tx += o.cv * o.dux;
                 ty += o.cv * o.duy;
                 tz += o.cv * o.duz;
-            }
-            if (o.f & 4) {
-                tx += -o.pij * o.gx;
-                ty += -o.pij * o.gy;
-                tz += -o.pij * o.gz;
             }
             if (eli < (R)1) {
                 ex += o.ex * o.mr;
