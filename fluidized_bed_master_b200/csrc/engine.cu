@@ -1536,7 +1536,6 @@ struct WEngineHost {
     Alloc A;
 };
 
-// launch KERN<R, L> with L lanes per particle (n L threads in blocks of TPB)
 // the settings whose step runs the fused pass (k_w_pair)
 static bool w_fused(const DevParams& P, const WParams& Q) {
     return P.kernel_type == 3 && P.kgc != 1 && Q.delsph == 0;
@@ -1567,6 +1566,7 @@ static cudaError_t w_pairs(int L, const DevParams& P, const WParams& Q, const WS
     return launch_pdl(k, nblocks(P.ns * l, TPB), TPB, 0, st, P, Q, S, W, (const DevFlags*)F);
 }
 
+// launch KERN<R, L> with L lanes per particle (n L threads in blocks of TPB)
 #define W_LAUNCH(L, KERN, n, st, ...)                                                                      \
     do {                                                                                                   \
         switch (L) {                                                                                       \

@@ -39,9 +39,9 @@
 // bound by L1 wavefronts and issue slots).  The sign of the volume tells the
 // types that the Shepard sums take (PA: p_type 1; PB: 1 or 3) from the
 // others, and a NaN volume marks a particle that a pass cannot take from the
-// record alone (outside the fixed-point range, p_type >= 1000, i_type 4, or
-// a volume that is not >= 0): pv_slow reads that pair from the tagged
-// records and the double positions.
+// record alone (outside the fixed-point range, p_type >= 1000, or a volume that
+// is not >= 0): pv_slow reads that pair from the tagged records and the double
+// positions.  Parked slots (i_type 3) are in no list; pass A leaves theirs unset.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -447,7 +447,7 @@ __host__ __device__ __forceinline__ size_t nb_at(int k, int n, int i) {
 // others, NaN for a particle of the slow path
 template <typename R>
 __device__ __forceinline__ R pv_code(R v, int tag, bool shepard) {
-    if (!(v >= (R)0) || (tag & TAG_OOR) || tag_ptype(tag) >= 1000 || tag_itype(tag) == 4)
+    if (!(v >= (R)0) || (tag & TAG_OOR) || tag_ptype(tag) >= 1000)
         return sizeof(R) == 4 ? (R)__int_as_float(0x7fffffff) : (R)__longlong_as_double(0x7fffffffffffffffll);
     return shepard ? v : -v;
 }

@@ -1282,7 +1282,7 @@ __global__ void __launch_bounds__(128) k_sps(DevParams P, SphState<R> S, SphWork
 // The delta-SPH density gradient of prep3D is not formed: no kernel of the
 // ISPH step reads it.
 // ---------------------------------------------------------------------------
-// The pair terms with G = dW/dr / r (KnlSum), d = x_i - x_j, V = m_j / rho_j,
+// The pair terms with G = dW/dr / r (C2Sum), d = x_i - x_j, V = m_j / rho_j,
 // C the symmetric gradient correction and du = u_i - u_j:
 //   pressure          (p_i + p_j) V G (C d)          C and factors after the loop
 //   viscous           du V G c_v (d . C d) / r^2
@@ -2689,7 +2689,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 5 : 1) k_ppe(DevParams P
         [&](int j, NbP4S<R>& t, PairV<R>& g) {
             int tag;
             if (!pv_fix(S, rec.pos, W.m_new, W.rho_new, slow_i, t.q, i, j, g, tag)) return;
-            if (tag_ptype(tag) >= 1000 || tag_itype(tag) == 4) {   // no neighbour of this sum
+            if (tag_ptype(tag) >= 1000) {   // no neighbour of this sum
                 g.v = 0;
                 t.b = pui;
                 t.s = prhoi;
