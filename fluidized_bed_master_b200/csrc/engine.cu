@@ -584,7 +584,11 @@ inline cudaError_t launch_neumann_tiled(Engine<float>& E, const SphState<float>&
                       (const int*)nullptr, (const int*)nullptr);
 }
 
-// the wall pass: tiled in FP32 and, for Wendland C2, in FP64; else a warp per wall
+// the wall pass: tiled in FP32 and, for Wendland C2 with more walls than this,
+// in FP64; else a warp per wall.  A tile's walls are one warp's serial work, 63 us
+// however few there are: 63, 63, 79 and 143 us on beds with 4,092, 13,020, 30,600
+// and 97,920 walls, a warp per wall 24, 51, 98 and 294.
+constexpr int FEW_WALLS = 16384;
 template <typename R>
 cudaError_t launch_neumann(Engine<R>& E, const SphState<R>& S, R* pres, int patch_p, cudaStream_t st) {
     const DevParams& P = E.P;
@@ -592,7 +596,7 @@ cudaError_t launch_neumann(Engine<R>& E, const SphState<R>& S, R* pres, int patc
     if constexpr (std::is_same<R, float>::value) {
         return launch_neumann_tiled(E, S, pres, patch_p, st);
     } else {
-        if (!P.c2_passes)
+        if (!P.c2_passes || P.nwall <= FEW_WALLS)
             return launch_pdl(k_neumann<R>, nblocks(P.nwall * 32, TPB), TPB, 0, st, P, S, W, pres, (const int4*)W.rows,
                               patch_p);
         if (cell_sort_sparse(E.cs_s, P.ns))
