@@ -1127,7 +1127,11 @@ __global__ void __launch_bounds__(128) k_dem_prep(DevParams P, SphState<R> S, Sp
 // kernel in nearly every round with a few lanes on.  The porosity sum takes
 // the spheres from k_dem_near's list where the kernel's radius lies inside its
 // range.  78 -> 66 us on the bench bed, 0.66 -> 0.57 ms on
-// 200,000 spheres: bound by the scan.
+// 200,000 spheres: bound by the scan.  The list in shared memory is longer than
+// the one k_dem_coupling reads, so that spheres with up to DEM_LIST SPH
+// neighbours are scanned once (20,000 with 300 each: 180 us, 276 with a second
+// scan, 196 summing inside the scan).
+constexpr int DEM_LIST = 512;
 template <typename R>
 __global__ void __launch_bounds__(128) k_dem_prep_c2(DevParams P, SphState<R> S, SphRec<R> rec, DemState<double> D,
                                                      DemWork<double> DW, const int4* __restrict__ srows,
@@ -1135,7 +1139,7 @@ __global__ void __launch_bounds__(128) k_dem_prep_c2(DevParams P, SphState<R> S,
     grid_dep_wait();
     const int i = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     __shared__ int s_rows[4][20];
-    __shared__ int s_list[4][DEM_SPH_CAP];
+    __shared__ int s_list[4][DEM_LIST];
     int* sm = s_rows[threadIdx.x >> 5];
     int* list = s_list[threadIdx.x >> 5];
     if (i >= P.nd) return;
@@ -1164,7 +1168,7 @@ __global__ void __launch_bounds__(128) k_dem_prep_c2(DevParams P, SphState<R> S,
         const unsigned m = __ballot_sync(0xffffffffu, in);
         if (in) {
             const int pos = cs + __popc(m & lt);
-            if (pos < DEM_SPH_CAP) list[pos] = j;
+            if (pos < DEM_LIST) list[pos] = j;
         }
         cs += __popc(m);
     });
@@ -1182,11 +1186,11 @@ __global__ void __launch_bounds__(128) k_dem_prep_c2(DevParams P, SphState<R> S,
         f1 += ptj == 1 ? c : (R)0;
         f3 += ptj == 3 ? c : (R)0;
     };
-    if (cs <= DEM_SPH_CAP) {
+    if (cs <= DEM_LIST) {
         int* __restrict__ nbs = DW.nbs + (size_t)i * DEM_SPH_CAP;
         for (int k = lane; k < cs; k += 32) {
             const int j = list[k];
-            nbs[k] = j;
+            if (k < DEM_SPH_CAP) nbs[k] = j;
             shep(j);
         }
     } else {   // more than the list holds: the stencil again
